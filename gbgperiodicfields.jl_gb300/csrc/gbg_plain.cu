@@ -964,14 +964,47 @@ __global__ void k_to_one_based(const uint32_t *__restrict__ perm, int32_t *__res
     order[i] = (int32_t)perm[i] + 1;
 }
 
-__global__ void k_validate(const int32_t *__restrict__ order, int64_t m, uint32_t *seen,
-                           unsigned long long *stats) {
+// Bound by the bitmap's L2 atomics, one per entry: a bit per point (an eighth of a byte to clear
+// and touch instead of a word), while the span and the number of points seen first are kept per
+// thread and reach the one global triple by three atomics a block.  With three atomics per entry, all
+// on that triple, 3e6 entries took 3.9 ms; now the order's whole rebuild, this check and a 9-component
+// gather at its points take 1.80 ms (5.72 before).
+__global__ void __launch_bounds__(kThreads)
+    k_validate(const int32_t *__restrict__ order, int64_t m, uint32_t *__restrict__ seen, unsigned long long *stats) {
+  __shared__ int32_t s_lo[kThreads / 32], s_hi[kThreads / 32];
+  __shared__ uint32_t s_new[kThreads / 32];
+  int32_t lo = INT32_MAX, hi = INT32_MIN;
+  uint32_t fresh = 0u;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const long long v = order[i];
-    atomicMin(reinterpret_cast<long long *>(stats), v);
-    atomicMax(reinterpret_cast<long long *>(stats + 1), v);
-    if (v >= 1 && v <= m && atomicExch(seen + (v - 1), 1u) == 0u) atomicAdd(stats + 2, 1ull);
+    const int32_t v = __ldg(order + i);
+    lo = min(lo, v);
+    hi = max(hi, v);
+    if (v >= 1 && v <= m) {
+      const uint32_t k = (uint32_t)v - 1u, bit = 1u << (k & 31u);
+      fresh += (atomicOr(seen + (k >> 5), bit) & bit) ? 0u : 1u;
+    }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  fresh = __reduce_add_sync(0xffffffffu, fresh);
+  if ((threadIdx.x & 31) == 0) {
+    s_lo[threadIdx.x >> 5] = lo;
+    s_hi[threadIdx.x >> 5] = hi;
+    s_new[threadIdx.x >> 5] = fresh;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kThreads / 32; ++w) {
+      lo = min(lo, s_lo[w]);
+      hi = max(hi, s_hi[w]);
+      fresh += s_new[w];
+    }
+    if (lo <= hi) {  // a block without entries has nothing to say
+      atomicMin(reinterpret_cast<long long *>(stats), (long long)lo);
+      atomicMax(reinterpret_cast<long long *>(stats + 1), (long long)hi);
+      atomicAdd(stats + 2, (unsigned long long)fresh);
+    }
   }
 }
 
@@ -1592,11 +1625,12 @@ gbg_status gbg_validate_traversal(const int32_t *order, int64_t npoints, int64_t
   if (!order) return set_error(GBG_EARG, "validate traversal: null order");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Scratch scratch;
-  const size_t need = 256 + sizeof(uint32_t) * (size_t)npoints;
+  const size_t words = ((size_t)npoints + 31) / 32;  // a bit per point
+  const size_t need = 256 + sizeof(uint32_t) * words;
   GBG_TRY(scratch.acquire(nullptr, 0, need, st));
   unsigned long long *stats = static_cast<unsigned long long *>(scratch.ptr);
   uint32_t *seen = reinterpret_cast<uint32_t *>(static_cast<char *>(scratch.ptr) + 256);
-  GBG_CUDA_TRY(cudaMemsetAsync(seen, 0, sizeof(uint32_t) * (size_t)npoints, st));
+  GBG_CUDA_TRY(cudaMemsetAsync(seen, 0, sizeof(uint32_t) * words, st));
   k_validate_init<<<1, 1, 0, st>>>(stats);
   note_launch();
   k_validate<<<launch_blocks(npoints, kThreads), kThreads, 0, st>>>(order, npoints, seen, stats);
