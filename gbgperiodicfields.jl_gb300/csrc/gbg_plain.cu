@@ -7,18 +7,13 @@
 //
 // The gather is one thread per work item, as in the reference, contracting the x
 // direction first for every component of the chunk.  The scatter is not the reference's
-// atomic push: points are sorted by brick and cell (a stable device counting sort), and each
-// brick's nodes are accumulated in shared memory as 128-bit integer sums on a scale local to
-// the brick (or, for a stencil wider than the grid, every node pulls its contributions).  No
-// float atomics are used, so the scatter is bitwise reproducible and independent of any
-// traversal order, and each node keeps the accuracy of an FP64 sum of its own
-// contributions.
-#include <mutex>
+// atomic push: points are grouped by brick and cell (a counting placement), and a thread per node
+// of a brick sums the node's contributions as integers on a scale local to the brick (or, for a
+// stencil wider than the grid, in floating point in a fixed order).  No float atomics are used, so
+// the scatter is bitwise reproducible and independent of any traversal order, and each node keeps
+// the accuracy of an FP64 sum of its own contributions.
+#include <algorithm>
 #include <string>
-
-#include <array>
-#include <map>
-#include <vector>
 
 #include "gbg_common.cuh"
 
@@ -32,6 +27,7 @@ struct GridT {
   int64_t nx, ny, nz, npf;
   T ox, oy, oz;  // T.(grid.origin)
   T dx, dy, dz;  // T.(grid.grid_spacing)
+  T rx, ry, rz;  // their reciprocals, rounded once
 };
 
 template <typename T>
@@ -47,6 +43,9 @@ GridT<T> make_grid(const gbg_grid &g) {
   r.dx = T(g.spacing[0]);
   r.dy = T(g.spacing[1]);
   r.dz = T(g.spacing[2]);
+  r.rx = T(1) / r.dx;
+  r.ry = T(1) / r.dy;
+  r.rz = T(1) / r.dz;
   return r;
 }
 
@@ -192,15 +191,14 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Fixed-point exponent P of the scatter's weights, w * 2^P: |w| <= L (the scheme's
-// Bernstein bound with evaluation slack) <= 1.5 * 2^lb, P = 62 - lb.  Then
-// |w * 2^P| < 1.5 * 2^62, a product of three weights' high halves stays below
-// 3.375 * 2^58, a contribution below 3.375 * 2^56, and a node's sum, shifted by
-// bits(K_max) - 5, below 2^63.
+// Bernstein bound with evaluation slack) <= 1.5 * 2^lb, P = 61 - lb.  Then |w * 2^P| < 1.5 *
+// 2^61 (its high digit of 31 bits fits an int32), a product of two less its low 62 bits stays
+// below 2.25 * 2^60 and of three below 3.375 * 2^59.
 int fixed_weight_exp(const gbg_scheme &sch) {
   const double L = weight_bound(sch, std::ldexp(1.0, -40));
   int lb = 0;
   while (1.5 * std::ldexp(1.0, lb) < L && lb < 60) ++lb;
-  return 62 - lb;
+  return 61 - lb;
 }
 
 // Run-time width (stencils of 10..16 nodes): nothing unrolled.
@@ -422,42 +420,121 @@ __global__ void __launch_bounds__(kThreads)
 
 // ------------------------------------------------------ brick scatter
 //
-// The default scatter.  Points are sorted by brick and by cell within the brick (a stable
-// counting sort, so the order is fixed).  A CTA owns one brick of nodes and accumulates, in
-// shared memory, every contribution of the points in the cells whose stencils reach the
-// brick (the extended region) as a 128-bit integer, so the sum does not depend on the
-// order in which threads add.  Each node is written to HBM once.
+// The default scatter.  Points are grouped by brick and by cell within the brick (a counting
+// placement; the order within a cell does not matter, every sum being an integer).  A CTA owns one
+// brick of nodes and a thread one of its nodes; the thread visits the points whose stencils reach
+// its node and sums their contributions in registers as integers, so the sum does not depend on
+// the order.  Each node is written to HBM once, and no atomic touches a node.
 
 struct BrickGeo {
-  int32_t b[3];
+  int32_t b[3];   // nodes (and cells) of a brick
   int64_t nb[3];
   int64_t bvol;
-  // the scatter's shared accumulators: node (x, y, z) of component c at
-  // c*slice + z*pp + y*p0 + x, pitches chosen so that a warp's atomics on one point's
-  // stencil spread over the banks (choose_acc_pitches)
-  int32_t p0 = 0, pp = 0;
-  int64_t slice = 0;
-  // most runs of consecutive keys along x in one row of any brick's region (brick_segments)
-  int32_t nseg = 1;
+  int32_t eb[3];  // the bricks that the largest quantity exponents are kept for
+  int64_t enb[3];
 };
 
-// Binary exponents of the quantities, biased so that 0 means "no non-zero quantity" and
-// kENonFinite (above every finite one) a NaN or an infinity: a non-zero finite v has
-// 2^(e-1) <= |v| < 2^e and is stored as e + kEBias.
+// The reference's _locate with the quotient from the reciprocal of the spacing, r = RN(1/d): q =
+// RN(a r), then q + r (a - q d) with the residual exact by a fused multiply-add (Markstein's
+// correction).  Before its rounding the corrected quotient is within 2^-104 of a/d, so it is the
+// correctly rounded one of _locate unless a/d lies that close to a midpoint.  The floor is taken on
+// the bits: GB300 starts an FP64 operation of a warp every 76 clocks per scheduler and these points
+// need five instead of about seventeen.  False where floor(Int, q) throws in the reference.
+__device__ __forceinline__ bool locate_recip(double x, double o, double d, double r, int64_t &base, double &t) {
+  const double a = x - o;
+  const double q0 = a * r;
+  const double q = fma(fma(-q0, d, a), r, q0);
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(q);
+  const unsigned long long mag = bits & 0x7fffffffffffffffull;
+  const bool ok = mag < 0x43df399b1438a100ull;  // the bits of 9.0e18; NaN and infinities order above
+  const int ex = (int)(mag >> 52) - 1023;
+  unsigned long long whole = 0ull, cut = 0ull;  // |trunc q|, and the fraction's bits
+  unsigned long long tb = bits & 0x8000000000000000ull;
+  if (ex >= 0 && ok) {
+    const unsigned long long man = (mag & 0xfffffffffffffull) | 0x10000000000000ull;
+    const unsigned long long low = ex < 52 ? (1ull << (52 - ex)) - 1ull : 0ull;
+    cut = bits & low;
+    tb = bits & ~low;
+    whole = ex <= 52 ? man >> (52 - ex) : man << (ex - 52);
+  } else if (ok) {
+    cut = mag;
+  }
+  double fl = __longlong_as_double((long long)tb);
+  base = (long long)whole;
+  if (bits >> 63) {
+    base = -base;
+    if (cut) {
+      base -= 1;
+      fl -= 1.0;
+    }
+  }
+  if (!ok) base = 0;
+  t = q - fl;
+  return ok;
+}
+__device__ __forceinline__ bool locate_recip(float x, float o, float d, float, int64_t &base, float &t) {
+  return locate(x, o, d, base, t);  // FP32 divides at full rate
+}
+
+template <typename T>
+__device__ __forceinline__ bool locate3_recip(const GridT<T> &g, const T *__restrict__ pos, int64_t p, int64_t m,
+                                              int64_t (&b)[3], T (&t)[3]) {
+  bool ok = locate_recip(__ldg(pos + p), g.ox, g.dx, g.rx, b[0], t[0]);
+  ok &= locate_recip(__ldg(pos + p + m), g.oy, g.dy, g.ry, b[1], t[1]);
+  ok &= locate_recip(__ldg(pos + p + 2 * m), g.oz, g.dz, g.rz, b[2], t[2]);
+  return ok;
+}
+
+// A quantity as an exact integer mantissa and a binary exponent, from its bits: v = mq 2^(e - 62)
+// with 2^61 <= |mq| < 2^62.  The exponent is kept biased so that 0 means zero and kENonFinite (above
+// every finite one) a NaN or an infinity.
 constexpr int kEBias = 2048;
 constexpr int kENonFinite = 4095;
 
-__device__ __forceinline__ int biased_exponent(double v) {
-  if (v == 0.0) return 0;
-  if (!isfinite(v)) return kENonFinite;
-  int e = 0;
-  frexp(v, &e);
+__device__ __forceinline__ int split_quantity(double v, long long &mq) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  const int be = (int)((bits >> 52) & 0x7ffu);
+  unsigned long long man = bits & 0xfffffffffffffull;
+  mq = 0;
+  if (be == 0x7ff) return kENonFinite;
+  if (be == 0 && man == 0ull) return 0;
+  int e = be - 1022;
+  if (be) {
+    man = (man | 0x10000000000000ull) << 9;
+  } else {  // subnormal: man 2^-1074
+    const int up = __clzll((long long)man) - 2;
+    man <<= up;
+    e = 62 - 1074 - up;
+  }
+  mq = (bits >> 63) ? -(long long)man : (long long)man;
+  return e + kEBias;
+}
+__device__ __forceinline__ int split_quantity(float v, long long &mq) {
+  const uint32_t bits = __float_as_uint(v);
+  const int be = (int)((bits >> 23) & 0xffu);
+  unsigned long long man = bits & 0x7fffffu;
+  mq = 0;
+  if (be == 0xff) return kENonFinite;
+  if (be == 0 && man == 0ull) return 0;
+  int e = be - 126;
+  if (be) {
+    man = (man | 0x800000ull) << 38;
+  } else {  // subnormal: man 2^-149
+    const int up = __clzll((long long)man) - 2;
+    man <<= up;
+    e = 62 - 149 - up;
+  }
+  mq = (bits >> 31) ? -(long long)man : (long long)man;
   return e + kEBias;
 }
 
+__device__ __forceinline__ int64_t wrap_cell(int64_t c, int64_t n) {
+  return (uint64_t)c < (uint64_t)n ? c : imod(c, n);
+}
+
 // One pass over the points in their own order: the locate, the brick-major key, the cell
-// count (the atomic's value is the point's rank in its cell, for the counting sort), and
-// per brick and component the largest exponent of the finite non-zero alpha*q.
+// count (the atomic's value is the point's rank in its cell, for the placement), and
+// per exponent brick and component the largest exponent of the finite non-zero alpha*q.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     k_brick_keys(GridT<T> g, BrickGeo bg, const T *__restrict__ pos, int64_t m, uint32_t *__restrict__ keys,
@@ -468,465 +545,632 @@ __global__ void __launch_bounds__(kThreads)
        p += (int64_t)gridDim.x * blockDim.x) {
     int64_t b[3];
     T t[3];
-    const bool ok = locate3(g, pos, p, m, b, t);
+    const bool ok = locate3_recip(g, pos, p, m, b, t);
     if (!ok && status) atomicOr(status, GBG_DEV_NONFINITE);
-    int64_t brick = 0, local = 0;
+    // cells, bricks and keys fit 32 bits (fewer than 2^32 keys)
+    uint32_t brick = 0, local = 0, eb = 0;
 #pragma unroll
     for (int d = 2; d >= 0; --d) {
-      const int64_t c = imod(b[d], n[d]);
-      brick = brick * bg.nb[d] + c / bg.b[d];
-      local = local * bg.b[d] + c % bg.b[d];
+      const uint32_t c = (uint32_t)wrap_cell(b[d], n[d]);
+      const uint32_t bd = c / (uint32_t)bg.b[d];
+      brick = brick * (uint32_t)bg.nb[d] + bd;
+      local = local * (uint32_t)bg.b[d] + (c - bd * (uint32_t)bg.b[d]);
+      eb = eb * (uint32_t)bg.enb[d] + c / (uint32_t)bg.eb[d];
     }
-    const uint32_t key = (uint32_t)(brick * bg.bvol + local);
+    const uint32_t key = brick * (uint32_t)bg.bvol + local;
     keys[p] = key;
     rank[p] = atomicAdd(counts + key, 1u);
     for (int c = 0; c < ncomp; ++c) {
-      const T v = mul_rn(alpha, q[p + m * c]);  // quantity = T(alpha)*q
-      const int e = biased_exponent((double)v);
+      long long mq;
+      const int e = split_quantity(mul_rn(alpha, __ldg(q + p + m * c)), mq);  // quantity = T(alpha)*q
       if (e == kENonFinite) {
         if (status) atomicOr(status, GBG_DEV_NONFINITE);
       } else if (e) {
-        atomicMax(ebrick + brick * ncomp + c, (uint32_t)e);
+        // most points find their brick's exponent at least as large already
+        uint32_t *at = ebrick + (size_t)eb * ncomp + c;
+        if (__ldcg(at) < (uint32_t)e) atomicMax(at, (uint32_t)e);
       }
     }
   }
 }
 
-// In sorted order, slot by slot: the point's three axes' stencil weights (the reference's
-// Horner with fused multiply-adds, once per point) as 64-bit fixed point w * 2^wexp, and
-// each alpha*q in floating form of its own: a 64-bit mantissa q * 2^(62 - e) (exact for
-// every double) beside its biased exponent e.  The weights are evaluated here, from the
-// position read through the permutation, rather than in the key pass, so they are written
-// once, already sorted.
+__device__ __forceinline__ long long weight_digits(long long w) {
+  return (long long)((unsigned long long)(w >> 31) << 32 | ((unsigned long long)w & 0x7fffffffull));
+}
+
+// The point of every slot: a point goes to its cell's first slot plus its rank there.
+__global__ void __launch_bounds__(kThreads)
+    k_brick_place(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ rank,
+                  const uint32_t *__restrict__ starts, int64_t m, uint32_t *__restrict__ perm) {
+  // four points a trip: keys and ranks, then the keys' starts, then the stores
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < m; p += 4 * stride) {
+    uint32_t k[4], r[4], a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = p + u * stride < m;
+      k[u] = in ? __ldg(keys + p + u * stride) : 0u;
+      r[u] = in ? __ldg(rank + p + u * stride) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = __ldg(starts + k[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p + u * stride < m) perm[a[u] + r[u]] = (uint32_t)(p + u * stride);
+  }
+}
+
+// Slot by slot: the point's three axes' stencil weights (the reference's Horner with fused
+// multiply-adds, once per point) as fixed point W = w * 2^wexp in two digits, the signed W >> 31 in the
+// high half of a word and the 31 bits below it in the low half, and each alpha*q as its mantissa and
+// exponent.  Reading the points through the permutation and writing in slot order moves a third less
+// than writing the points' own order to its slots (1e7 points at width 4: 2.5 ms so).
 template <typename T, int N2, int M2>
 __global__ void __launch_bounds__(kThreads)
     k_brick_order(GridT<T> g, SchemeT<T, N2> sch, const T *__restrict__ pos, const uint32_t *__restrict__ perm,
                   int64_t m, int wexp, long long *__restrict__ wts, const T *__restrict__ q, int ncomp, T alpha,
-                  long long *__restrict__ qi, int32_t *__restrict__ qe) {
+                  long long *__restrict__ qi, int16_t *__restrict__ qe) {
   for (int64_t sl = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; sl < m;
        sl += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = perm[sl];
+    const int64_t p = __ldg(perm + sl);
+    for (int c = 0; c < ncomp; ++c) {
+      long long mq;
+      const int e = split_quantity(mul_rn(alpha, __ldg(q + p + m * c)), mq);
+      qi[sl * ncomp + c] = mq;
+      qe[sl * ncomp + c] = (int16_t)e;
+    }
     int64_t b[3];
     T t[3];
-    const bool ok = locate3(g, pos, p, m, b, t);
-    long long *dst = wts + sl * (3 * N2);
+    const bool ok = locate3_recip(g, pos, p, m, b, t);
+    longlong2 *dst = reinterpret_cast<longlong2 *>(wts + sl * (3 * N2));  // 48, 96, 144 or 192 bytes a point
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       T w[N2];
-      axis_weights_fma<T, N2, M2>(sch, ok ? t[d] : quiet_nan<T>(), w);
+      axis_weights_fma<T, N2, M2>(sch, ok ? t[d] : T(0), w);
 #pragma unroll
-      for (int k = 0; k < N2; ++k) dst[d * N2 + k] = ok ? fixed_rn((double)w[k], wexp) : 0ll;
-    }
-    for (int c = 0; c < ncomp; ++c) {
-      const T v = mul_rn(alpha, q[p + m * c]);
-      const int e = biased_exponent((double)v);
-      qi[sl * ncomp + c] = (e && e != kENonFinite) ? fixed_rn((double)v, 62 - (e - kEBias)) : 0ll;
-      qe[sl * ncomp + c] = e;
+      for (int k = 0; k < N2; k += 2)
+        dst[(d * N2 + k) / 2] = make_longlong2(ok ? weight_digits(fixed_rn((double)w[k], wexp)) : 0ll,
+                                               ok ? weight_digits(fixed_rn((double)w[k + 1], wexp)) : 0ll);
     }
   }
 }
 
-// Adds the 128-bit integer (hi:lo) to the sum kept in shared memory as four 32-bit words
-// w0 (lowest) .. w3, with native 32-bit atomics: each word's add returns the old value,
-// whose wrap is the carry into the next word.  Each add wraps a word at most once, so
-// after all adds the words hold the exact 128-bit sum (mod 2^128) in any order, as the
-// two-word form atomic_add_split64 does for 64 bits.
-__device__ __forceinline__ void atomic_add_split128(uint32_t *w0, uint32_t *w1, uint32_t *w2, uint32_t *w3, int i,
-                                                    unsigned long long lo, unsigned long long hi) {
-  const uint32_t v0 = (uint32_t)lo, v1 = (uint32_t)(lo >> 32), v2 = (uint32_t)hi, v3 = (uint32_t)(hi >> 32);
-  const uint32_t o0 = atomicAdd(w0 + i, v0);
-  const uint32_t c1 = (uint32_t)(o0 + v0 < v0);
-  const uint32_t s1 = v1 + c1;  // wraps only when v1 == 2^32 - 1 and c1 == 1 (then s1 == 0)
-  const uint32_t o1 = atomicAdd(w1 + i, s1);
-  const uint32_t c2 = (uint32_t)(s1 < c1) + (uint32_t)(o1 + s1 < s1);
-  const uint32_t s2 = v2 + c2;
-  const uint32_t o2 = atomicAdd(w2 + i, s2);
-  const uint32_t c3 = (uint32_t)(s2 < c2) + (uint32_t)(o2 + s2 < s2);
-  atomicAdd(w3 + i, v3 + c3);
+// A 192-bit two's-complement integer (s2 its signed top): s += v << sh.
+struct Int192 {
+  unsigned long long s0, s1, s2;
+};
+template <int SH>
+__device__ __forceinline__ void add_shifted(Int192 &s, long long v) {
+  constexpr int b = SH & 63;
+  const unsigned long long ext = (unsigned long long)(v >> 63);
+  const unsigned long long lo = (unsigned long long)v << b;
+  const unsigned long long hi = b ? (unsigned long long)(v >> ((64 - b) & 63)) : ext;
+  if constexpr (SH < 64) {
+    s.s0 += lo;
+    unsigned long long c = s.s0 < lo;
+    const unsigned long long h = hi + c;
+    c = h < c;
+    s.s1 += h;
+    c += s.s1 < h;
+    s.s2 += ext + c;
+  } else {
+    s.s1 += lo;
+    const unsigned long long c = s.s1 < lo;
+    s.s2 += hi + c;
+  }
 }
 
-// One contribution: the node weight wn (64-bit fixed point) times the quantity's mantissa
-// mq (exact signed 64 x 64 -> 128-bit product), shifted right by d with rounding (half up),
-// added to the node's 128-bit sum.  d >= 127 leaves nothing to add.
-__device__ __forceinline__ void add_contribution(uint32_t *a0, uint32_t *a1, uint32_t *a2, uint32_t *a3, int i,
-                                                 long long wn, long long mq, int d) {
-  if (mq == 0 || wn == 0 || d >= 127) return;
-  unsigned long long lo = (unsigned long long)wn * (unsigned long long)mq;
-  long long hi = __mul64hi(wn, mq);
-  if (d > 0) {
-    // + 2^(d-1), then an arithmetic shift right by d
-    if (d <= 64) {
-      const unsigned long long h = 1ull << (d - 1);
-      const unsigned long long s = lo + h;
-      hi += (long long)(s < lo);
-      lo = s;
-    } else {
-      hi += (long long)(1ull << (d - 65));
-    }
-    if (d < 64) {
-      lo = (lo >> d) | ((unsigned long long)hi << (64 - d));
-      hi >>= d;
-    } else if (d == 64) {
-      lo = (unsigned long long)hi;
-      hi = hi < 0 ? -1ll : 0ll;
-    } else {
-      lo = (unsigned long long)(hi >> (d - 64));
-      hi = hi < 0 ? -1ll : 0ll;
+// s * 2^e rounded once to a double (ties to even); the rare results outside the normal range are
+// left to ldexp.
+__device__ __forceinline__ double to_double(Int192 s, int e) {
+  const bool neg = (long long)s.s2 < 0;
+  if (neg) {
+    s.s0 = ~s.s0 + 1ull;
+    const unsigned long long c0 = s.s0 == 0ull;
+    s.s1 = ~s.s1 + c0;
+    s.s2 = ~s.s2 + (unsigned long long)(c0 && s.s1 == 0ull);
+  }
+  if ((s.s0 | s.s1 | s.s2) == 0ull) return 0.0;
+  // the leading bit to bit 191
+  if (s.s2 == 0ull) {
+    s.s2 = s.s1;
+    s.s1 = s.s0;
+    s.s0 = 0ull;
+    e -= 64;
+    if (s.s2 == 0ull) {
+      s.s2 = s.s1;
+      s.s1 = 0ull;
+      e -= 64;
     }
   }
-  atomic_add_split128(a0, a1, a2, a3, i, lo, (unsigned long long)hi);
+  const int up = __clzll((long long)s.s2);
+  if (up) {
+    s.s2 = (s.s2 << up) | (s.s1 >> (64 - up));
+    s.s1 = (s.s1 << up) | (s.s0 >> (64 - up));
+    s.s0 <<= up;
+  }
+  e += 191 - up;  // what the leading bit weighs
+  const unsigned long long top = s.s2 >> 11, rem = s.s2 & 0x7ffull;
+  const bool sticky = (s.s1 | s.s0) != 0ull;
+  const unsigned long long man =
+      top + (unsigned long long)(rem > 0x400ull || (rem == 0x400ull && (sticky || (top & 1ull))));
+  const int biased = e + 1023;
+  if (biased >= 1 && biased <= 2045) {
+    const unsigned long long bits = ((unsigned long long)biased << 52) + (man - 0x10000000000000ull);
+    return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+  }
+  const double v = ldexp((double)man, e - 52);
+  return neg ? -v : v;
 }
 
-template <int N, typename T>
-__device__ __forceinline__ T pick_t(const T (&w)[N], int q) {
-  T v = w[0];
-#pragma unroll
-  for (int i = 1; i < N; ++i)
-    if (i == q) v = w[i];
+__device__ __forceinline__ void mad_wide(long long &acc, int a, int b) {
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
+}
+
+// The product of two fixed-point numbers of two 31-bit digits, h 2^31 + l, less its low 62 bits (to
+// two units: the lowest partial product is left out).
+__device__ __forceinline__ long long mul_high62(int ah, int al, int bh, int bl) {
+  long long mid = 0, top;
+  mad_wide(mid, ah, bl);
+  mad_wide(mid, al, bh);
+  top = mid >> 31;
+  mad_wide(top, ah, bh);
+  return top;
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ int2 lds64(uint32_t a) {
+  int2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
   return v;
 }
 
-// The default scatter (deterministic, FP64-grade per node).  A CTA owns one brick of
-// nodes.  It lists the points of every cell whose stencil reaches the brick (the extended
-// region), gives each warp a point (its lanes cover the point's nodes inside the brick),
-// and adds every contribution w1*w2*w3*alpha*q to a 128-bit integer accumulator in shared
-// memory.
-//
-// The arithmetic is integer: GB300's FP64 rate is 1/58 of its FP32 rate, while 64-bit
-// integer products run on the integer pipes.  The weights are 64-bit fixed point w * 2^P
-// (P = 62 - lb, |w| <= 1.5 * 2^lb from the scheme's Bernstein bound), converted once per
-// point; a node's weight is hi(wx, hi(wy, wz)), the high halves of two signed 64 x 64-bit
-// products (w1 w2 w3 * 2^(3P - 128), to 2^-58 of itself).  Each quantity keeps its own
-// binary exponent e_p beside an exact 64-bit mantissa q * 2^(62 - e_p), and every
-// component of the brick's region has a scale: the largest exponent e_r among its points.
-// A contribution is the exact 128-bit product of the node weight and the mantissa, shifted
-// right (rounded) by (e_r - e_p) + sh onto that common scale; sh = max(0, bits(K_max) - 5),
-// K_max the brick's largest node coverage, keeps the sum of a node's contributions below
-// 2^127 (each is below 3.375 * 2^(120 - sh)).  The largest contribution keeps about
-// 120 - sh significant bits and one 2^-k of it keeps 120 - sh - k, so a node's sum has the
-// accuracy of an FP64 sum of its own contributions unless the region spans more than about
-// 2^60 in magnitude: the scale is local to the brick, not global.  Integer addition is
-// associative, so the result does not depend on which thread adds first; the 128-bit sums
-// are added as four 32-bit words with carries (atomic_add_split128).  A non-finite quantity
-// marks every node its stencil reaches, which is written as NaN (the reference's 0 * NaN
-// included).
-constexpr int kFlatChunk = 1024;
-// the scatter's static shared memory: one count per warp for the block scan
-constexpr int kScanSlots = 32;
-// quantities of a point the warp-per-point scatter holds in registers (the rest are read per use)
-constexpr int kQReg = 4;
+// Digits of a quantity on its region's scale, ND of kDigit bits to a window.  With 2^e_r above every
+// quantity of the region, window 0 holds q / 2^(e_r + 1 - 24 ND) down to its whole part (a signed top
+// digit, the others unsigned), window k the next 24 ND k bits below it.  Three digits keep a double
+// whole unless it is below 2^-18 of the region's largest, two a float below 2^-23: what is left
+// then makes further windows, up to kWindows, that are summed apart.
+constexpr int kDigit = 24, kWindows = 3;
+template <typename T>
+constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 
-template <typename T, int N2>
-__global__ void __launch_bounds__(kThreads)
-    k_scatter_fixed128(GridT<T> g, BrickGeo bg, int ncomp,
-                       const uint32_t *__restrict__ cell_start, const long long *__restrict__ wts,
-                       const long long *__restrict__ qi, const int32_t *__restrict__ qe,
-                       const uint32_t *__restrict__ ebrick, int wexp, T *__restrict__ field, T beta, int beta_zero) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int half = N2 / 2;
-  const int E0 = bg.b[0] + N2 - 1, E1 = bg.b[1] + N2 - 1, E2 = bg.b[2] + N2 - 1;
-  const int ecount = E0 * E1 * E2;
+// The default scatter (deterministic, at least FP64-grade per node).  A CTA takes a brick of nodes (up
+// to 8x8x4) and each thread one node.  The brick's region (its cells widened by N2 - 1) is listed with
+// per-cell offsets; its points are staged in shared memory (three axes' weights, the quantities'
+// digits for CC components), and a thread walks the N2 x N2 rows of cells that feed its node, one
+// trip a point: no lane works for a node that the point does not reach.
+//
+// The arithmetic is integer: an FP64 operation of a warp takes 76 clocks of a scheduler, a 32 x 32 ->
+// 64-bit multiply-add 2.  A node's weight is the product of three fixed-point weights w * 2^P (P = 61 -
+// lb, |w| <= 1.5 * 2^lb from the scheme's Bernstein bound), each product less its low 62 bits: w1 w2 w3
+// * 2^(3P - 124), to a few units of 2^-59 and below 2^61.  Cut in two digits, of 30 bits and the signed
+// rest, it meets the quantity's digits in
+// 2 ND products below 2^54, each added by one multiply-add to an accumulator of its own: no shifts
+// and no carries per contribution, and up to 511 points before one could overflow.  The accumulators
+// are folded at their weights into a 192-bit sum, which holds any number of contributions exactly;
+// the only roundings of a node are those of its weights, the last window's end (2^-155 of the
+// region's largest contribution, or less) and the final conversion.  A non-finite quantity marks
+// every node its stencil reaches, which is written as NaN (the reference's 0 * NaN included).
+//
+// Bound by issue and by the latency of a brick's phases (at 256^3 x 3 and 6e6 uniform points half of its
+// time is the listing and staging, half the trips, at 23 of 32 lanes).  What it replaced gave each warp
+// a point and added to 128-bit sums in shared memory by four dependent atomics per contribution; 256^3
+// x 3, 1e7 points with 30% in blobs, cubic: 21.4 ms, now 10.5.  Three CTAs per SM (80 registers, which
+// spill) take 12.0.
+constexpr int kOwnerPoints = 508;  // staged points: at most 511 trips between folds
+
+// Shared words of a staged point: the digits of CC components and the meta word, in 16-byte units of
+// an odd count (or one), so that lanes reading neighbouring points meet different banks.
+template <int CC, int ND>
+constexpr int kDigitWords = CC * ND + 1 <= 4 ? 4 : 12;
+template <int N2>
+constexpr int kWeightWords = 3 * N2 + 1;  // 64-bit words, odd
+
+// The trips of one lane's node over the staged points: `rows` marks (bit kk * 8 + jj) the rows of cells
+// (lx..lx+N2-1, ly+jj, lz+kk) to take.  The loop is the warp's, held together by its vote: a trip takes
+// one point of every lane that has one left, and a lane whose row is done moves to its next row within
+// the trip.  (Left to itself the compiler makes this a loop over rows around a loop over their points,
+// where the lanes wait for the fullest of 32 rows at every row.)  Returns the points' meta words, or-ed.
+template <int N2, int CC, int ND>
+__device__ __forceinline__ uint32_t owner_walk(unsigned long long rows, const uint32_t *po, int ebase, int E0, int E1,
+                                               int xk, uint32_t c0, uint32_t c1, uint32_t digits, uint32_t weights,
+                                               long long (&A)[CC][2 * ND]) {
+  constexpr int DW = kDigitWords<CC, ND>, WW = kWeightWords<N2>;
+  int todo = 0;
+  uint32_t marks = 0u, dp = 0, wp = 0, wy = 0, wz = 0;  // the point's digits and weights
+  auto next_row = [&]() {
+    const int s = __ffsll((long long)rows) - 1;
+    rows &= rows - 1ull;
+    const int kk = s >> 3, jj = s & 7;
+    const int e0 = ebase + (kk * E1 + jj) * E0;
+    const uint32_t p0 = max(po[e0], c0);
+    todo = (int)(min(po[e0 + N2], c1) - p0);
+    dp = digits + (p0 - c0) * (DW * 4);
+    wp = weights + (p0 - c0) * (WW * 8);
+    wy = wp + 8 * (2 * N2 - 1 - jj);
+    wz = wp + 8 * (3 * N2 - 1 - kk);
+    wp += 8 * xk;
+  };
+  if (rows) next_row();
+#pragma unroll
+  for (int c = 0; c < CC; ++c)
+#pragma unroll
+    for (int j = 0; j < 2 * ND; ++j) A[c][j] = 0ll;
+  while (__any_sync(0xffffffffu, todo > 0)) {
+    if (todo > 0) {
+      uint32_t d[12];
+#pragma unroll
+      for (int j = 0; j < (CC * ND + 4) / 4; ++j) {
+        const uint4 v = lds128(dp + 16 * j);
+        d[4 * j] = v.x;
+        d[4 * j + 1] = v.y;
+        d[4 * j + 2] = v.z;
+        d[4 * j + 3] = v.w;
+      }
+      const uint32_t meta = d[CC * ND];
+      const int2 b = lds64(wy), c = lds64(wz), a = lds64(wp - 8 * (meta & 0xffu));
+      const long long u = mul_high62(b.y, b.x, c.y, c.x);
+      const long long w = mul_high62((int)(u >> 31), (int)((uint32_t)u & 0x7fffffffu), a.y, a.x);
+      marks |= meta;
+      const int w0 = (int)((uint32_t)w & 0x3fffffffu), w1 = (int)(w >> 30);
+#pragma unroll
+      for (int c = 0; c < CC; ++c)
+#pragma unroll
+        for (int j = 0; j < ND; ++j) {
+          mad_wide(A[c][j], w0, (int)d[c * ND + j]);
+          mad_wide(A[c][ND + j], w1, (int)d[c * ND + j]);
+        }
+      dp += DW * 4;
+      wp += WW * 8;
+      wy += WW * 8;
+      wz += WW * 8;
+      if (--todo == 0 && rows) next_row();
+    }
+  }
+  return marks;
+}
+
+// The accumulators folded at their weights.
+template <int ND>
+__device__ __forceinline__ Int192 owner_fold(const long long (&A)[2 * ND]) {
+  Int192 s{0ull, 0ull, 0ull};
+  add_shifted<0>(s, A[0]);
+  add_shifted<24>(s, A[1]);
+  if constexpr (ND == 3) add_shifted<48>(s, A[2]);
+  add_shifted<30>(s, A[ND]);
+  add_shifted<54>(s, A[ND + 1]);
+  if constexpr (ND == 3) add_shifted<78>(s, A[ND + 2]);
+  return s;
+}
+
+template <typename T, int N2, int CC>
+__global__ void __launch_bounds__(kThreads, 2)
+    k_scatter_owner(GridT<T> g, BrickGeo bg, int ncomp, int chunk, int chunk1, int sums_bytes,
+                    const uint32_t *__restrict__ cell_start, const long long *__restrict__ wts,
+                    const long long *__restrict__ qi, const int16_t *__restrict__ qe,
+                    const uint32_t *__restrict__ ebrick, int wexp, T *__restrict__ field, T beta, int beta_zero,
+                    uint32_t *__restrict__ ticket) {
+  constexpr int ND = kDigits<T>, DW = kDigitWords<CC, ND>, WW = kWeightWords<N2>, half = N2 / 2;
+  static_assert(CC * ND + 1 <= DW, "");
+  extern __shared__ __align__(16) unsigned char smem_owner[];
+  __shared__ uint32_t warp_tot[32];
+  __shared__ uint32_t s_brick[2], s_unit;
+  const int B0 = bg.b[0], B1 = bg.b[1], B2 = bg.b[2];
+  const int E0 = B0 + N2 - 1, E1 = B1 + N2 - 1, E2 = B2 + N2 - 1, ecount = E0 * E1 * E2;
   const int bvol = (int)bg.bvol;
-  // ncomp * slice 128-bit accumulators, comp-major and pitched, as four planes of 32-bit
-  // words, lowest first (atomic_add_split128)
-  const size_t plane = (size_t)bg.slice * ncomp;
-  uint32_t *acc0 = reinterpret_cast<uint32_t *>(smem_raw);
-  uint32_t *acc1 = acc0 + plane, *acc2 = acc1 + plane, *acc3 = acc2 + plane;
-  uint32_t *off = acc3 + plane;                                              // ecount: exclusive prefix
-  // along a row of the region, cells whose keys are consecutive hold consecutive slots, so
-  // one base (first slot - prefix) serves each such run of cells (segment)
-  uint32_t *segbase = off + ecount;                                          // E1*E2*nseg: slot bases
-  uint32_t *pslot = segbase + E1 * E2 * bg.nseg;                             // kFlatChunk: point slot
-  uint32_t *pxyz = pslot + kFlatChunk;                                       // kFlatChunk: packed cell
-  uint32_t *kx = pxyz + kFlatChunk, *ky = kx + E0, *kz = ky + E1;             // per-axis key tables
-  uint32_t *kcnt = kz + E2;                                                   // bvol coverage counts + max
-  uint32_t *segx = kcnt + bvol + 1;                                          // E0: segment of each x
-  uint32_t *segfirst = segx + E0;                                            // nseg: first x of each
-  int32_t *ereg = reinterpret_cast<int32_t *>(segfirst + bg.nseg);           // ncomp: region scales
-  uint32_t *poison = reinterpret_cast<uint32_t *>(ereg + ncomp);             // slice: NaN marks
-  __shared__ uint32_t warp_tot[kScanSlots];
-  const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nwarps = (int)blockDim.x >> 5;
-  const int64_t nbricks = bg.nb[0] * bg.nb[1] * bg.nb[2];
+  const size_t per = DW * 4 + WW * 8 + 4;
+  const size_t staging = max((size_t)sums_bytes + (size_t)chunk * per, (size_t)chunk1 * per);
+  uint32_t *off = reinterpret_cast<uint32_t *>(smem_owner + staging);  // ecount + 1 offsets
+  uint32_t *r0s = off + ecount + 1;                                    // the cells' first slots
+  uint32_t *poff = r0s + ecount;                                       // the same of one pass's share
+  uint32_t *pr0 = poff + ecount + 1;
+  uint32_t *kx = pr0 + ecount, *ky = kx + E0, *kz = ky + E1;           // per-axis key tables
+  uint32_t *xe = kz + E2, *ye = xe + E0, *ze = ye + E1;                // per-axis exponent brick tables
+  uint32_t *marked = ze + E2;                                          // bvol nodes' non-finite marks
+  uint32_t *ereg = marked + bvol;                                      // ncomp region scales
+  unsigned long long *sums = reinterpret_cast<unsigned long long *>(smem_owner);  // bvol * CC 192-bit sums
+  const uint32_t nbricks = (uint32_t)(bg.nb[0] * bg.nb[1] * bg.nb[2]);
   const int n[3] = {(int)g.nx, (int)g.ny, (int)g.nz};
-  const int nb0 = (int)bg.nb[0], nb1 = (int)bg.nb[1];
-  // each thread's first region cell and node, and its stride, as coordinates
-  const int ex0 = (int)threadIdx.x % E0, ey0 = ((int)threadIdx.x / E0) % E1, ez0 = (int)threadIdx.x / (E0 * E1);
+  const int tid = (int)threadIdx.x;
+  // a thread's node; a warp's are a block of 4x4x2 in a full brick, so that its lanes' stencils overlap
+  // and their point counts differ little
+  int nx0 = tid % B0, ny0 = (tid / B0) % B1, nz0 = tid / (B0 * B1);
+  if (B0 == 8 && B1 == 8 && B2 == 4) {
+    const int warp = tid >> 5, lane = tid & 31;
+    nx0 = (lane & 3) + 4 * (warp & 1);
+    ny0 = ((lane >> 2) & 3) + 4 * ((warp >> 1) & 1);
+    nz0 = (lane >> 4) + 2 * (warp >> 2);
+  }
+  // a thread's first region cell and the step to its next, as coordinates
+  const int ex0 = tid % E0, ey0 = (tid / E0) % E1, ez0 = tid / (E0 * E1);
   const int esx = (int)blockDim.x % E0, esy = ((int)blockDim.x / E0) % E1, esz = (int)blockDim.x / (E0 * E1);
-  const int B0 = bg.b[0], B1 = bg.b[1];
-  const int lx0 = (int)threadIdx.x % B0, ly0 = ((int)threadIdx.x / B0) % B1, lz0 = (int)threadIdx.x / (B0 * B1);
-  const int lsx = (int)blockDim.x % B0, lsy = ((int)blockDim.x / B0) % B1, lsz = (int)blockDim.x / (B0 * B1);
-  for (int64_t brick = blockIdx.x; brick < nbricks; brick += gridDim.x) {
-    const int bc[3] = {(int)(brick % nb0), (int)((brick / nb0) % nb1), (int)(brick / ((int64_t)nb0 * nb1))};
-    const int vx = min(B0, n[0] - bc[0] * B0), vy = min(B1, n[1] - bc[1] * B1), vz = min(bg.b[2], n[2] - bc[2] * bg.b[2]);
+  if (tid == 0) s_brick[0] = atomicAdd(ticket, 1u);
+  for (int it = 0;; ++it) {
     __syncthreads();
-    for (int t = threadIdx.x; t < E0 + E1 + E2; t += blockDim.x) {
+    const uint32_t brick = s_brick[it & 1];
+    if (brick >= nbricks) break;
+    // the next brick's number arrives while this one is summed
+    if (tid == 0) s_brick[(it & 1) ^ 1] = atomicAdd(ticket, 1u);
+    const int bc[3] = {(int)(brick % (uint32_t)bg.nb[0]), (int)((brick / (uint32_t)bg.nb[0]) % (uint32_t)bg.nb[1]),
+                       (int)(brick / (uint32_t)(bg.nb[0] * bg.nb[1]))};
+    for (int t = tid; t < E0 + E1 + E2 + ncomp; t += blockDim.x) {
+      if (t >= E0 + E1 + E2) {
+        ereg[t - (E0 + E1 + E2)] = 0u;
+        continue;
+      }
       const int d = t < E0 ? 0 : (t < E0 + E1 ? 1 : 2);
       const int e = t - (d == 0 ? 0 : (d == 1 ? E0 : E0 + E1));
       int c = (bc[d] * bg.b[d] - half + e) % n[d];
       if (c < 0) c += n[d];
       const uint32_t cb = (uint32_t)c / (uint32_t)bg.b[d], cl = (uint32_t)c - cb * (uint32_t)bg.b[d];
       if (d == 0) kx[e] = cb * (uint32_t)bvol + cl;
-      else if (d == 1) ky[e] = cb * (uint32_t)nb0 * (uint32_t)bvol + cl * (uint32_t)B0;
-      else kz[e] = cb * (uint32_t)nb1 * (uint32_t)nb0 * (uint32_t)bvol + cl * (uint32_t)(B0 * B1);
+      else if (d == 1) ky[e] = cb * (uint32_t)bg.nb[0] * (uint32_t)bvol + cl * (uint32_t)B0;
+      else kz[e] = cb * (uint32_t)(bg.nb[1] * bg.nb[0]) * (uint32_t)bvol + cl * (uint32_t)(B0 * B1);
+      // the exponent brick of the cell, marked where the axis enters one
+      const uint32_t eb = (uint32_t)c / (uint32_t)bg.eb[d], before = (uint32_t)(c ? c - 1 : n[d] - 1) / (uint32_t)bg.eb[d];
+      const uint32_t step = d == 0 ? 1u : (uint32_t)(d == 1 ? bg.enb[0] : bg.enb[0] * bg.enb[1]);
+      xe[t] = eb * step | (e == 0 || eb != before ? 0x80000000u : 0u);
     }
     __syncthreads();
-    if (warp == 0) {
-      // segments along x (E0 <= 32): a new one wherever the key does not step by one
-      const bool in = lane < E0;
-      const bool brk = in && (lane == 0 || kx[lane] != kx[lane - 1] + 1u);
-      const uint32_t starts = __ballot_sync(0xffffffffu, brk);
-      if (in) segx[lane] = (uint32_t)__popc(starts & (0xffffffffu >> (31 - lane))) - 1u;
-      const int sg = __popc(starts & ((1u << lane) - 1u));
-      if (brk && sg < bg.nseg) segfirst[sg] = (uint32_t)lane;
+    // the cells, and each component's scale: the largest exponent of the exponent bricks that hold a
+    // cell of the region
+    for (int e = tid, ex = ex0, ey = ey0, ez = ez0; e < ecount; e += blockDim.x) {
+      const uint32_t key = kx[ex] + ky[ey] + kz[ez];
+      const uint32_t a = __ldg(cell_start + key);
+      r0s[e] = a;
+      off[e] = __ldg(cell_start + key + 1) - a;
+      if (xe[ex] & ye[ey] & ze[ez] & 0x80000000u) {
+        const size_t eb = (size_t)(xe[ex] & 0x7fffffffu) + (ye[ey] & 0x7fffffffu) + (ze[ez] & 0x7fffffffu);
+        for (int c = 0; c < ncomp; ++c) atomicMax(ereg + c, __ldg(ebrick + eb * ncomp + c));
+      }
+      ex += esx;
+      ey += esy;
+      ez += esz;
+      if (ex >= E0) { ex -= E0; ++ey; }
+      if (ey >= E1) { ey -= E1; ++ez; }
     }
     __syncthreads();
-    {
-      int ex = ex0, ey = ey0, ez = ez0;
-      for (int e = threadIdx.x; e < ecount; e += blockDim.x) {
-        const uint32_t key = kx[ex] + ky[ey] + kz[ez];
-        const uint32_t r0 = __ldg(cell_start + key);
-        const uint32_t sg = segx[ex];
-        // first slot, for now (the host's bound on the segments keeps sg below nseg)
-        if (segfirst[sg] == (uint32_t)ex && sg < (uint32_t)bg.nseg) segbase[(ez * E1 + ey) * bg.nseg + sg] = r0;
-        off[e] = __ldg(cell_start + key + 1) - r0;
-        ex += esx;
-        ey += esy;
-        ez += esz;
-        if (ex >= E0) { ex -= E0; ++ey; }
-        if (ey >= E1) { ey -= E1; ++ez; }
-      }
-    }
-    __syncthreads();
-    // coverage of every node (points whose stencil reaches it): window sums of the cell
-    // counts, over x and y into the accumulators as scratch, then over z
-    if (threadIdx.x == 0) kcnt[bvol] = 0u;
-    uint32_t *scratch = acc0;
-    if (E2 <= 4 * bg.b[2] * ncomp) {
-      for (int o = threadIdx.x; o < B0 * B1 * E2; o += blockDim.x) {
-        const int lx = o % B0, r = o / B0, ly = r % B1, ez = r / B1;
-        uint32_t sum = 0;
-#pragma unroll
-        for (int j = 0; j < N2; ++j) {
-          const uint32_t *row = off + (ez * E1 + ly + j) * E0 + lx;
-#pragma unroll
-          for (int i = 0; i < N2; ++i) sum += row[i];
-        }
-        scratch[o] = sum;
-      }
-      __syncthreads();
-      for (int nl = threadIdx.x; nl < bvol; nl += blockDim.x) {
-        uint32_t sum = 0;
-#pragma unroll
-        for (int k = 0; k < N2; ++k) sum += scratch[nl + k * B0 * B1];
-        kcnt[nl] = sum;
-      }
-    } else {
-      for (int nl = threadIdx.x; nl < bvol; nl += blockDim.x) {
-        const int lx = nl % B0, ly = (nl / B0) % B1, lz = nl / (B0 * B1);
-        uint32_t sum = 0;
-        for (int k = 0; k < N2; ++k)
-          for (int j = 0; j < N2; ++j)
-            for (int i = 0; i < N2; ++i) sum += off[((lz + k) * E1 + ly + j) * E0 + lx + i];
-        kcnt[nl] = sum;
-      }
-    }
-    __syncthreads();
-    {
-      uint32_t mx = 0;
-      for (int nl = threadIdx.x; nl < bvol; nl += blockDim.x) mx = max(mx, kcnt[nl]);
-      mx = __reduce_max_sync(0xffffffffu, mx);
-      if ((threadIdx.x & 31) == 0) atomicMax(kcnt + bvol, mx);
-    }
-    for (int i = threadIdx.x; i < 4 * (int)plane; i += blockDim.x) acc0[i] = 0u;
-    for (int i = threadIdx.x; i < (int)bg.slice; i += blockDim.x) poison[i] = 0u;
-    // each component's scale: the largest exponent in the 27 bricks around this one (the
-    // region lies within them; periodic wrap)
-    for (int c = threadIdx.x; c < ncomp; c += blockDim.x) {
-      uint32_t e = 0;
-      for (int d = 0; d < 27; ++d) {
-        const int64_t x = (bc[0] + d % 3 - 1 + nb0) % nb0, y = (bc[1] + (d / 3) % 3 - 1 + nb1) % nb1,
-                      z = (bc[2] + d / 9 - 1 + bg.nb[2]) % bg.nb[2];
-        e = max(e, __ldg(ebrick + ((z * nb1 + y) * nb0 + x) * ncomp + c));
-      }
-      ereg[c] = (int32_t)e;
-    }
-    __syncthreads();
-    const uint32_t kmax = kcnt[bvol];
     const uint32_t count = block_scan_counts(off, ecount, warp_tot);
-    {
-      // each segment's base: its first slot less its first cell's prefix
-      const int nsg = min((int)segx[E0 - 1] + 1, bg.nseg);
-      for (int r = threadIdx.x; r < E1 * E2 * nsg; r += blockDim.x) {
-        const int row = r / nsg, sg = r - row * nsg;
-        segbase[row * bg.nseg + sg] -= off[row * E0 + (int)segfirst[sg]];
-      }
-    }
-    __syncthreads();
-    const int sh = max(0, (32 - __clz((int)kmax)) - 5);
-    // a contribution of exponent e_p lands on the component's scale: d = (e_r - e_p) + sh;
-    // value = sum * 2^(66 + e_r + sh - 3P) (e_r unbiased), P = wexp
-    const bool accumulated = count > 0;
-    if (accumulated) {
-      for (uint32_t c0 = 0; c0 < count; c0 += kFlatChunk) {
-        const uint32_t c1 = min(count, c0 + kFlatChunk);
-        {
-          int ex = ex0, ey = ey0, ez = ez0;
-          for (int e = threadIdx.x; e < ecount; e += blockDim.x) {
-            const uint32_t lo = max(off[e], c0), hi = min(e + 1 < ecount ? off[e + 1] : count, c1);
-            const uint32_t base = segbase[(ez * E1 + ey) * bg.nseg + min(segx[ex], (uint32_t)bg.nseg - 1u)];
-            const uint32_t packed = (uint32_t)ex | ((uint32_t)ey << 8) | ((uint32_t)ez << 16);
-            for (uint32_t t = lo; t < hi; ++t) {
-              pslot[t - c0] = base + t;
-              pxyz[t - c0] = packed;
-            }
-            ex += esx;
-            ey += esy;
-            ez += esz;
-            if (ex >= E0) { ex -= E0; ++ey; }
-            if (ey >= E1) { ey -= E1; ++ez; }
-          }
+    if (tid == 0) off[ecount] = count;
+    for (int cc0 = 0; cc0 < ncomp; cc0 += CC) {
+      long long A[CC][2 * ND] = {};  // the products' accumulators, [weight digit * ND + quantity digit]
+      auto inside = [&](int lx, int ly, int lz) -> bool {
+        return bc[0] * B0 + lx < n[0] && bc[1] * B1 + ly < n[1] && bc[2] * B2 + lz < n[2];
+      };
+      auto write = [&](int c, int lx, int ly, int lz, const Int192 &s, uint32_t marks) {
+        const int e = (int)ereg[cc0 + c];
+        T v = e ? (T)to_double(s, (e - kEBias) + 1 - kDigit * ND + 124 - 3 * wexp) : T(0);
+        if ((marks >> c) & 1u) v = quiet_nan<T>();
+        T *f = field + (bc[0] * B0 + lx) + g.nx * ((bc[1] * B1 + ly) + g.ny * (bc[2] * B2 + lz)) + g.npf * (cc0 + c);
+        *f = beta_zero ? v : add_rn(mul_rn(beta, *f), v);
+      };
+      // staging room for the whole region at once, or pieces beside the 192-bit sums
+      bool multi = count > (uint32_t)chunk1, again;
+      do {
+        again = false;
+        if (multi) {
+          for (int i = tid; i < 3 * CC * bvol; i += blockDim.x) sums[i] = 0ull;
+          for (int i = tid; i < bvol; i += blockDim.x) marked[i] = 0u;
         }
-        __syncthreads();
-        if constexpr (N2 <= 2) {
-          // two-node stencils: a thread per point
-          for (uint32_t t = c0 + threadIdx.x; t < c1; t += blockDim.x) {
-            const uint32_t sl = pslot[t - c0], packed = pxyz[t - c0];
-            const int ex = (int)(packed & 0xffu), ey = (int)((packed >> 8) & 0xffu), ez = (int)(packed >> 16);
-            const long long *wp = wts + (int64_t)sl * (3 * N2);
-            long long w1[N2], w2[N2], w3[N2];
-#pragma unroll
-            for (int k = 0; k < N2; ++k) {
-              w1[k] = wp[k];
-              w2[k] = wp[N2 + k];
-              w3[k] = wp[2 * N2 + k];
+        const int P = multi ? chunk : chunk1;
+        unsigned char *st = smem_owner + (multi ? sums_bytes : 0);
+        uint4 *dig = reinterpret_cast<uint4 *>(st);
+        long long *wgt = reinterpret_cast<long long *>(st + (size_t)P * DW * 4);
+        uint32_t *pslot = reinterpret_cast<uint32_t *>(wgt + (size_t)P * WW);
+        const uint32_t digits = (uint32_t)__cvta_generic_to_shared(dig),
+                       weights = (uint32_t)__cvta_generic_to_shared(wgt);
+        // A crowded region goes in passes that each take an even share of every cell (the cells'
+        // remainders falling in passes of their own), so that every pass has work for every node;
+        // a pass above the staging's size goes in pieces.
+        const uint32_t even = (uint32_t)(P * 7 / 8), passes = multi ? (count + even - 1) / even : 1u;
+        for (uint32_t pass = 0; pass < passes && !again; ++pass) {
+          const uint32_t *po = off, *pr = r0s;
+          uint32_t total = count;
+          if (multi) {
+            __syncthreads();  // the previous pass is listed no longer
+            for (int e = tid; e < ecount; e += blockDim.x) {
+              const unsigned long long cells = off[e + 1] - off[e], phase = (uint32_t)e * 2654435761u % passes;
+              const unsigned long long at0 = cells * pass + phase, at1 = at0 + cells;
+              const bool wide = (at1 >> 32) != 0ull;
+              const uint32_t a = wide ? (uint32_t)(at0 / passes) : (uint32_t)at0 / passes;
+              const uint32_t b = wide ? (uint32_t)(at1 / passes) : (uint32_t)at1 / passes;
+              pr0[e] = r0s[e] + a;
+              poff[e] = b - a;
             }
-            const long long *qv = qi + (int64_t)sl * ncomp;
-            const int kz0 = max(0, N2 - 1 - ez), kz1 = min(N2, vz + N2 - 1 - ez);
-            const int ky0 = max(0, N2 - 1 - ey), ky1 = min(N2, vy + N2 - 1 - ey);
-            const int lxb = ex - (N2 - 1);
-  #pragma unroll 1
-            for (int k = kz0; k < kz1; ++k) {
-              const int lz = ez + k - (N2 - 1);
-              const long long wz = pick_t(w3, k);
-  #pragma unroll 1
-              for (int j = ky0; j < ky1; ++j) {
-                const int ly = ey + j - (N2 - 1);
-                const long long wyz = __mul64hi(pick_t(w2, j), wz);
-                const int row = lz * bg.pp + ly * bg.p0;
-  #pragma unroll
-                for (int i = 0; i < N2; ++i) {
-                  const int lx = lxb + i;
-                  if (lx < 0 || lx >= vx) continue;
-                  const long long w = __mul64hi(w1[i], wyz);
-                  for (int c = 0; c < ncomp; ++c) {
-                    const int ep = __ldg(qe + (int64_t)sl * ncomp + c);
-                    if (ep == kENonFinite) atomicOr(poison + row + lx, 1u << (c & 31));
-                    else if (ep) add_contribution(acc0, acc1, acc2, acc3, c * (int)bg.slice + row + lx, w,
-                                                  __ldg(qv + c), ereg[c] - ep + sh);
+            __syncthreads();
+            total = block_scan_counts(poff, ecount, warp_tot);
+            if (tid == 0) poff[ecount] = total;
+            po = poff;
+            pr = pr0;
+          }
+          // (an empty region takes one empty piece, which writes its nodes)
+          for (uint32_t c0 = 0; (c0 < total || (c0 == 0 && !multi)) && !again; c0 += (uint32_t)P) {
+            const uint32_t c1 = min(total, c0 + (uint32_t)P);
+            const int np = (int)(c1 - c0);
+            for (int win = 0; win < kWindows; ++win) {
+              __syncthreads();  // the previous points are summed (and the offsets' end is set)
+              if (win == 0) {
+                for (int e = tid, ex = ex0; e < ecount; e += blockDim.x) {
+                  const uint32_t o0 = po[e], lo = max(o0, c0), hi = min(po[e + 1], c1);
+                  for (uint32_t t = lo; t < hi; ++t) {
+                    pslot[t - c0] = pr[e] + (t - o0);
+                    reinterpret_cast<uint32_t *>(dig)[(t - c0) * DW + CC * ND] = (uint32_t)ex;
+                  }
+                  ex += esx;
+                  if (ex >= E0) ex -= E0;
+                }
+                __syncthreads();
+              }
+              int left = 0;  // some quantity has bits below this window
+              for (int t = tid; t < np; t += blockDim.x) {
+                const uint32_t slot = pslot[t];
+                longlong2 v[3 * N2 / 2];
+                if (win == 0) {
+#pragma unroll
+                  for (int k = 0; k < 3 * N2 / 2; ++k)
+                    v[k] = __ldg(reinterpret_cast<const longlong2 *>(wts + (int64_t)slot * (3 * N2)) + k);
+                }
+                uint32_t w[DW];
+                const int64_t q0 = (int64_t)slot * ncomp + cc0;
+                uint32_t meta = reinterpret_cast<uint32_t *>(dig)[t * DW + CC * ND] & 0xffu;
+#pragma unroll
+                for (int k = 0; k < DW; ++k) w[k] = 0u;
+#pragma unroll
+                for (int c = 0; c < CC; ++c) {
+                  const int e = __ldg(qe + q0 + c);
+                  const long long mq = __ldg(qi + q0 + c);  // 0 for a zero or non-finite quantity
+                  if (e == kENonFinite) meta |= 256u << c;
+                  const int r0 = 63 + (e ? max((int)ereg[cc0 + c] - e, 0) : 0) - kDigit * ND * (win + 1);
+                  if (win == 0) {
+                    // the mantissa's bits from r0 up: 24 (ND - 1) of them, and the signed rest above
+                    const int rt = r0 + kDigit * (ND - 1);  // >= 39
+                    w[c * ND + ND - 1] = (uint32_t)(mq >> min(rt, 63));
+                    const unsigned long long low =
+                        r0 >= 0 ? (unsigned long long)(mq >> min(r0, 63)) : (unsigned long long)mq << -r0;
+                    w[c * ND] = (uint32_t)low & 0xffffffu;
+                    if constexpr (ND == 3) w[c * ND + 1] = (uint32_t)(low >> kDigit) & 0xffffffu;
+                  } else {
+#pragma unroll
+                    for (int j = 0; j < ND; ++j) {
+                      const int r = r0 + kDigit * j;
+                      w[c * ND + j] =
+                          (r >= 0 ? (uint32_t)(mq >> min(r, 63)) : r > -kDigit ? (uint32_t)mq << -r : 0u) & 0xffffffu;
+                    }
+                  }
+                  if (r0 > 0 && (mq & ((1ll << min(r0, 63)) - 1ll)) != 0) left = 1;
+                }
+                w[CC * ND] = meta;
+#pragma unroll
+                for (int k = 0; k < DW / 4; ++k)
+                  dig[t * (DW / 4) + k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+                if (win == 0) {
+#pragma unroll
+                  for (int k = 0; k < 3 * N2 / 2; ++k) {
+                    wgt[t * WW + 2 * k] = v[k].x;
+                    wgt[t * WW + 2 * k + 1] = v[k].y;
                   }
                 }
               }
-            }
-          }
-        } else {
-          // a warp per point: its lanes cover the nodes of the point's stencil that lie in
-          // the brick (the sub-box i0..i1 x j0..j1 x k0..k1), so every lane of every atomic
-          // does work; lanes 0..3*N2-1 load one axis weight each, and each node's three
-          // weights arrive by shuffle.  The weight products are formed in the same order as
-          // in the gather (wz * S first, then wy, then wx).  The next point's weights and
-          // first kQReg quantities are loaded while this one is added.
-          uint32_t t = c0 + warp;
-          uint32_t sl_n = 0, packed_n = 0;
-          long long wl_n = 0ll, q_n[kQReg];
-          int e_n[kQReg];
-          auto fetch = [&](uint32_t tt) {
-            sl_n = pslot[tt - c0];
-            packed_n = pxyz[tt - c0];
-            wl_n = lane < 3 * N2 ? __ldg(wts + (int64_t)sl_n * (3 * N2) + lane) : 0ll;
+              if (tid == 0) s_unit = 0u;
+              left = __syncthreads_or(left);
+              if (left && !multi) {  // several windows fold into the sums: start over with room for them
+                again = true;
+                break;
+              }
+              if (!multi) {
+                const bool node = tid < bvol && inside(nx0, ny0, nz0);
+                const int ebase = (nz0 * E1 + ny0) * E0 + nx0;
+                unsigned long long rows = 0ull;
+                if (node) {
 #pragma unroll
-            for (int r = 0; r < kQReg; ++r) {
-              q_n[r] = r < ncomp ? __ldg(qi + (int64_t)sl_n * ncomp + r) : 0ll;
-              e_n[r] = r < ncomp ? __ldg(qe + (int64_t)sl_n * ncomp + r) : 0;
-            }
-          };
-          if (t < c1) fetch(t);
-          for (; t < c1; t += nwarps) {
-            const uint32_t sl = sl_n, packed = packed_n;
-            const long long wl = wl_n;
-            long long qr[kQReg];
-            int er[kQReg];
+                  for (int kk = 0; kk < N2; ++kk)
 #pragma unroll
-            for (int r = 0; r < kQReg; ++r) {
-              qr[r] = q_n[r];
-              er[r] = e_n[r];
-            }
-            if (t + nwarps < c1) fetch(t + nwarps);
-            const int ex = (int)(packed & 0xffu), ey = (int)((packed >> 8) & 0xffu), ez = (int)(packed >> 16);
-            const int i0 = max(0, N2 - 1 - ex), i1 = min(N2, vx + N2 - 1 - ex);
-            const int j0 = max(0, N2 - 1 - ey), j1 = min(N2, vy + N2 - 1 - ey);
-            const int k0 = max(0, N2 - 1 - ez), k1 = min(N2, vz + N2 - 1 - ez);
-            const int nx = i1 - i0, ny = j1 - j0, nz = k1 - k0;
-            if (nx <= 0 || ny <= 0 || nz <= 0) continue;  // warp-uniform
-            const long long *qv = qi + (int64_t)sl * ncomp;
-            const int32_t *ev = qe + (int64_t)sl * ncomp;
-            const int count = nx * ny * nz;
-            // idx -> (ii, jj, kk) by multiply-shift division: exact for idx < 4096, divisors <= 8
-            const uint32_t rnx = (65536u + nx - 1) / nx, rny = (65536u + ny - 1) / ny;
-            const int node0 = (ez - (N2 - 1)) * bg.pp + (ey - (N2 - 1)) * bg.p0 + ex - (N2 - 1);
-            for (int base = 0; base < count; base += 32) {
-              const int idx = base + lane;
-              const int r1 = (int)(((uint32_t)idx * rnx) >> 16), ii = idx - r1 * nx;
-              const int kk = (int)(((uint32_t)r1 * rny) >> 16), jj = r1 - kk * ny;
-              const int i = min(i0 + ii, N2 - 1), j = min(j0 + jj, N2 - 1), k = min(k0 + kk, N2 - 1);
-              const long long wxi = __shfl_sync(0xffffffffu, wl, i);
-              const long long wyj = __shfl_sync(0xffffffffu, wl, N2 + j);
-              const long long wzk = __shfl_sync(0xffffffffu, wl, 2 * N2 + k);
-              if (idx < count) {
-                const long long w = __mul64hi(wxi, __mul64hi(wyj, wzk));
-                const int node = node0 + k * bg.pp + j * bg.p0 + i;
+                    for (int jj = 0; jj < N2; ++jj) {
+                      const int e0 = ebase + (kk * E1 + jj) * E0;
+                      if (po[e0] < po[e0 + N2]) rows |= 1ull << (kk * 8 + jj);
+                    }
+                }
+                const uint32_t marks = owner_walk<N2, CC, ND>(rows, po, ebase, E0, E1, nx0 + N2 - 1, c0, c1, digits, weights, A);
+                if (node)
 #pragma unroll
-                for (int r = 0; r < kQReg; ++r)
-                  if (r < ncomp) {
-                    if (er[r] == kENonFinite) atomicOr(poison + node, 1u << (r & 31));
-                    else if (er[r]) add_contribution(acc0, acc1, acc2, acc3, r * (int)bg.slice + node, w, qr[r],
-                                                     ereg[r] - er[r] + sh);
+                  for (int c = 0; c < CC; ++c) write(c, nx0, ny0, nz0, owner_fold<ND>(A[c]), marks >> 8);
+                break;  // no window is left
+              }
+              // A crowded region's nodes differ much in their points (at a blob's edge tenfold within a
+              // brick), so a node has four lanes, each with a quarter of its rows, and the warps take the
+              // 2x2x2 blocks of nodes as they get free.  (A thread a node there kept a fifth of the lanes
+              // busy.)
+              const int nu0 = (B0 + 1) / 2, nu1 = (B1 + 1) / 2, units = nu0 * nu1 * ((B2 + 1) / 2);
+              const int lane = tid & 31, part = lane & 3;
+              while (true) {
+                int u = lane == 0 ? (int)atomicAdd(&s_unit, 1u) : 0;
+                u = __shfl_sync(0xffffffffu, u, 0);
+                if (u >= units) break;
+                const int lx = 2 * (u % nu0) + ((lane >> 2) & 1), ly = 2 * ((u / nu0) % nu1) + ((lane >> 3) & 1),
+                          lz = 2 * (u / (nu0 * nu1)) + (lane >> 4);
+                const bool node = lx < B0 && ly < B1 && lz < B2 && inside(lx, ly, lz);
+                const int ebase = (lz * E1 + ly) * E0 + lx;
+                unsigned long long rows = 0ull;
+                if (node) {
+#pragma unroll
+                  for (int i = 0; i < (N2 * N2 + 3) / 4; ++i) {
+                    const int r = 4 * i + part;  // rows r of this lane's quarter, turned so that each has every y
+                    const int kk = r / N2, jj = (r + kk) % N2;
+                    if (kk < N2) {
+                      const int e0 = ebase + (kk * E1 + jj) * E0;
+                      if (max(po[e0], c0) < min(po[e0 + N2], c1)) rows |= 1ull << (kk * 8 + jj);
+                    }
                   }
-                for (int c = kQReg; c < ncomp; ++c) {
-                  const int ep = __ldg(ev + c);
-                  if (ep == kENonFinite) atomicOr(poison + node, 1u << (c & 31));
-                  else if (ep) add_contribution(acc0, acc1, acc2, acc3, c * (int)bg.slice + node, w, __ldg(qv + c),
-                                                ereg[c] - ep + sh);
+                }
+                uint32_t marks = owner_walk<N2, CC, ND>(rows, po, ebase, E0, E1, lx + N2 - 1, c0, c1, digits, weights, A);
+                // the four lanes' sums, then a component a lane
+                long long mine[2 * ND];
+#pragma unroll
+                for (int j = 0; j < 2 * ND; ++j) {
+#pragma unroll
+                  for (int c = 0; c < CC; ++c) {
+                    A[c][j] += __shfl_xor_sync(0xffffffffu, A[c][j], 1);
+                    A[c][j] += __shfl_xor_sync(0xffffffffu, A[c][j], 2);
+                  }
+                  mine[j] = A[0][j];
+#pragma unroll
+                  for (int c = 1; c < CC; ++c)
+                    if (part == c) mine[j] = A[c][j];
+                }
+                marks |= __shfl_xor_sync(0xffffffffu, marks, 1);
+                marks |= __shfl_xor_sync(0xffffffffu, marks, 2);
+                if (node && part < CC) {
+                  const int nl = (lz * B1 + ly) * B0 + lx;
+                  if (part == 0 && (marks >> 8)) marked[nl] |= marks >> 8;
+                  Int192 s = owner_fold<ND>(mine);
+                  for (int j = 0; j < win; ++j) {  // down to window 0's weight: 24 ND bits each
+                    constexpr int D = kDigit * ND;
+                    if constexpr (D >= 64) {
+                      s.s0 = (s.s1 >> (D - 64)) | (s.s2 << (128 - D));
+                      s.s1 = (unsigned long long)((long long)s.s2 >> (D - 64));
+                      s.s2 = (unsigned long long)((long long)s.s2 >> 63);
+                    } else {
+                      s.s0 = (s.s0 >> D) | (s.s1 << (64 - D));
+                      s.s1 = (s.s1 >> D) | (s.s2 << (64 - D));
+                      s.s2 = (unsigned long long)((long long)s.s2 >> D);
+                    }
+                  }
+                  unsigned long long *at = sums + (size_t)3 * part * bvol + nl;
+                  Int192 t{at[0], at[bvol], at[2 * bvol]};
+                  t.s0 += s.s0;
+                  unsigned long long cy = t.s0 < s.s0;
+                  const unsigned long long h = s.s1 + cy;
+                  cy = h < cy;
+                  t.s1 += h;
+                  cy += t.s1 < h;
+                  t.s2 += s.s2 + cy;
+                  at[0] = t.s0;
+                  at[bvol] = t.s1;
+                  at[2 * bvol] = t.s2;
                 }
               }
+              if (!left) break;
             }
           }
         }
+        if (again) multi = true;
+      } while (again);
+      if (multi) {
         __syncthreads();
-      }
-    }
-    __syncthreads();
-    // write-back in the reference layout: node fastest, so a warp writes a contiguous row
-    for (int c = 0; c < ncomp; ++c) {
-      int lx = lx0, ly = ly0, lz = lz0;
-      for (int nl = threadIdx.x; nl < bvol; nl += blockDim.x) {
-        if (lx < vx && ly < vy && lz < vz) {
-          const int64_t x = (int64_t)bc[0] * B0 + lx, y = (int64_t)bc[1] * B1 + ly, z = (int64_t)bc[2] * bg.b[2] + lz;
-          T *f = field + x + g.nx * (y + g.ny * z) + g.npf * c;
-          const int64_t ni = lz * bg.pp + ly * bg.p0 + lx, ai = c * bg.slice + ni;
-          // the 128-bit sum as a double (one rounding of the high part, one of the sum)
-          const long long hi = (long long)(((unsigned long long)acc3[ai] << 32) | acc2[ai]);
-          const unsigned long long lo = ((unsigned long long)acc1[ai] << 32) | acc0[ai];
-          const double sum = fma((double)hi, 18446744073709551616.0, (double)lo);
-          T v = (accumulated && ereg[c] > 0) ? (T)ldexp(sum, 66 + (ereg[c] - kEBias) + sh - 3 * wexp) : T(0);
-          if ((poison[ni] >> (c & 31)) & 1u) v = quiet_nan<T>();
-          *f = beta_zero ? v : add_rn(mul_rn(beta, *f), v);
+        if (tid < bvol && inside(nx0, ny0, nz0)) {
+          const int nl = (nz0 * B1 + ny0) * B0 + nx0;
+#pragma unroll
+          for (int c = 0; c < CC; ++c) {
+            const unsigned long long *at = sums + (size_t)3 * c * bvol + nl;
+            write(c, nx0, ny0, nz0, Int192{at[0], at[bvol], at[2 * bvol]}, marked[nl]);
+          }
         }
-        lx += lsx;
-        ly += lsy;
-        lz += lsz;
-        if (lx >= B0) { lx -= B0; ++ly; }
-        if (ly >= B1) { ly -= B1; ++lz; }
       }
+      __syncthreads();  // the sums and the staging are free for the next components
     }
   }
 }
@@ -1079,151 +1323,51 @@ gbg_status dispatch_gather(const gbg_grid &grid, const gbg_scheme &sch, int ncom
   }
 }
 
-// Which scatter runs, and its bricks: the brick push whenever every axis is at least a
-// stencil wide and a brick's accumulators fit in shared memory, else the node pull
-// (which also handles a stencil wider than the grid, reached several times per node).
+// Which scatter runs, and its bricks: a thread per node of a brick whenever every axis is at least
+// a stencil wide, else the node pull (which also handles a stencil wider than the grid, reached
+// several times per node).  More than 22 components keep the pull, as their quantities' mantissas
+// and exponents would need more workspace than the pull's own copy of them.
 struct ScatterPlan {
   bool bricked = false;
   BrickGeo bg{};
   int64_t nkeys = 0;
-  size_t smem = 0;
 };
-
-// Pitches of the scatter's shared accumulators.  A warp adds one point's contributions to
-// the nodes of its stencil inside the brick, x fastest, 32 nodes at a time, with 32-bit
-// atomics on a plane of low words and then a plane of high words (node i's word on bank
-// i mod 32); with the brick's own row and plane pitches the stencil's rows fall on the same
-// banks.  Over row pitches b0..b0+31 and plane pitches b1*p0..b1*p0+31 whose slice stays
-// within max_slice nodes (so that the padding costs no CTA per SM), this takes the pair
-// with the fewest shared-memory wavefronts summed over every position of a full n^3
-// stencil in the brick.
-void choose_acc_pitches(BrickGeo &bg, int n2, int64_t max_slice) {
-  const int b0 = bg.b[0], b1 = bg.b[1], b2 = bg.b[2];
-  const int nx = std::min(n2, b0), ny = std::min(n2, b1), nz = std::min(n2, b2);
-  int64_t best = -1;
-  int best_p0 = b0, best_pp = b0 * b1;
-  std::vector<int> words;
-  for (int p0 = b0; p0 < b0 + 32; ++p0) {
-    for (int pp = b1 * p0; pp < b1 * p0 + 32; ++pp) {
-      if ((int64_t)b2 * pp > max_slice && !(p0 == b0 && pp == b0 * b1)) continue;
-      int64_t total = 0;
-      for (int z0 = 0; z0 + nz <= b2; ++z0)
-        for (int y0 = 0; y0 + ny <= b1; ++y0)
-          for (int x0 = 0; x0 + nx <= b0; ++x0) {
-            words.clear();
-            for (int k = 0; k < nz; ++k)
-              for (int j = 0; j < ny; ++j)
-                for (int i = 0; i < nx; ++i) words.push_back((z0 + k) * pp + (y0 + j) * p0 + x0 + i);
-            for (size_t c = 0; c < words.size(); c += 32) {
-              // wavefronts of one warp instruction: the words are distinct and word w sits on
-              // bank w mod 32, so the most words sharing a bank
-              int per_bank[32] = {0};
-              for (size_t l = c; l < std::min(words.size(), c + 32); ++l) ++per_bank[words[l] & 31];
-              int mx = 0;
-              for (int q = 0; q < 32; ++q) mx = std::max(mx, per_bank[q]);
-              total += mx;
-            }
-          }
-      if (best < 0 || total < best) {
-        best = total;
-        best_p0 = p0;
-        best_pp = pp;
-      }
-    }
-  }
-  bg.p0 = best_p0;
-  bg.pp = best_pp;
-  bg.slice = (int64_t)b2 * best_pp;
-}
-
-// The most segments (runs of consecutive keys) along x in one row of any brick's region:
-// the region's x cells of brick column bc0 are (bc0*b0 - n2/2 + e) mod n0, e < b0 + n2 - 1,
-// keyed by brick * bvol + cell-in-brick, exactly as the scatter kernel keys them.
-int brick_segments(const BrickGeo &bg, int64_t n0, int n2) {
-  const int e0 = bg.b[0] + n2 - 1;
-  int most = 1;
-  for (int64_t bc0 = 0; bc0 < bg.nb[0]; ++bc0) {
-    int segs = 0;
-    int64_t prev = 0;
-    for (int e = 0; e < e0; ++e) {
-      const int64_t c = imod(bc0 * bg.b[0] - n2 / 2 + e, n0);
-      const int64_t key = (c / bg.b[0]) * bg.bvol + c % bg.b[0];
-      if (e == 0 || key != prev + 1) ++segs;
-      prev = key;
-    }
-    most = std::max(most, segs);
-  }
-  return most;
-}
 
 ScatterPlan plan_scatter(const gbg_grid &g, int ncomp, size_t esize, int n2) {
   ScatterPlan p;
-  const int base[3] = {(size_t)ncomp * esize > 24 ? 8 : 16, 8, 8};
-  bool wide_enough = n2 <= 8;
+  // 256 nodes, one a thread: at width 4 a region of 847 cells (3.3 a node), which one staging holds up
+  // to 0.6 points a cell.  8x8x8 bricks with two nodes a thread (2.6 cells a node, half the bricks) took
+  // 14.5 ms where these took 12.8 (256^3 x 3, 1e7 points, 30% in blobs): more regions go in passes.
+  const int base[3] = {8, 8, 4};
+  const int ebase[3] = {(size_t)ncomp * esize > 24 ? 8 : 16, 8, 8};
+  bool wide_enough = n2 <= 8 && ncomp <= 22;
   int64_t nbricks = 1;
   for (int d = 0; d < 3; ++d) {
     p.bg.b[d] = (int32_t)std::min<int64_t>(base[d], g.n[d]);
     p.bg.nb[d] = (g.n[d] + p.bg.b[d] - 1) / p.bg.b[d];
+    p.bg.eb[d] = (int32_t)std::min<int64_t>(ebase[d], g.n[d]);
+    p.bg.enb[d] = (g.n[d] + p.bg.eb[d] - 1) / p.bg.eb[d];
     nbricks *= p.bg.nb[d];
     if (g.n[d] < n2 || g.n[d] >= (int64_t(1) << 31)) wide_enough = false;
   }
   p.bg.bvol = (int64_t)p.bg.b[0] * p.bg.b[1] * p.bg.b[2];
-  const int e0 = p.bg.b[0] + n2 - 1, e1 = p.bg.b[1] + n2 - 1, e2 = p.bg.b[2] + n2 - 1;
-  const size_t ecount = (size_t)e0 * e1 * e2;
-  if (e0 > 32) wide_enough = false;  // the kernel finds the x segments with one warp
-  p.bg.nseg = brick_segments(p.bg, g.n[0], n2);
-  // shared memory besides the accumulators: region offsets and segment bases, the point
-  // chunk, the key tables, the coverage counts, the segment of each x and first x of each,
-  // the components' scales and the NaN marks (one word per node of the padded slice, at
-  // most the accumulators' slice: bvol words plus the padding counted with the slice)
-  const size_t rest = sizeof(uint32_t) * ecount + sizeof(uint32_t) * (size_t)e1 * e2 * p.bg.nseg +
-                      2 * sizeof(uint32_t) * kFlatChunk + sizeof(uint32_t) * (size_t)(e0 + e1 + e2) +
-                      sizeof(uint32_t) * (size_t)(p.bg.bvol + 1) + sizeof(uint32_t) * (size_t)(e0 + p.bg.nseg) +
-                      sizeof(int32_t) * (size_t)ncomp;
-  {
-    // accumulator pitches that keep the unpadded layout's CTAs per SM (228 KB per SM, 1 KB
-    // reserved per CTA by the runtime, the kernel's static scan slots) and its 200 KB cap;
-    // they depend on the brick, the width and the components alone, so each is searched once
-    const size_t per_node = (size_t)ncomp * 16 + sizeof(uint32_t), sm = 228 * 1024,
-                 reserve = 1024 + kScanSlots * sizeof(uint32_t);
-    const size_t unpadded = (size_t)p.bg.bvol * per_node + rest;
-    const size_t ctas = std::max<size_t>(1, sm / (unpadded + reserve));
-    const size_t room = std::min<size_t>(sm / ctas - reserve, 200 * 1024);
-    const int64_t max_slice = room > rest ? (int64_t)((room - rest) / per_node) : p.bg.bvol;
-    static std::mutex mu;
-    static std::map<std::array<int, 5>, std::pair<int, int>> cache;
-    const std::array<int, 5> key = {p.bg.b[0], p.bg.b[1], p.bg.b[2], n2, ncomp};
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it == cache.end()) {
-      choose_acc_pitches(p.bg, n2, std::max<int64_t>(max_slice, p.bg.bvol));
-      cache[key] = {p.bg.p0, p.bg.pp};
-    } else {
-      p.bg.p0 = it->second.first;
-      p.bg.pp = it->second.second;
-      p.bg.slice = (int64_t)p.bg.b[2] * p.bg.pp;
-    }
-  }
-  p.smem = (size_t)p.bg.slice * (ncomp * 16 + sizeof(uint32_t)) + rest;
-  (void)esize;
-  if (ecount > 65535) wide_enough = false;
-  p.bricked = wide_enough && p.smem <= 200 * 1024 && nbricks * p.bg.bvol < (int64_t(1) << 32) - 1;
+  p.bricked = wide_enough && nbricks * p.bg.bvol < (int64_t(1) << 32) - 1;
   p.nkeys = p.bricked ? nbricks * p.bg.bvol : g.n[0] * g.n[1] * g.n[2];
   return p;
 }
 
-// The scatter's workspace: keys, per-cell counts (then slot starts), ranks within a cell
-// (then the fallback sort's keys), the permutation, the counting sort's long-run flag and
-// scratch, the scan's scratch, per sorted slot the three axes' weights (64-bit fixed point
-// for the brick scatter) and the quantities (for the brick scatter as mantissas and
-// exponents, with per brick the largest exponent of every component).
+// The scatter's workspace: keys, per-cell counts (then slot starts), ranks within a cell, the
+// permutation, the scan's scratch, per slot the three axes' weights (64-bit fixed point for the
+// brick scatter) and the quantities (for the brick scatter as mantissas and exponents, with per
+// exponent brick the largest exponent of every component); for the pull also the stable sort's
+// scratch.  flag: the sort's long-run flag, or the brick scatter's ticket.
 struct ScatterLayout {
   uint32_t *keys, *counts, *rank, *perm, *flag;
   void *sort_tmp;
   uint32_t *scan_tmp;
   void *rec, *qs;
   long long *qi;
-  int32_t *qe;
+  int16_t *qe;
   uint32_t *ebrick;
 };
 
@@ -1234,15 +1378,15 @@ ScatterLayout scatter_layout(Arena &a, int64_t m, const ScatterPlan &P, int ncom
   L.rank = a.take<uint32_t>((size_t)m);
   L.perm = a.take<uint32_t>((size_t)m);
   L.flag = a.take<uint32_t>(4);
-  L.sort_tmp = a.take<char>(radix_sort_temp_bytes(m));
+  L.sort_tmp = P.bricked ? nullptr : a.take<char>(radix_sort_temp_bytes(m));
   L.scan_tmp = a.take<uint32_t>(scan_temp_elems(P.nkeys + 1));
   const size_t rec_bytes = 3 * (size_t)n2 * (P.bricked ? sizeof(long long) : esize);
   L.rec = a.take<char>((size_t)m * rec_bytes);
   L.qs = P.bricked ? nullptr : a.take<char>((size_t)m * ncomp * esize);
   L.qi = P.bricked ? a.take<long long>((size_t)m * ncomp) : nullptr;
-  L.qe = P.bricked ? a.take<int32_t>((size_t)m * ncomp) : nullptr;
-  const int64_t nbricks = P.bricked ? P.bg.nb[0] * P.bg.nb[1] * P.bg.nb[2] : 0;
-  L.ebrick = P.bricked ? a.take<uint32_t>((size_t)nbricks * ncomp) : nullptr;
+  L.qe = P.bricked ? a.take<int16_t>((size_t)m * ncomp) : nullptr;
+  const int64_t nexp = P.bricked ? P.bg.enb[0] * P.bg.enb[1] * P.bg.enb[2] : 0;
+  L.ebrick = P.bricked ? a.take<uint32_t>((size_t)nexp * ncomp) : nullptr;
   return L;
 }
 
@@ -1252,6 +1396,39 @@ int bits_for(uint64_t max_value) {
   return b;
 }
 
+// The owner kernel for CC components at a time.
+template <typename T, int N2, int CC>
+gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int wexp, const ScatterLayout &L,
+                        T *field, double beta, cudaStream_t st) {
+  constexpr size_t per = kDigitWords<CC, kDigits<T>> * 4 + kWeightWords<N2> * 8 + 4;
+  const BrickGeo &bg = P.bg;
+  const size_t e[3] = {(size_t)bg.b[0] + N2 - 1, (size_t)bg.b[1] + N2 - 1, (size_t)bg.b[2] + N2 - 1};
+  const size_t tables = sizeof(uint32_t) * (4 * e[0] * e[1] * e[2] + 2 + 2 * (e[0] + e[1] + e[2]) + (size_t)bg.bvol + (size_t)ncomp);
+  const size_t sums = ((size_t)bg.bvol * CC * 24 + 15) & ~size_t(15);
+  // an SM's 228 KB over the CTAs that the launch bounds ask for, less 1 KB reserved and the static part
+  const size_t budget = 228 * 1024 / 2 - 1024 - 512;
+  const int chunk = (int)(std::min<size_t>(kOwnerPoints, (budget - tables - sums) / per) & ~size_t(3));
+  const int chunk1 = (int)(std::min<size_t>(kOwnerPoints, (budget - tables) / per) & ~size_t(3));
+  const size_t smem = std::max(sums + chunk * per, chunk1 * per) + tables;
+  auto kernel = k_scatter_owner<T, N2, CC>;
+  GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  int dev = 0, sms = 1, per_sm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem);
+  const int64_t nbricks = bg.nb[0] * bg.nb[1] * bg.nb[2];
+  const int blocks = (int)std::min<int64_t>(nbricks, (int64_t)sms * std::max(per_sm, 1));
+  mark_main_start(st);
+  kernel<<<blocks, kThreads, smem, st>>>(g, bg, ncomp, chunk, chunk1, (int)sums, L.counts,
+                                         static_cast<const long long *>(L.rec), L.qi, L.qe, L.ebrick, wexp, field,
+                                         T(beta), beta == 0.0, L.flag);
+  mark_main_stop(st);
+  note_launch();
+  GBG_CUDA_TRY(cudaGetLastError());
+  return GBG_OK;
+}
+
 template <typename T, int N2, bool FIXED>
 gbg_status launch_bricked(const GridT<T> &g, const ScatterPlan &P, const gbg_scheme &sch, int ncomp,
                           const T *x, const T *q, int64_t m, double alpha, const ScatterLayout &L, T *field,
@@ -1259,56 +1436,29 @@ gbg_status launch_bricked(const GridT<T> &g, const ScatterPlan &P, const gbg_sch
   const SchemeT<T, N2> s = make_scheme<T, N2>(sch);
   const int wexp = fixed_weight_exp(sch);
   const int blocks_m = launch_blocks(m, kThreads);
-  const int64_t nbricks = P.bg.nb[0] * P.bg.nb[1] * P.bg.nb[2];
-  GBG_CUDA_TRY(cudaMemsetAsync(L.ebrick, 0, sizeof(uint32_t) * (size_t)nbricks * ncomp, st));
+  const int64_t nexp = P.bg.enb[0] * P.bg.enb[1] * P.bg.enb[2];
+  GBG_CUDA_TRY(cudaMemsetAsync(L.ebrick, 0, sizeof(uint32_t) * (size_t)nexp * ncomp, st));
   GBG_CUDA_TRY(cudaMemsetAsync(L.flag, 0, sizeof(uint32_t), st));
   k_brick_keys<T><<<blocks_m, kThreads, 0, st>>>(g, P.bg, x, m, L.keys, L.counts, L.rank, q, ncomp, T(alpha),
                                                  L.ebrick, status);
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
   GBG_TRY(exclusive_scan_u32(L.counts, L.counts, P.nkeys + 1, L.scan_tmp, st));
-  GBG_TRY(stable_counting_sort(L.keys, L.rank, L.counts, m, bits_for((uint64_t)(P.nkeys - 1)), L.perm, L.rank,
-                               L.flag, L.sort_tmp, st));
+  k_brick_place<<<blocks_m, kThreads, 0, st>>>(L.keys, L.rank, L.counts, m, L.perm);
+  note_launch();
   k_brick_order<T, N2, FIXED ? N2 : 0><<<blocks_m, kThreads, 0, st>>>(
       g, s, x, L.perm, m, wexp, static_cast<long long *>(L.rec), q, ncomp, T(alpha), L.qi, L.qe);
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
-  auto kernel = k_scatter_fixed128<T, N2>;
-  GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
-  int dev = 0, sms = 1, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, P.smem);
-  // the padded pitches only where the occupancy query agrees that they cost no CTA per SM
-  BrickGeo bg = P.bg;
-  size_t smem = P.smem;
-  if (bg.slice != bg.bvol) {
-    const size_t flat = smem - (size_t)(bg.slice - bg.bvol) * (ncomp * 16 + sizeof(uint32_t));
-    int flat_per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&flat_per_sm, kernel, kThreads, flat);
-    if (flat_per_sm > per_sm) {
-      bg.p0 = bg.b[0];
-      bg.pp = bg.b[0] * bg.b[1];
-      bg.slice = bg.bvol;
-      smem = flat;
-      per_sm = flat_per_sm;
-    }
-  }
-  const int blocks = (int)std::min<int64_t>(nbricks, (int64_t)sms * std::max(per_sm, 1));
-  mark_main_start(st);
-  kernel<<<blocks, kThreads, smem, st>>>(g, bg, ncomp, L.counts, static_cast<const long long *>(L.rec), L.qi,
-                                         L.qe, L.ebrick, wexp, field, T(beta), beta == 0.0);
-  mark_main_stop(st);
-  note_launch();
-  GBG_CUDA_TRY(cudaGetLastError());
-  return GBG_OK;
+  // three components share a point's weights and its trip; other counts go one at a time
+  return ncomp % 3 == 0 ? launch_owner<T, N2, 3>(g, P, ncomp, wexp, L, field, beta, st)
+                        : launch_owner<T, N2, 1>(g, P, ncomp, wexp, L, field, beta, st);
 }
 
-
-// The deterministic scatter.  The brick push (128-bit integer sums, FP64-grade per node)
-// whenever every axis is at least a stencil wide and a brick's accumulators fit in shared
-// memory; otherwise the node pull (points sorted by cell, one thread per node summing its
-// contributions in T in a fixed order), which also takes a stencil wider than the grid.
+// The deterministic scatter.  The brick scatter (integer sums, FP64-grade per node)
+// whenever every axis is at least a stencil wide; otherwise the node pull (points sorted by
+// cell, one thread per node summing its contributions in T in a fixed order), which also takes
+// a stencil wider than the grid.
 template <typename T>
 gbg_status dispatch_scatter(const gbg_grid &grid, const gbg_scheme &sch, int ncomp, void *field,
                             const void *pos, int64_t m, const void *q, double alpha, double beta,

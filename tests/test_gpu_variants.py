@@ -41,3 +41,103 @@ def test_traversal_validation_counts_every_entry(gbg, dev, m):
         twice[0] = twice[m - 1]
         with pytest.raises(gbg.ArgumentError, match="names %d of %d" % (m - 1, m)):
             gbg.PointTraversalOrder(torch.from_numpy(twice).to(dev))
+
+
+def _contribution_sizes(coef, n, pos, q, spacing):
+    """Per node the sums over its contributions of |w1 w2 w3 q| and of |q|."""
+    width, powers = coef.shape
+    ci = pos / spacing
+    base = np.floor(ci).astype(np.int64)
+    t = ci - base
+    w = np.zeros(pos.shape + (width,))
+    for p in range(powers - 1, -1, -1):
+        w = w * t[..., None] + coef[:, p]
+    w = np.abs(w)
+    out, reach = np.zeros(tuple(n) + (q.shape[1],)), np.zeros(tuple(n) + (q.shape[1],))
+    for k in range(width):
+        for j in range(width):
+            for i in range(width):
+                at = [(base[:, d] - (width // 2 - 1) + s) % n[d] for d, s in enumerate((i, j, k))]
+                wt = w[:, 0, i] * w[:, 1, j] * w[:, 2, k]
+                for c in range(q.shape[1]):
+                    np.add.at(out[..., c], tuple(at), wt * np.abs(q[:, c]))
+                    np.add.at(reach[..., c], tuple(at), np.abs(q[:, c]))
+    return out, reach
+
+
+# grids of one brick, of bricks with a last cell of one, and of axes no longer than the stencil; point
+# counts below, at and above one staging (508 points of a brick's region); quantities of one size and
+# spread over many windows of digits, region by region and point by point
+@pytest.mark.parametrize("n,m", [((8, 8, 4), 300), ((8, 8, 4), 509), ((9, 17, 5), 4000), ((25, 9, 13), 20_000),
+                                 ((8, 25, 33), 60)])
+@pytest.mark.parametrize("width,comps", [(2, 3), (4, 1), (4, 3), (4, 2), (6, 9), (8, 3)])
+@pytest.mark.parametrize("spread", [0, 14, 45])
+def test_fp64_scatter_per_node(gbg, oracle, dev, n, m, width, comps, spread):
+    n = tuple(max(v, width) for v in n)
+    rng = np.random.default_rng(1000 * width + m + spread)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    pos = TWO_PI * rng.random((m, 3))
+    pos[: m // 4] = pos[0] + 1e-3 * rng.random((m // 4, 3))  # a crowded cell
+    q = rng.standard_normal((m, comps)) * 10.0 ** (-spread * rng.random((m, 1)))
+    q[rng.random(m) < 0.05] = 0.0
+    pos, q = np.asfortranarray(pos), np.asfortranarray(q)
+    scheme = gbg.LalescuSpline(width)
+    old = np.asfortranarray(rng.standard_normal(n + (comps,)))
+    got = _scatter_abi(gbg, grid, dev, old, pos, q, scheme, 0.75, -0.5)
+    # the deposit by the oracle, then beta * old (the oracle's own adds onto beta * old would each round there)
+    want = oracle.scatter(g, np.zeros(n + (comps,), order="F"), pos, q, scheme.coefficients, alpha=0.75) - 0.5 * old
+    size, reach = _contribution_sizes(np.asarray(scheme.coefficients), n, pos, q, TWO_PI / np.array(n))
+    # the path's bar for a node (1e-12 of its own contributions), the unit of a node's fixed-point weight
+    # (2^(128 - 3 P), P >= 61, a few of them) for each point, and the roundings of beta * old and the sum
+    assert np.all(np.abs(got - want) <= 0.75 * (1e-12 * size + 4 * 2.0 ** -55 * reach) + 4e-16 * np.abs(old))
+    again = _scatter_abi(gbg, grid, dev, old, pos[::-1], q[::-1], scheme, 0.75, -0.5)
+    assert np.array_equal(got, again)  # integers: the points' order is no matter
+
+
+def _scatter_abi(gbg, grid, dev, old, pos, q, scheme, alpha, beta):
+    """gbg_anterpolate for any number of components."""
+    from gbgperiodicfields_gb300 import _lib
+    f, x, v = (to_dev(np.asfortranarray(a), dev) for a in (old, pos, q))
+    st = _lib.load().gbg_anterpolate(grid.c(), _lib.GBG_F64 if f.dtype == torch.float64 else _lib.GBG_F32, q.shape[1],
+                                     f.data_ptr(), x.data_ptr(), q.shape[0], v.data_ptr(), None, scheme.c(), alpha, beta,
+                                     None, 0, None, torch.cuda.current_stream().cuda_stream)
+    _lib.check(st, "scatter")
+    torch.cuda.synchronize()
+    return f.cpu().numpy()
+
+
+@pytest.mark.parametrize("comps", [1, 3])
+@pytest.mark.parametrize("spread", [0, 20])
+def test_fp32_scatter_windows(gbg, oracle, dev, comps, spread):
+    n, m = (25, 9, 13), 5000
+    rng = np.random.default_rng(comps + spread)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, dtype=torch.float32)
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin, dtype=np.float32)
+    pos = np.asfortranarray((TWO_PI * rng.random((m, 3))).astype(np.float32))
+    q = np.asfortranarray((rng.standard_normal((m, comps)) * 10.0 ** (-spread * rng.random((m, 1)))).astype(np.float32))
+    zero = np.zeros(n + (comps,), np.float32, order="F")
+    got = _scatter_abi(gbg, grid, dev, zero, pos, q, gbg.CatmullRom, 1.0, 0.0)
+    want = oracle.scatter(g, zero.copy(order="F"), pos, q, gbg.CatmullRom.coefficients)
+    assert relerr(got, want) <= 2e-5
+
+
+def test_fp64_scatter_marks_what_a_nan_reaches(gbg, oracle, dev):
+    n, m = (20, 16, 12), 3000
+    rng = np.random.default_rng(5)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    pos = np.asfortranarray(TWO_PI * rng.random((m, 3)))
+    q = np.asfortranarray(rng.standard_normal((m, 3)))
+    q[17, 1], q[40, 2] = np.nan, np.inf
+    zero = np.zeros(n + (3,), order="F")
+    got = _scatter_abi(gbg, grid, dev, zero, pos, q, gbg.CatmullRom, 1.0, 0.0)
+    clean = q.copy(order="F")
+    clean[17, 1] = clean[40, 2] = 0.0
+    want = oracle.scatter(g, zero.copy(order="F"), pos, clean, gbg.CatmullRom.coefficients)
+    base = np.floor(pos / (TWO_PI / np.array(n))).astype(int)
+    reach = np.zeros(n + (3,), bool)
+    for p, c in ((17, 1), (40, 2)):
+        reach[np.ix_(*[(base[p, d] - 1 + np.arange(4)) % n[d] for d in range(3)], [c])] = True
+    assert np.array_equal(np.isnan(got), reach)
+    assert np.abs(got - want)[~reach].max() <= 1e-13 * np.abs(want).max()
