@@ -1185,6 +1185,37 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Shared loads by 32-bit shared address.
+__device__ __forceinline__ float lds_f32(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+// Four floats as two pairs, as fma_pair takes them.
+__device__ __forceinline__ void lds_pairs(uint32_t a, unsigned long long &lo, unsigned long long &hi) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(a));
+}
+__device__ __forceinline__ unsigned long long pair_of(float x, float y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ void of_pair(unsigned long long v, float &x, float &y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+// Two fused multiply-adds in one instruction, each rounded as fmaf rounds it (the same rate as two
+// fmaf, half the issue slots).
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+
 // One compensated step (Knuth's TwoSum, every operation rounded on its own): s + x into
 // the pair (s, c), c collecting the exact rounding error of each addition.
 __device__ __forceinline__ void twosum_add(float &s, float &c, float x) {
@@ -1235,9 +1266,8 @@ __device__ __forceinline__ void weights_rt(const float *c, int m2, float t, floa
 
 // Shared memory of one scatter CTA, in this order: the brick's running sums (CP floats per
 // node), one chunk of the region's points (CP quantities and 3*N2+4 weights each), the
-// region's per-cell point offsets (+ the total) and first slots, the per-axis key tables
-// of the region's cells (this brick's, then the next brick's), and the points' region x
-// cells.  (With compensation, a region of several chunks keeps its sums' corrections in the
+// region's per-cell point offsets (+ the total) and first slots, and the per-axis key tables
+// of the region's cells (this brick's, then the next brick's).  (With compensation, a region of several chunks keeps its sums' corrections in the
 // CTA's own slot of a global scratch; the next brick's cell table, copied ahead, uses the
 // free end of the staging area.)
 size_t scatter_nodes_fixed(const FixGeo &g, int cp) {
@@ -1247,28 +1277,37 @@ size_t scatter_nodes_fixed(const FixGeo &g, int cp) {
 }
 
 // Floats of weights per staged point: the N2 x weights, then the y and the z weights each
-// with a zero on either side (so that a node's index past the stencil reads a zero),
-// rounded up to an odd count: lanes reading the same weight of different points then
+// with a zero on either side (so that a node's index past the stencil reads a zero), then the
+// point's region x cell (an integer's bits): 3 N2 + 5, an odd count for the even N2: lanes reading the same weight of different points then
 // fall in different banks (an even stride such as 16 would put 32 lanes in 2 banks).
 template <int N2>
-constexpr int kScatterWStride = (3 * N2 + 4) | 1;
-inline int scatter_wstride(int n2) { return (3 * n2 + 4) | 1; }
+constexpr int kScatterWStride = 3 * N2 + 5;
+inline int scatter_wstride(int n2) { return 3 * n2 + 5; }
 
 size_t scatter_nodes_smem(const FixGeo &g, int cp, int n2) {
-  return scatter_nodes_fixed(g, cp) + sizeof(float) * (size_t)g.chunk * (cp + scatter_wstride(n2)) + (size_t)g.chunk1;
+  return scatter_nodes_fixed(g, cp) + sizeof(float) * (size_t)g.chunk * (cp + scatter_wstride(n2));
 }
 
 // Sets the chunk sizes: the largest chunk (a multiple of 4, 64..1024 points) whose CTA
 // fits in `budget` bytes, and the larger one that also takes the running sums' space when
 // the whole region fits in one chunk.
 void scatter_nodes_chunk(FixGeo &g, int cp, int n2, size_t budget) {
-  const size_t per = sizeof(float) * (cp + scatter_wstride(n2)) + 1, fixed = scatter_nodes_fixed(g, cp);
+  const size_t per = sizeof(float) * (cp + scatter_wstride(n2)), fixed = scatter_nodes_fixed(g, cp);
   const size_t fit = budget > fixed ? (budget - fixed) / per : 0;
   g.chunk = (int32_t)std::max<size_t>(64, std::min<size_t>(1024, fit & ~size_t(3)));
   g.chunk1 = g.chunk + (int32_t)(((size_t)g.bvol * cp * sizeof(float) / per) & ~size_t(3));
 }
 
-// Shared memory per scatter CTA: half an SM's (two CTAs per SM) less the block's reserved
+// Scatter CTAs per SM that registers and shared memory are shared out for.  The setup of a brick is a
+// chain of short phases with barriers between them, so a third CTA pays where a region still fits
+// one staging: width 4 or less and four components (256^3 x 3, 6e6 points: 1.80 ms with two, 1.53 with
+// three, 1.99 with four; at width 6 a region of 644 points takes two stagings and 128^3 x 3 goes from
+// 388 to 648 us).
+constexpr int scatter_ctas(int n2, int cp) { return cp == 4 && n2 <= 4 ? 3 : 2; }
+template <int N2, int CP>
+constexpr int kScatterCtas = scatter_ctas(N2, CP);
+
+// Shared memory per scatter CTA: its share of an SM's less the block's reserved
 // and static share, or more when a region of 512 points would not fit one chunk (a brick's
 // region holds a few hundred at the usual densities, and each extra chunk re-stages and
 // re-walks the rows; a single chunk may also use the running sums' space).  It depends on
@@ -1276,10 +1315,10 @@ void scatter_nodes_chunk(FixGeo &g, int cp, int n2, size_t budget) {
 // compensated summation folds its partial sums, so the same chunks for every launch keep
 // the results bitwise independent of the threads per CTA and of batching.
 size_t scatter_nodes_budget(const FixGeo &g, int cp, int n2) {
-  const size_t per = sizeof(float) * (cp + scatter_wstride(n2)) + 1;
+  const size_t per = sizeof(float) * (cp + scatter_wstride(n2));
   const size_t sums = sizeof(float) * (size_t)g.bvol * cp;
   const size_t want = scatter_nodes_fixed(g, cp) + (512 * per > sums ? 512 * per - sums : 0) + 4 * per;
-  const size_t half = 228 * 1024 / 2 - 4096;
+  const size_t half = 228 * 1024 / scatter_ctas(n2, cp) - 4096;
   return want <= half ? half : std::min<size_t>(200 * 1024, 228 * 1024 - 4096);
 }
 
@@ -1328,7 +1367,6 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
   uint32_t *r0s = off + ecount + 1;
   uint32_t *kx = r0s + ecount, *ky = kx + E0, *kz = ky + E1;
   uint32_t *knx = kz + E2;  // the next brick's per-axis key tables (same layout)
-  unsigned char *scx = reinterpret_cast<unsigned char *>(knx + E0 + E1 + E2);
   // the next brick's cell table, copied by cp.async while this brick computes: the last
   // 2 * ecount words of the staging area (first slots, then ends)
   uint32_t *pre_a = off - 2 * ecount, *pre_z = off - ecount;
@@ -1559,8 +1597,8 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
         const uint32_t t = t0 + u * blockDim.x;
         if (t >= c1) break;
         const int tl = (int)(t - c0);
-        scx[tl] = (unsigned char)(cell[u] % E0);
         float *wt = sw + tl * kScatterWStride<N2>;
+        wt[3 * N2 + 4] = __uint_as_float((uint32_t)(cell[u] % E0));
         float w[N2];
         if constexpr (FIXED) weights_ptr<N2>(coef, r[u].x, w); else weights_rt<N2>(coef, m2, r[u].x, w);
 #pragma unroll
@@ -1590,7 +1628,6 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
       for (uint32_t t = threadIdx.x; t < count; t += blockDim.x) {
         const uint32_t sl = sorted_s[t];
         const float4 r = __ldg(rec + sl);
-        scx[t] = (unsigned char)(sorted_e[t] % (uint32_t)E0);
         float *wt = sw + t * kScatterWStride<N2>;
         float w[N2];
         if constexpr (FIXED) weights_ptr<N2>(coef, r.x, w); else weights_rt<N2>(coef, m2, r.x, w);
@@ -1641,7 +1678,8 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
       cp_async_commit();
       issued = true;
     }
-    for (int qi = threadIdx.x; qi < nquads; qi += blockDim.x) {
+    // whole warps (their trips below are taken together); a quad past the last owns no node
+    for (int qi = threadIdx.x; qi - (int)(threadIdx.x & 31) < nquads; qi += blockDim.x) {
       const int lx = qi % B0, ly = ((qi / B0) % QY) * BY, lz = (qi / (B0 * QY)) * BZ;
       float acc[BY * BZ][CP];
 #pragma unroll
@@ -1702,19 +1740,91 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
         // lane's trip count is its quad's number of points, not a count per row.
         const int ebase = (lz * E1 + ly) * E0 + lx;
         unsigned long long rows = 0;
+        if (qi < nquads) {
 #pragma unroll
-        for (int kk = 0; kk < RZ; ++kk)
+          for (int kk = 0; kk < RZ; ++kk)
 #pragma unroll
-          for (int jj = 0; jj < RY; ++jj)
-            if (ly + jj < E1 && lz + kk < E2) {
-              const int e0 = ebase + kk * slab + jj * E0;
-              if (max(off[e0], c0) < min(off[e0 + N2], c1)) rows |= 1ull << (kk * 8 + jj);
+            for (int jj = 0; jj < RY; ++jj)
+              if (ly + jj < E1 && lz + kk < E2) {
+                const int e0 = ebase + kk * slab + jj * E0;
+                if (max(off[e0], c0) < min(off[e0 + N2], c1)) rows |= 1ull << (kk * 8 + jj);
+              }
+        }
+        if constexpr (CP > 4) {
+          const uint32_t weights = smem_addr(sw), quantities = smem_addr(sq);
+          uint32_t wp = 0, wx = 0, wy = 0, wz = 0, qp = 0;  // the point's record, its weights, its quantities
+          int left = 0, jj = 0, kk = 0;
+          auto next_row = [&]() {
+            const int s = __ffsll((long long)rows) - 1;
+            rows &= rows - 1;
+            kk = s >> 3;
+            jj = s & 7;
+            const int e0 = ebase + kk * slab + jj * E0;
+            const uint32_t p0 = max(off[e0], c0);
+            left = (int)(min(off[e0 + N2], c1) - p0);
+            const uint32_t tl = p0 - c0;
+            qp = quantities + tl * (CP * 4);
+            wp = weights + tl * (kScatterWStride<N2> * 4) + 4 * (3 * N2 + 4);
+            wx = wp - 4 * (3 * N2 + 4) + 4 * (lx + N2 - 1);
+            wy = wp - 4 * (N2 + 4 + jj);  // y weight of node ly (padded; +4 for node ly+1)
+            wz = wp - 4 * (2 + kk);       // z weight of node lz (padded; +4 for node lz+1)
+          };
+          // Twelve components: pairs of multiply-adds (24 issue slots a point instead of 48, the same bits),
+          // and trips that are the warp's, held together by the vote: each takes one point of every lane
+          // that has one left, and a lane whose row is done moves on within the trip.  512^3 x 12, 3.2e7
+          // points: 10.35 ms, 11.85 with the loop below.  With four components the loop below wins (128^3 x
+          // 3, 5e5 points, width 6: 336 us, 387 this way): a point's 16 multiply-adds are too few to pay for
+          // the pairs' weights and the vote.
+          unsigned long long acc2[BY * BZ][CP / 2];
+#pragma unroll
+          for (int n = 0; n < BY * BZ; ++n)
+#pragma unroll
+            for (int c = 0; c < CP / 2; ++c) acc2[n][c] = pair_of(acc[n][2 * c], acc[n][2 * c + 1]);
+          auto trips = [&](auto reach_only) {
+            auto trip = [&]() {
+              unsigned long long q[CP / 2];
+#pragma unroll
+              for (int v = 0; v < CP / 4; ++v) lds_pairs(qp + 16 * v, q[2 * v], q[2 * v + 1]);
+              const float x = lds_f32(wx - 4 * lds_u32(wp));
+              float y[BY], z[BZ];
+#pragma unroll
+              for (int a = 0; a < BY; ++a) y[a] = x * lds_f32(wy + 4 * a);
+#pragma unroll
+              for (int bb = 0; bb < BZ; ++bb) z[bb] = lds_f32(wz + 4 * bb);
+#pragma unroll
+              for (int n = 0; n < BY * BZ; ++n) {
+                if constexpr (decltype(reach_only)::value) {
+                  const int a = n % BY, bb = n / BY;
+                  if (!(jj - a >= 0 && jj - a <= N2 - 1 && kk - bb >= 0 && kk - bb <= N2 - 1)) continue;
+                }
+                const float wgt = y[n % BY] * z[n / BY];
+                const unsigned long long w2 = pair_of(wgt, wgt);
+#pragma unroll
+                for (int c = 0; c < CP / 2; ++c) acc2[n][c] = fma_pair(w2, q[c], acc2[n][c]);
+              }
+              wp += kScatterWStride<N2> * 4;
+              wx += kScatterWStride<N2> * 4;
+              wy += kScatterWStride<N2> * 4;
+              wz += kScatterWStride<N2> * 4;
+              qp += CP * 4;
+            };
+            if (rows) next_row();
+            while (__any_sync(0xffffffffu, left > 0)) {
+              if (left > 0) {
+                trip();
+                if (--left == 0 && rows) next_row();
+              }
             }
-        if (rows) {
+          };
+          if (exact) trips(std::true_type{}); else trips(std::false_type{});
+#pragma unroll
+          for (int n = 0; n < BY * BZ; ++n)
+#pragma unroll
+            for (int c = 0; c < CP / 2; ++c) of_pair(acc2[n][c], acc[n][2 * c], acc[n][2 * c + 1]);
+        } else if (rows) {
           const int xk = lx + N2 - 1;
           const float *wp = nullptr, *wy = nullptr, *wz = nullptr;
           const float4 *qp = nullptr;
-          const unsigned char *xp = nullptr;
           uint32_t left = 0;
           int jj = 0, kk = 0;
           auto next_row = [&]() {
@@ -1730,12 +1840,11 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
             wy = wp + (2 * N2 - jj);      // y weight of node ly (padded; +1 for node ly+1)
             wz = wp + (3 * N2 + 2 - kk);  // z weight of node lz (padded; +1 for node lz+1)
             qp = reinterpret_cast<const float4 *>(sq) + tl * (CP / 4);
-            xp = scx + tl;
           };
           next_row();
           if (!exact) {
             while (true) {
-              const float wx = wp[xk - (int)*xp];
+              const float wx = wp[xk - (int)__float_as_uint(wp[3 * N2 + 4])];
               float q[CP];
 #pragma unroll
               for (int v = 0; v < CP / 4; ++v) {
@@ -1755,7 +1864,6 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
               wy += kScatterWStride<N2>;
               wz += kScatterWStride<N2>;
               qp += CP / 4;
-              ++xp;
               if (--left == 0) {
                 if (!rows) break;
                 next_row();
@@ -1763,7 +1871,7 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
             }
           } else {
             while (true) {
-              const float wx = wp[xk - (int)*xp];
+              const float wx = wp[xk - (int)__float_as_uint(wp[3 * N2 + 4])];
               float q[CP];
 #pragma unroll
               for (int v = 0; v < CP / 4; ++v) {
@@ -1787,7 +1895,6 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
               wy += kScatterWStride<N2>;
               wz += kScatterWStride<N2>;
               qp += CP / 4;
-              ++xp;
               if (--left == 0) {
                 if (!rows) break;
                 next_row();
@@ -1851,7 +1958,7 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
 }
 
 template <int N2, bool FIXED, int CP>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, kScatterCtas<N2, CP>)
     k_scatter_nodes(FixGeo g, SchemeT<float, N2> s, const uint32_t *__restrict__ cell_start,
                     const float4 *__restrict__ rec, const float *__restrict__ qs,
                     const unsigned *__restrict__ qmax_bits, float *__restrict__ field, float beta,
