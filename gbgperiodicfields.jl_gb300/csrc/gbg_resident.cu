@@ -641,6 +641,93 @@ __device__ __forceinline__ void brick_coords(const StagedGeo &g, int64_t b, int6
   bz = b / (g.nb[0] * g.nb[1]);
 }
 
+// The CP sums of a point over its eight lanes, stored: halves by lane bit 2, then bit 1, then the sum of
+// bit 0.
+template <int CP, typename TO>
+__device__ __forceinline__ void reduce_store(const float (&acc)[CP], int sub, unsigned seg_mask, int64_t pt, TO *out,
+                                             int64_t m, int ncomp) {
+  constexpr int H = CP / 2, Q = CP / 4;
+  const bool up2 = sub & 4, up1 = sub & 2;
+  float h[H];
+#pragma unroll
+  for (int v = 0; v < H; ++v) {
+    const float keep = up2 ? acc[H + v] : acc[v];
+    const float give = up2 ? acc[v] : acc[H + v];
+    h[v] = keep + __shfl_xor_sync(seg_mask, give, 4, 8);
+  }
+  float qv[Q];
+#pragma unroll
+  for (int v = 0; v < Q; ++v) {
+    const float keep = up1 ? h[Q + v] : h[v];
+    const float give = up1 ? h[v] : h[Q + v];
+    qv[v] = keep + __shfl_xor_sync(seg_mask, give, 2, 8);
+  }
+#pragma unroll
+  for (int v = 0; v < Q; ++v) qv[v] += __shfl_xor_sync(seg_mask, qv[v], 1, 8);
+  if ((sub & 1) == 0) {
+    const int cbase = (up2 ? H : 0) + (up1 ? Q : 0);
+#pragma unroll
+    for (int v = 0; v < Q; ++v)
+      if (cbase + v < ncomp) store_out(out, pt + m * (cbase + v), qv[v]);
+  }
+}
+
+// Horner for this lane's node of a width-N2 stencil from its column of coefficients (the roundings of
+// weights_all).
+template <int M2>
+__device__ __forceinline__ float column_weight(const float (&c)[M2], float t) {
+  float w = c[M2 - 1];
+#pragma unroll
+  for (int p = M2 - 2; p >= 0; --p) w = fmaf(w, t, c[p]);
+  return w;
+}
+
+// One point of a width-6 or width-8 gather by its quarter-warp, given this lane's three weights: lane i
+// takes the x node i of every row (lanes past the stencil read the last node and count for nothing),
+// contracts y and then z with the weights of the other lanes, and the x weight comes last.  A row is
+// one contiguous read of its lanes -- no bank conflicts in a tile, whole sectors in the field -- and a
+// node costs CP multiply-adds.  Bound by the shared loads (36 reads of 128 bytes a point at width 6,
+// six of eight lanes in use; 64% of their peak) and by blobs' bricks falling unevenly on the SMs: 256^3
+// x 3, 4e6 points, width 6: 0.80 ms, 0.93 with a thread per point, whose reads met 2.5 at a bank.  The
+// nodes are base[(origin + x + y*sy + z*sz) * CP], in a tile or in
+// the field, with the same bits.
+template <int N2, int CP, typename TO, typename I>
+__device__ __forceinline__ void gather_rows_point(float w1, float w2, float w3, int sub, unsigned seg_mask, float4 r,
+                                                  int64_t pt, const float *base, I sy, I sz, I origin, TO *out,
+                                                  int64_t m, int ncomp) {
+  int lx, ly, lz;
+  unpack_local(r.w, lx, ly, lz);
+  float wy[N2];
+#pragma unroll
+  for (int j = 0; j < N2; ++j) wy[j] = __shfl_sync(seg_mask, w2, j, 8);
+  float acc[CP];
+#pragma unroll
+  for (int c = 0; c < CP; ++c) acc[c] = 0.0f;
+  const float *row = base + (origin + lz * sz + ly * sy + lx + min(sub, N2 - 1)) * CP;
+#pragma unroll
+  for (int k = 0; k < N2; ++k) {
+    const float wz = __shfl_sync(seg_mask, w3, k, 8);
+    float s[CP];
+#pragma unroll
+    for (int j = 0; j < N2; ++j) {
+      const float4 *p = reinterpret_cast<const float4 *>(row + (k * sz + j * sy) * CP);
+#pragma unroll
+      for (int q4 = 0; q4 < CP / 4; ++q4) {
+        const float4 v = p[q4];
+        s[4 * q4 + 0] = j ? fmaf(wy[j], v.x, s[4 * q4 + 0]) : wy[0] * v.x;
+        s[4 * q4 + 1] = j ? fmaf(wy[j], v.y, s[4 * q4 + 1]) : wy[0] * v.y;
+        s[4 * q4 + 2] = j ? fmaf(wy[j], v.z, s[4 * q4 + 2]) : wy[0] * v.z;
+        s[4 * q4 + 3] = j ? fmaf(wy[j], v.w, s[4 * q4 + 3]) : wy[0] * v.w;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CP; ++c) acc[c] = fmaf(wz, s[c], acc[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < CP; ++c) acc[c] = sub < N2 ? w1 * acc[c] : 0.0f;
+  reduce_store<CP>(acc, sub, seg_mask, pt, out, m, ncomp);
+}
+
 // One point of a width-4 gather by its quarter-warp: this lane's x node qi and y nodes
 // 2jj, 2jj+1 over all four z nodes, then a reduce-scatter of the CP sums over the eight
 // lanes.  The nodes are base[(origin + x + y*sy + z*sz) * CP] at stencil-relative
@@ -695,41 +782,17 @@ __device__ __forceinline__ void gather4_point(const SchemeT<float, 4> &s, const 
       }
     }
   }
-  // reduce-scatter over the 8 lanes: halves by lane bit 2, then bit 1, then sum bit 0
-  constexpr int H = CP / 2, Q = CP / 4;
-  const bool up2 = sub & 4, up1 = sub & 2;
-  float h[H];
-#pragma unroll
-  for (int v = 0; v < H; ++v) {
-    const float keep = up2 ? acc[H + v] : acc[v];
-    const float give = up2 ? acc[v] : acc[H + v];
-    h[v] = keep + __shfl_xor_sync(seg_mask, give, 4, 8);
-  }
-  float qv[Q];
-#pragma unroll
-  for (int v = 0; v < Q; ++v) {
-    const float keep = up1 ? h[Q + v] : h[v];
-    const float give = up1 ? h[v] : h[Q + v];
-    qv[v] = keep + __shfl_xor_sync(seg_mask, give, 2, 8);
-  }
-#pragma unroll
-  for (int v = 0; v < Q; ++v) qv[v] += __shfl_xor_sync(seg_mask, qv[v], 1, 8);
-  if ((sub & 1) == 0) {
-    const int cbase = (up2 ? H : 0) + (up1 ? Q : 0);
-#pragma unroll
-    for (int v = 0; v < Q; ++v)
-      if (cbase + v < ncomp) store_out(out, pt + m * (cbase + v), qv[v]);
-  }
+  reduce_store<CP>(acc, sub, seg_mask, pt, out, m, ncomp);
 }
 
-// Gather: width-4 stencils, a point per quarter-warp, 512 threads (64 quarter-warps) per
+// Gather: a point per quarter-warp (widths 4, 6 and 8), 512 threads (64 quarter-warps) per
 // CTA; each quarter-warp loads its next point's record and index while it computes.  With
 // two tile buffers the warps run free of CTA barriers (the warp that releases a buffer last
 // refills it); with one (a large tile, two CTAs per SM) the CTA waits at each brick.
 constexpr int kGatherThreads = 512;
-template <int M2, int CP, typename TO>
+template <int N2, int M2, int CP, typename TO>
 __global__ void __launch_bounds__(kGatherThreads, 1)
-    k_gather_staged4(const __grid_constant__ CUtensorMap tmap, StagedGeo g, SchemeT<float, 4> s,
+    k_gather_staged(const __grid_constant__ CUtensorMap tmap, StagedGeo g, SchemeT<float, N2> s,
                      const uint32_t *__restrict__ cell_start, const float4 *__restrict__ rec,
                      const uint32_t *__restrict__ perm, TO *__restrict__ out, int32_t *status, int nbuf,
                      uint32_t tile_bytes, uint32_t box_bytes, const uint32_t *__restrict__ list,
@@ -746,16 +809,39 @@ __global__ void __launch_bounds__(kGatherThreads, 1)
   const int qi = sub & 3, jj = sub >> 2;
   const unsigned seg_mask = 0xFFu << (lane & ~7);
   const int qw = threadIdx.x >> 3;  // quarter-warp id within the CTA
-  // this lane's coefficient columns (x node qi, y nodes 2jj and 2jj+1), fixed for the launch
+  // this lane's coefficient columns, fixed for the launch (width 4: x node qi, y nodes 2jj and 2jj+1;
+  // else node sub of every axis)
   float cx[M2 > 0 ? M2 : 1], cya[M2 > 0 ? M2 : 1], cyb[M2 > 0 ? M2 : 1];
   if constexpr (M2 > 0) {
 #pragma unroll
     for (int p = 0; p < M2; ++p) {
-      cx[p] = s.c[qi + 4 * p];
-      cya[p] = s.c[2 * jj + 4 * p];
-      cyb[p] = s.c[2 * jj + 1 + 4 * p];
+      if constexpr (N2 == 4) {
+        cx[p] = s.c[qi + 4 * p];
+        cya[p] = s.c[2 * jj + 4 * p];
+        cyb[p] = s.c[2 * jj + 1 + 4 * p];
+      } else {
+        cx[p] = s.c[min(sub, N2 - 1) + N2 * p];
+      }
     }
   }
+  auto point = [&](const float4 &r, int64_t p, const float *tile) {
+    if constexpr (N2 == 4) {
+      gather4_point<M2, CP>(s, cx, cya, cyb, qi, jj, sub, seg_mask, r, p, tile, g.w[0], g.w[0] * g.w[1], 0, out, g.m,
+                            g.ncomp);
+    } else {
+      float w1, w2, w3;
+      if constexpr (M2 > 0) {
+        w1 = column_weight<M2>(cx, r.x);
+        w2 = column_weight<M2>(cx, r.y);
+        w3 = column_weight<M2>(cx, r.z);
+      } else {
+        w1 = poly<N2>(s, min(sub, N2 - 1), r.x);
+        w2 = poly<N2>(s, min(sub, N2 - 1), r.y);
+        w3 = poly<N2>(s, min(sub, N2 - 1), r.z);
+      }
+      gather_rows_point<N2, CP>(w1, w2, w3, sub, seg_mask, r, p, tile, g.w[0], g.w[0] * g.w[1], 0, out, g.m, g.ncomp);
+    }
+  };
   const int nqw = (int)blockDim.x / 8;
   uint32_t phase[2] = {0, 0};
   bool failed = false;
@@ -843,9 +929,7 @@ __global__ void __launch_bounds__(kGatherThreads, 1)
           p_next = __ldg(perm + a1 + qw);
           ahead = true;
         }
-        gather4_point<M2, CP>(s, cx, cya, cyb, qi, jj, sub, seg_mask, r, p,
-                              reinterpret_cast<const float *>(smem + buf * tile_bytes), g.w[0], g.w[0] * g.w[1], 0,
-                              out, g.m, g.ncomp);
+        point(r, p, reinterpret_cast<const float *>(smem + buf * tile_bytes));
       }
       if (!ahead && a1 + qw < z1) {
         r_next = __ldg(rec + a1 + qw);
@@ -923,9 +1007,7 @@ __global__ void __launch_bounds__(kGatherThreads, 1)
           p_next = __ldg(perm + n0 + qw);
           ahead = true;
         }
-        gather4_point<M2, CP>(s, cx, cya, cyb, qi, jj, sub, seg_mask, r, p,
-                              reinterpret_cast<const float *>(smem + buf * tile_bytes), g.w[0], g.w[0] * g.w[1], 0,
-                              out, g.m, g.ncomp);
+        point(r, p, reinterpret_cast<const float *>(smem + buf * tile_bytes));
       }
     }
     if (!ahead && n0 + qw < n1) {
@@ -945,7 +1027,7 @@ __global__ void __launch_bounds__(kGatherThreads, 1)
   }
 }
 
-// One point of a gather of another width, by one thread over its N2^3 stencil; the nodes
+// One point of a width-2 gather, by one thread over its N2^3 stencil; the nodes
 // are base[(origin + x + y*sy + z*sz) * CP] as for the width-4 gather.
 template <int N2, int M2, int CP, typename TO, typename I>
 __device__ __forceinline__ void gather_point(const SchemeT<float, N2> &s, float4 r, int64_t pt, const float *base, I sy,
@@ -989,7 +1071,7 @@ __device__ __forceinline__ void gather_point(const SchemeT<float, N2> &s, float4
     if (c < ncomp) store_out(out, pt + m * c, acc[c]);
 }
 
-// Gather for other widths: a point per thread over its N2^3 stencil in the tile.
+// Gather for width 2: a point per thread over its N2^3 stencil in the tile.
 template <int N2, int M2, int CP, typename TO>
 __global__ void __launch_bounds__(kThreads, 1)
     k_gather_staged_generic(const __grid_constant__ CUtensorMap tmap, StagedGeo g, SchemeT<float, N2> s,
@@ -1117,6 +1199,38 @@ __global__ void __launch_bounds__(kThreads)
     const int64_t pt = __ldg(perm + sl);
     const int64_t origin = direct_origin(g, px, py, __ldg(keys + pt));
     gather4_point<M2, CP>(s, cx, cya, cyb, qi, jj, sub, seg_mask, r, pt, field, px, px * py, origin, out, g.m, g.ncomp);
+  }
+}
+
+// Widths 6 and 8, a quarter-warp per point as in the staged kernel.
+template <int N2, int M2, int CP, typename TO>
+__global__ void __launch_bounds__(kThreads)
+    k_gather_direct_rows(StagedGeo g, SchemeT<float, N2> s, const float *__restrict__ field, int64_t px, int64_t py,
+                         const float4 *__restrict__ rec, const uint32_t *__restrict__ perm,
+                         const uint32_t *__restrict__ keys, TO *__restrict__ out) {
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  const unsigned seg_mask = 0xFFu << (lane & ~7);
+  float c[M2 > 0 ? M2 : 1];
+  if constexpr (M2 > 0) {
+#pragma unroll
+    for (int p = 0; p < M2; ++p) c[p] = s.c[min(sub, N2 - 1) + N2 * p];
+  }
+  const int64_t nq = ((int64_t)gridDim.x * blockDim.x) >> 3;
+  for (int64_t sl = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; sl < g.m; sl += nq) {
+    const float4 r = __ldg(rec + sl);
+    const int64_t pt = __ldg(perm + sl);
+    const int64_t origin = direct_origin(g, px, py, __ldg(keys + pt));
+    float w1, w2, w3;
+    if constexpr (M2 > 0) {
+      w1 = column_weight<M2>(c, r.x);
+      w2 = column_weight<M2>(c, r.y);
+      w3 = column_weight<M2>(c, r.z);
+    } else {
+      w1 = poly<N2>(s, min(sub, N2 - 1), r.x);
+      w2 = poly<N2>(s, min(sub, N2 - 1), r.y);
+      w3 = poly<N2>(s, min(sub, N2 - 1), r.z);
+    }
+    gather_rows_point<N2, CP>(w1, w2, w3, sub, seg_mask, r, pt, field, px, px * py, origin, out, g.m, g.ncomp);
   }
 }
 
@@ -2032,7 +2146,7 @@ gbg_status launch_direct_gather(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme 
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t lanes = N2 == 4 ? 8 * b->npoints : b->npoints;  // a quarter-warp per width-4 point
+  const int64_t lanes = N2 >= 4 ? 8 * b->npoints : b->npoints;  // a quarter-warp per point, or a thread
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((lanes + kThreads - 1) / kThreads, (int64_t)sms * 8));
   mark_main_start(st);
   if constexpr (N2 == 4) {
@@ -2040,6 +2154,11 @@ gbg_status launch_direct_gather(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme 
       k_gather_direct4<M2, 4, TO><<<blocks, kThreads, 0, st>>>(g, s, f->data, f->px, f->py, b->rec, b->perm, b->keys, out);
     else
       k_gather_direct4<M2, 12, TO><<<blocks, kThreads, 0, st>>>(g, s, f->data, f->px, f->py, b->rec, b->perm, b->keys, out);
+  } else if constexpr (N2 > 4) {
+    if (f->cp == 4)
+      k_gather_direct_rows<N2, M2, 4, TO><<<blocks, kThreads, 0, st>>>(g, s, f->data, f->px, f->py, b->rec, b->perm, b->keys, out);
+    else
+      k_gather_direct_rows<N2, M2, 12, TO><<<blocks, kThreads, 0, st>>>(g, s, f->data, f->px, f->py, b->rec, b->perm, b->keys, out);
   } else {
     if (f->cp == 4)
       k_gather_direct<N2, M2, 4, TO><<<blocks, kThreads, 0, st>>>(g, s, f->data, f->px, f->py, b->rec, b->perm, b->keys, out);
@@ -2067,7 +2186,7 @@ gbg_status launch_staged_gather(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme 
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int threads = b->gather_threads ? b->gather_threads : (N2 == 4 ? kGatherThreads : kThreads);
+  const int threads = b->gather_threads ? b->gather_threads : (N2 >= 4 ? kGatherThreads : kThreads);
   auto go = [&](auto kernel) -> gbg_status {
     // Double-buffer the tile when that leaves as many CTAs per SM as a single buffer
     // would; otherwise (a large tile whose registers allow two CTAs) keep one buffer per
@@ -2094,9 +2213,9 @@ gbg_status launch_staged_gather(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme 
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;
   };
-  if constexpr (N2 == 4) {
-    if (f->cp == 4) return go(k_gather_staged4<M2, 4, TO>);
-    return go(k_gather_staged4<M2, 12, TO>);
+  if constexpr (N2 >= 4) {
+    if (f->cp == 4) return go(k_gather_staged<N2, M2, 4, TO>);
+    return go(k_gather_staged<N2, M2, 12, TO>);
   } else {
     if (f->cp == 4) return go(k_gather_staged_generic<N2, M2, 4, TO>);
     return go(k_gather_staged_generic<N2, M2, 12, TO>);
@@ -2528,6 +2647,18 @@ __device__ void batch_gather_points(const BatchDev *d, const float *tile, uint32
         for (int v = 0; v < Q; ++v)
           if (cbase + v < g.ncomp) d->out[p + g.m * (cbase + v)] = qv[v];
       }
+    }
+  } else if constexpr (N2 > 4) {
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    const unsigned seg_mask = 0xFFu << (lane & ~7);
+    float c[N2];
+#pragma unroll
+    for (int p = 0; p < N2; ++p) c[p] = d->coef[min(sub, N2 - 1) + N2 * p];
+    for (uint32_t sl = s0 + (threadIdx.x >> 3); sl < s1; sl += kBatchGatherThreads / 8) {
+      const float4 r = __ldg(d->rec + sl);
+      const int64_t p = __ldg(d->perm + sl);
+      gather_rows_point<N2, CP>(column_weight<N2>(c, r.x), column_weight<N2>(c, r.y), column_weight<N2>(c, r.z), sub,
+                                seg_mask, r, p, tile, g.w[0], g.w[0] * g.w[1], 0, d->out, g.m, g.ncomp);
     }
   } else {
     for (uint32_t sl = s0 + threadIdx.x; sl < s1; sl += kBatchGatherThreads) {

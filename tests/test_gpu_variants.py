@@ -141,3 +141,36 @@ def test_fp64_scatter_marks_what_a_nan_reaches(gbg, oracle, dev):
         reach[np.ix_(*[(base[p, d] - 1 + np.arange(4)) % n[d] for d in range(3)], [c])] = True
     assert np.array_equal(np.isnan(got), reach)
     assert np.abs(got - want)[~reach].max() <= 1e-13 * np.abs(want).max()
+
+
+# a quarter-warp per point at widths 6 and 8: a few points, a brick's points no multiple of the CTA's
+# quarter-warps, bricks with and without a second tile buffer, schemes with fewer powers than nodes
+@pytest.mark.parametrize("m", [1, 7, 65, 5000])
+@pytest.mark.parametrize("ncomp", [1, 3, 9, 12])
+@pytest.mark.parametrize("name", ["L6", "L6m1", "L8", "L8m2", "G8"])
+def test_wide_gather_staged_direct_and_batched(gbg, oracle, dev, m, ncomp, name):
+    from gbgperiodicfields_gb300 import resident
+    scheme = {"L6": gbg.LalescuSpline(6), "L6m1": gbg.LalescuSpline(6, 1), "L8": gbg.LalescuSpline(8),
+              "L8m2": gbg.LalescuSpline(8, 2), "G8": gbg.LagrangeSpline(8)}[name]
+    n = (19, 16, 21)
+    rng = np.random.default_rng(m + 100 * ncomp)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, origin=(0.5, -1.0, 2.0))
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    pos = np.asfortranarray(np.array(grid.origin) + TWO_PI * (rng.random((m, 3)) * 1.2 - 0.1))
+    f = np.asfortranarray(rng.standard_normal(n + (ncomp,)))
+    want = oracle.gather(g, f, pos, scheme.coefficients)
+    field = resident.ResidentField(grid, ncomp, max_stencil_width=8).load(to_dev(f, dev))
+    got = {}
+    for brick in ((19, 16, 21), (4, 4, 4), (11, 8, 8)):
+        # one brick of m points is staged, hundreds of bricks with few points each are read directly
+        if (brick[0] + 7) * (brick[1] + 7) * (brick[2] + 7) * (16 if ncomp <= 4 else 48) > 200 * 1024:
+            continue
+        bins = resident.PointBins(grid, m, brick=brick).build(to_dev(pos, dev))
+        got[brick] = resident.interpolate_binned(field, bins, scheme, dtype=torch.float32).cpu().numpy()
+        assert relerr(got[brick], want) <= 1e-5
+        if scheme.coefficients.shape[1] == scheme.stencil_width:
+            out = gbg.empty_colmajor((m, ncomp), torch.float32, dev)
+            resident.Batch([dict(field=field, bins=bins, scheme=scheme, out=out)]).run()
+            assert np.array_equal(out.cpu().numpy(), got[brick])
+    first = next(iter(got.values()))
+    assert all(np.array_equal(v, first) for v in got.values())
