@@ -174,3 +174,48 @@ def test_wide_gather_staged_direct_and_batched(gbg, oracle, dev, m, ncomp, name)
             assert np.array_equal(out.cpu().numpy(), got[brick])
     first = next(iter(got.values()))
     assert all(np.array_equal(v, first) for v in got.values())
+
+
+@pytest.mark.parametrize("ncomp", [1, 4, 5, 12])
+@pytest.mark.parametrize("n", [(8, 9, 33), (65, 8, 8), (31, 40, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_import_rows_and_ghosts(gbg, oracle, dev, ncomp, n, dtype):
+    # axes no longer than the widest stencil, rows below, at and above a warp's width
+    from gbgperiodicfields_gb300 import resident
+    rng = np.random.default_rng(ncomp + n[0])
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    f = np.asfortranarray(rng.standard_normal(n + (ncomp,)))
+    data = to_dev(f, dev).to(dtype)
+    field = resident.ResidentField(grid, ncomp, max_stencil_width=8).load(data)
+    assert torch.equal(field.read(torch.float32), data.float())
+    pos = np.asfortranarray(np.concatenate([TWO_PI * rng.random((200, 3)), TWO_PI * rng.integers(0, 2, (50, 3))]))
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    scheme = gbg.LalescuSpline(8)
+    got = resident.interpolate_binned(field, resident.PointBins(grid, 250).build(to_dev(pos, dev)), scheme)
+    assert relerr(got.cpu().numpy(), oracle.gather(g, f, pos, scheme.coefficients)) <= 1e-5
+
+
+@pytest.mark.parametrize("T", [np.float64, np.float32])
+@pytest.mark.parametrize("origin", [0.0, -0.75, 1e-3])
+def test_wrap_around_every_bound(gbg, oracle, dev, T, origin):
+    # coordinates a few units either side of every bound that the wrap decides at, and far beyond
+    L, o = T(TWO_PI), T(origin)
+    grid = gbg.Grid3D((8, 8, 8), (float(L),) * 3, origin=(origin,) * 3,
+                      dtype=torch.float64 if T is np.float64 else torch.float32)
+    at = [T(0), -T(0), L, -L, L + L, -(L + L), L / T(2), T(3) * L, T(1e6) * L]
+    tiny = np.finfo(T).tiny
+    xs = [T(v) for v in (np.inf, -np.inf, np.nan, tiny, -tiny, np.finfo(T).max, -np.finfo(T).max, 1e-30, -1e-30)]
+    for v in at:
+        for k in (-2, -1, 0, 1, 2):
+            w = v
+            for _ in range(abs(k)):
+                w = np.nextafter(w, T(np.inf) if k > 0 else T(-np.inf))
+            xs += [w, T(w + o)]
+    x = np.asfortranarray(np.stack([np.array(xs, T), np.array(xs[::-1], T), np.array(xs, T)], 1))
+    pts = gbg.PointSet(to_dev(x, dev))
+    gbg.wrap_(pts, grid)
+    want = oracle.displace(x, [], {"domain": grid.domain_size, "origin": grid.origin})
+    got = pts.positions.cpu().numpy()
+    assert np.array_equal(got.view(np.uint64 if T is np.float64 else np.uint32)[~np.isnan(want)],
+                          want.view(np.uint64 if T is np.float64 else np.uint32)[~np.isnan(want)])
+    assert np.array_equal(np.isnan(got), np.isnan(want))
