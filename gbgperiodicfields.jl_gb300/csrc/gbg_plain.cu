@@ -1360,11 +1360,10 @@ ScatterPlan plan_scatter(const gbg_grid &g, int ncomp, size_t esize, int n2) {
 // permutation, the scan's scratch, per slot the three axes' weights (64-bit fixed point for the
 // brick scatter) and the quantities (for the brick scatter as mantissas and exponents, with per
 // exponent brick the largest exponent of every component); for the pull also the stable sort's
-// scratch.  flag: the sort's long-run flag, or the brick scatter's ticket.
+// scratch.  flag: the sort's count of long runs, or the brick scatter's ticket.
 struct ScatterLayout {
   uint32_t *keys, *counts, *rank, *perm, *flag;
-  void *sort_tmp;
-  uint32_t *scan_tmp;
+  uint32_t *sort_tmp, *scan_tmp;
   void *rec, *qs;
   long long *qi;
   int16_t *qe;
@@ -1378,7 +1377,7 @@ ScatterLayout scatter_layout(Arena &a, int64_t m, const ScatterPlan &P, int ncom
   L.rank = a.take<uint32_t>((size_t)m);
   L.perm = a.take<uint32_t>((size_t)m);
   L.flag = a.take<uint32_t>(4);
-  L.sort_tmp = P.bricked ? nullptr : a.take<char>(radix_sort_temp_bytes(m));
+  L.sort_tmp = P.bricked ? nullptr : a.take<uint32_t>((size_t)m);
   L.scan_tmp = a.take<uint32_t>(scan_temp_elems(P.nkeys + 1));
   const size_t rec_bytes = 3 * (size_t)n2 * (P.bricked ? sizeof(long long) : esize);
   L.rec = a.take<char>((size_t)m * rec_bytes);
@@ -1487,8 +1486,7 @@ gbg_status dispatch_scatter(const gbg_grid &grid, const gbg_scheme &sch, int nco
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
   GBG_TRY(exclusive_scan_u32(L.counts, L.counts, ncells + 1, L.scan_tmp, st));
-  GBG_TRY(stable_counting_sort(L.keys, L.rank, L.counts, m, bits_for((uint64_t)(ncells - 1)), L.perm, L.rank,
-                               L.flag, L.sort_tmp, st));
+  GBG_TRY(stable_counting_sort(L.keys, L.rank, L.counts, m, L.perm, L.flag, L.sort_tmp, st));
   T *rec = static_cast<T *>(L.rec);
   T *qs = static_cast<T *>(L.qs);
   k_scatter_prep<T><<<launch_blocks(m, kThreads), kThreads, 0, st>>>(

@@ -55,10 +55,9 @@ struct gbg_bins_s {
   int32_t b[3] = {11, 8, 8};
   int64_t nb[3] = {0, 0, 0};
   int64_t nbricks = 0, bvol = 0, nkeys = 0;
-  uint32_t *keys = nullptr, *skeys = nullptr, *perm = nullptr, *cell_start = nullptr;
+  uint32_t *keys = nullptr, *rank = nullptr, *perm = nullptr, *cell_start = nullptr;
   float4 *rec_user = nullptr, *rec = nullptr;
-  void *sort_tmp = nullptr;
-  uint32_t *scan_tmp = nullptr;
+  uint32_t *sort_tmp = nullptr, *scan_tmp = nullptr;
   float *qs = nullptr;  // sorted, alpha-scaled quantities for the scatter (max_points x 12)
   unsigned *qmax_bits = nullptr;  // largest |alpha q| of the last scatter, as float bits
   void *block = nullptr;
@@ -84,18 +83,19 @@ namespace gbg {
 inline void bins_layout(Arena &a, gbg_bins_s *b) {
   const int64_t m = b->max_points > 0 ? b->max_points : 1;
   b->keys = a.take<uint32_t>(m);
-  b->skeys = a.take<uint32_t>(m);
+  b->rank = a.take<uint32_t>(m);
   b->perm = a.take<uint32_t>(m);
+  // the list lengths and the cells' counts are cleared together
+  b->lists_n = a.take<uint32_t>(64);
   b->cell_start = a.take<uint32_t>((size_t)b->nkeys + 1);
   b->rec_user = a.take<float4>(m);
   b->rec = a.take<float4>(m);
-  b->sort_tmp = a.take<char>(radix_sort_temp_bytes(m));
+  b->sort_tmp = a.take<uint32_t>(m);
   b->scan_tmp = a.take<uint32_t>(scan_temp_elems(b->nkeys + 1));
   b->qs = a.take<float>((size_t)m * 12);
   b->qmax_bits = a.take<unsigned>(64);
   b->active = a.take<uint32_t>((size_t)b->nbricks);
   b->reach = a.take<uint32_t>((size_t)b->nbricks);
-  b->lists_n = a.take<uint32_t>(4);
   b->overflow = a.take<uint32_t>((size_t)b->nbricks);
   b->cscratch = a.take<float>((size_t)b->cslots * b->bvol * 12);
 }
@@ -526,24 +526,6 @@ __global__ void k_brick_lists(const uint32_t *__restrict__ cell_start, int64_t n
       near = holds((z * nby + y) * nbx + x);
     }
     if (near) reach[atomicAdd(lists_n + 1, 1u)] = (uint32_t)b;
-  }
-}
-
-__global__ void k_gather_records(const float4 *__restrict__ rec_user, const uint32_t *__restrict__ perm,
-                                 int64_t m, float4 *__restrict__ rec, const uint32_t *gate = nullptr) {
-  if (gate && __ldg(gate) == 0u) return;  // the stable placement wrote the records
-  // four slots a trip: their indices, then their records, then the stores
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < m; s += 4 * stride) {
-    uint32_t p[4];
-    float4 r[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) p[u] = s + u * stride < m ? __ldg(perm + s + u * stride) : 0u;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) r[u] = s + u * stride < m ? __ldg(rec_user + p[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (s + u * stride < m) rec[s + u * stride] = r[u];
   }
 }
 
@@ -3100,7 +3082,7 @@ gbg_status gbg_bins_create(const gbg_grid *grid, int64_t max_points, const int32
     return set_error(GBG_ENOMEM, "cudaMalloc of the bins failed");
   }
   bins_carve(b);
-  cudaMemset(b->cell_start, 0, sizeof(uint32_t) * ((size_t)b->nkeys + 1));
+  cudaMemset(b->lists_n, 0, sizeof(uint32_t) * (64 + (size_t)b->nkeys + 1));
   if (gbg_status e = side_pool_ready()) {
     cudaFree(b->block);
     delete b;
@@ -3187,9 +3169,8 @@ template <typename T>
 gbg_status bins_build_impl(gbg_bins_s *b, const T *positions, int64_t npoints, int32_t *device_status,
                            cudaStream_t st, const DisplaceArgs<T> *disp) {
   b->npoints = npoints;
-  GBG_CUDA_TRY(cudaMemsetAsync(b->cell_start, 0, sizeof(uint32_t) * ((size_t)b->nkeys + 1), st));
-  // the two work-list lengths and the counting sort's long-run flag
-  GBG_CUDA_TRY(cudaMemsetAsync(b->lists_n, 0, sizeof(uint32_t) * 3, st));
+  // the two work-list lengths and the counting sort's long runs, and the cells' counts behind them
+  GBG_CUDA_TRY(cudaMemsetAsync(b->lists_n, 0, sizeof(uint32_t) * (64 + (size_t)b->nkeys + 1), st));
   if (npoints == 0) return GBG_OK;
   BinGeom g;
   for (int d = 0; d < 3; ++d) {
@@ -3204,27 +3185,20 @@ gbg_status bins_build_impl(gbg_bins_s *b, const T *positions, int64_t npoints, i
   }
   g.bvol = b->bvol;
   const int blocks = launch_blocks(npoints, kThreads);
-  // the rank of each point within its key goes to skeys (free until the fallback sort)
   if (disp)
-    k_bin_keys<T, true><<<blocks, kThreads, 0, st>>>(g, positions, npoints, b->keys, b->cell_start, b->skeys,
+    k_bin_keys<T, true><<<blocks, kThreads, 0, st>>>(g, positions, npoints, b->keys, b->cell_start, b->rank,
                                                      b->rec_user, device_status, *disp);
   else
-    k_bin_keys<T, false><<<blocks, kThreads, 0, st>>>(g, positions, npoints, b->keys, b->cell_start, b->skeys,
+    k_bin_keys<T, false><<<blocks, kThreads, 0, st>>>(g, positions, npoints, b->keys, b->cell_start, b->rank,
                                                       b->rec_user, device_status);
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
-  int bits = 0;
-  while (bits < 32 && ((uint64_t)(b->nkeys - 1) >> bits) != 0) ++bits;
   // one counting pass: the scan of the counts gives every cell its slots, the atomic ranks
   // place the points, and a per-cell pass puts each cell's points in index order (the
-  // stable order; a cell of more than 1024 points sends the whole sort to the radix sort)
+  // stable order) with their records
   GBG_TRY(exclusive_scan_u32(b->cell_start, b->cell_start, b->nkeys + 1, b->scan_tmp, st));
-  GBG_TRY(stable_counting_sort(b->keys, b->skeys, b->cell_start, npoints, bits, b->perm, b->skeys, b->lists_n + 2,
-                               b->sort_tmp, st, b->rec_user, b->rec));
-  // the records in sorted order come with the stable placement; only the radix fallback's
-  // order (a cell of more than 1024 points) gathers them again
-  k_gather_records<<<blocks, kThreads, 0, st>>>(b->rec_user, b->perm, npoints, b->rec, b->lists_n + 2);
-  note_launch();
+  GBG_TRY(stable_counting_sort(b->keys, b->rank, b->cell_start, npoints, b->perm, b->lists_n + 2, b->sort_tmp, st,
+                               b->rec_user, b->rec));
   k_brick_lists<<<launch_blocks(b->nbricks, kThreads), kThreads, 0, st>>>(
       b->cell_start, b->nb[0], b->nb[1], b->nb[2], b->bvol, b->reach_ok ? 1 : 0, b->active, b->reach, b->lists_n);
   note_launch();

@@ -14,6 +14,7 @@ namespace {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;  // 2048
+constexpr int kScanChunks = 1216;                     // eight blocks per SM
 
 constexpr int kRsThreads = 256;
 constexpr int kRsItems = 16;
@@ -48,62 +49,86 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *w
   return warp_prefix + x - v;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_block_sums(const uint32_t *in, int64_t n,
-                                                             uint32_t *sums, const uint32_t *gate) {
-  if (gate && __ldg(gate) == 0u) return;
-  __shared__ uint32_t ws[32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  uint32_t s = 0;
+// Eight consecutive words of a thread (16-byte loads where all eight are inside).
+__device__ __forceinline__ void load_eight(const uint32_t *in, int64_t at, int64_t end, uint32_t (&v)[kScanItems]) {
+  if (at + kScanItems <= end) {
+    const uint4 x = *reinterpret_cast<const uint4 *>(in + at), y = *reinterpret_cast<const uint4 *>(in + at + 4);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+  } else {
 #pragma unroll
-  for (int r = 0; r < kScanItems; ++r) {
-    const int64_t i = base + r * kScanThreads + threadIdx.x;
-    if (i < n) s += in[i];
+    for (int r = 0; r < kScanItems; ++r) v[r] = at + r < end ? in[at + r] : 0u;
+  }
+}
+
+// The sum of every chunk (a whole number of tiles) of the input.
+__global__ void __launch_bounds__(kScanThreads) k_chunk_sums(const uint32_t *in, int64_t n, int64_t chunk,
+                                                             uint32_t *sums) {
+  __shared__ uint32_t ws[32];
+  const int64_t end = min(n, (int64_t)(blockIdx.x + 1) * chunk);
+  uint32_t s = 0;
+#pragma unroll 2
+  for (int64_t at = (int64_t)blockIdx.x * chunk + threadIdx.x * kScanItems; at < end; at += kScanTile) {
+    uint32_t v[kScanItems];
+    load_eight(in, at, end, v);
+#pragma unroll
+    for (int r = 0; r < kScanItems; ++r) s += v[r];
   }
   uint32_t total;
   block_exclusive_scan(s, ws, &total);
   if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// Scans one tile (coalesced through shared memory) and adds offsets[blockIdx.x] if given.
-// in may equal out: a block only reads and writes its own tile.
-__global__ void __launch_bounds__(kScanThreads) k_scan_tile(const uint32_t *in, uint32_t *out,
-                                                            int64_t n, const uint32_t *offsets,
-                                                            const uint32_t *gate) {
-  if (gate && __ldg(gate) == 0u) return;
-  __shared__ uint32_t tile[kScanTile];
+// Scans one chunk tile by tile, from the sum of the chunks before it, which every block adds up for
+// itself (at most kScanChunks words): two launches whatever the length, where a tile per block needed a
+// scan of the tiles' sums between them, in up to three more.  The next tile is loaded while one is
+// scanned.  in may equal out: a block only reads and writes its own chunk.
+__global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const uint32_t *in, uint32_t *out, int64_t n,
+                                                              int64_t chunk, const uint32_t *sums) {
   __shared__ uint32_t ws[32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-#pragma unroll
-  for (int r = 0; r < kScanItems; ++r) {
-    const int64_t i = base + r * kScanThreads + threadIdx.x;
-    tile[r * kScanThreads + threadIdx.x] = i < n ? in[i] : 0u;
+  uint32_t before = 0;
+  if (sums) {
+    for (unsigned i = threadIdx.x; i < blockIdx.x; i += kScanThreads) before += sums[i];
+    uint32_t total;
+    block_exclusive_scan(before, ws, &total);
+    before = total;
+    __syncthreads();
   }
-  __syncthreads();
-  uint32_t v[kScanItems];
-  uint32_t s = 0;
+  const int64_t end = min(n, (int64_t)(blockIdx.x + 1) * chunk);
+  int64_t at = (int64_t)blockIdx.x * chunk + threadIdx.x * kScanItems;
+  uint32_t next[kScanItems];
+  load_eight(in, at, end, next);
+  for (int64_t tile = (int64_t)blockIdx.x * chunk; tile < end; tile += kScanTile, at += kScanTile) {
+    uint32_t v[kScanItems], s = 0;
 #pragma unroll
-  for (int r = 0; r < kScanItems; ++r) {
-    v[r] = tile[threadIdx.x * kScanItems + r];
-    s += v[r];
-  }
-  uint32_t total;
-  uint32_t run = block_exclusive_scan(s, ws, &total) + (offsets ? offsets[blockIdx.x] : 0u);
+    for (int r = 0; r < kScanItems; ++r) {
+      v[r] = next[r];
+      s += v[r];
+    }
+    load_eight(in, at + kScanTile, end, next);
+    uint32_t total;
+    uint32_t run = before + block_exclusive_scan(s, ws, &total);
+    before += total;
+    __syncthreads();  // the warps' sums are read before the next tile's
 #pragma unroll
-  for (int r = 0; r < kScanItems; ++r) {
-    tile[threadIdx.x * kScanItems + r] = run;
-    run += v[r];
-  }
-  __syncthreads();
+    for (int r = 0; r < kScanItems; ++r) {
+      const uint32_t x = v[r];
+      v[r] = run;
+      run += x;
+    }
+    if (at + kScanItems <= end) {
+      *reinterpret_cast<uint4 *>(out + at) = make_uint4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<uint4 *>(out + at + 4) = make_uint4(v[4], v[5], v[6], v[7]);
+    } else {
 #pragma unroll
-  for (int r = 0; r < kScanItems; ++r) {
-    const int64_t i = base + r * kScanThreads + threadIdx.x;
-    if (i < n) out[i] = tile[r * kScanThreads + threadIdx.x];
+      for (int r = 0; r < kScanItems; ++r)
+        if (at + r < end) out[at + r] = v[r];
+    }
   }
 }
 
 __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t *keys, int64_t n, int shift,
-                                                        uint32_t *hist, int64_t nb, const uint32_t *gate) {
-  if (gate && __ldg(gate) == 0u) return;
+                                                        uint32_t *hist, int64_t nb) {
   __shared__ uint32_t h[kRsWarps][kRsBins];
   for (int i = threadIdx.x; i < kRsWarps * kRsBins; i += kRsThreads) (&h[0][0])[i] = 0u;
   __syncthreads();
@@ -131,9 +156,8 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *keys_
                                                            const uint32_t *vals_in, int64_t n,
                                                            int shift, const uint32_t *offsets,
                                                            int64_t nb, uint32_t *keys_out,
-                                                           uint32_t *vals_out, const uint32_t *gate) {
+                                                           uint32_t *vals_out) {
   static_assert(kRsThreads == kRsBins, "one thread per digit in the tile's digit scan");
-  if (gate && __ldg(gate) == 0u) return;
   __shared__ uint32_t wh[kRsWarps][kRsBins];
   __shared__ uint32_t sbase[kRsBins], goff[kRsBins], ws[32];
   __shared__ uint32_t skey[kRsTile], sval[kRsTile];
@@ -235,12 +259,13 @@ __global__ void k_place_unstable(const uint32_t *__restrict__ keys, const uint32
 
 // Makes the placement stable: the point in slot s moves to the position, within its key's
 // run of slots, given by the number of the run's points with a smaller index.  Runs longer
-// than kPlaceMaxRun are left alone and raise *big instead (the radix sort then redoes the
-// whole order), so no thread does more than kPlaceMaxRun steps.
+// than kPlaceMaxRun are left alone and listed instead (their first slots, *big of them), so no
+// thread does more than kPlaceMaxRun steps.
 constexpr uint32_t kPlaceMaxRun = 1024;
 __global__ void k_place_stable(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ starts,
                                const uint32_t *__restrict__ perm_u, int64_t n, uint32_t *__restrict__ perm,
-                               uint32_t *big, const float4 *__restrict__ rec_user, float4 *__restrict__ rec) {
+                               uint32_t *big, uint32_t *__restrict__ runs, const float4 *__restrict__ rec_user,
+                               float4 *__restrict__ rec) {
   // two slots a trip, each level of their loads issued together
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s0 < n; s0 += 2 * stride) {
@@ -269,7 +294,7 @@ __global__ void k_place_stable(const uint32_t *__restrict__ keys, const uint32_t
         continue;
       }
       if (c > kPlaceMaxRun) {
-        atomicOr(big, 1u);
+        if ((uint32_t)s == a) runs[atomicAdd(big, 1u)] = a;
         continue;
       }
       uint32_t r = 0;
@@ -277,6 +302,91 @@ __global__ void k_place_stable(const uint32_t *__restrict__ keys, const uint32_t
       perm[a + r] = p;
       if (rec) rec[a + r] = rv[u];
     }
+  }
+}
+
+// The long runs, one CTA each at a time: a stable LSD radix sort of the run's point indices between its
+// slots of perm_u and of perm, eight bits a pass, and the records in their order.  One launch that
+// returns at once when no run is listed, where a radix sort of every point, gated kernel by kernel,
+// took 15 to 25.  A run of 2e3 points takes a few microseconds; only a cell that holds most of a large
+// set sorts slower than the whole chip would.
+constexpr int kRunThreads = 512, kRunWarps = kRunThreads / 32, kRunItems = 4;
+__global__ void __launch_bounds__(kRunThreads)
+    k_sort_runs(const uint32_t *big, const uint32_t *runs, const uint32_t *__restrict__ keys,
+                const uint32_t *__restrict__ starts, uint32_t *perm_u, uint32_t *perm, int bits,
+                const float4 *__restrict__ rec_user, float4 *__restrict__ rec) {
+  const uint32_t nruns = *big;
+  if (nruns == 0u) return;
+  __shared__ uint32_t wh[kRunWarps][kRsBins], base[kRsBins], ws[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t lower = (1u << lane) - 1u;
+  for (uint32_t i = blockIdx.x; i < nruns; i += gridDim.x) {
+    const uint32_t a = runs[i], key = keys[perm_u[a]], c = starts[key + 1] - a;
+    __syncthreads();  // every thread has read the run's first slot (and the last run is done)
+    const int passes = (bits + 7) / 8;
+    uint32_t *src = perm_u + a, *dst = perm + a;
+    if (passes % 2 == 0) {  // the last pass writes perm
+      for (uint32_t t = threadIdx.x; t < c; t += kRunThreads) dst[t] = src[t];
+      uint32_t *x = src;
+      src = dst;
+      dst = x;
+      __syncthreads();
+    }
+    for (int pass = 0; pass < passes; ++pass) {
+      const int shift = 8 * pass;
+      if (threadIdx.x < kRsBins) base[threadIdx.x] = 0u;
+      __syncthreads();
+      for (uint32_t t = threadIdx.x; t < c; t += kRunThreads) atomicAdd(&base[(src[t] >> shift) & 0xffu], 1u);
+      __syncthreads();
+      {
+        uint32_t total;
+        const uint32_t v = threadIdx.x < kRsBins ? base[threadIdx.x] : 0u;
+        const uint32_t x = block_exclusive_scan(v, ws, &total);
+        if (threadIdx.x < kRsBins) base[threadIdx.x] = x;
+      }
+      __syncthreads();
+      for (uint32_t t0 = 0; t0 < c; t0 += kRunThreads * kRunItems) {
+        for (int k = threadIdx.x; k < kRunWarps * kRsBins; k += kRunThreads) (&wh[0][0])[k] = 0u;
+        __syncthreads();
+        uint32_t v[kRunItems];
+        const uint32_t seg = t0 + warp * (32 * kRunItems) + lane;  // a warp's items are consecutive
+#pragma unroll
+        for (int r = 0; r < kRunItems; ++r) {
+          v[r] = seg + 32 * r < c ? src[seg + 32 * r] : 0u;
+          if (seg + 32 * r < c) atomicAdd(&wh[warp][(v[r] >> shift) & 0xffu], 1u);
+        }
+        __syncthreads();
+        if (threadIdx.x < kRsBins) {
+          uint32_t run = base[threadIdx.x];
+#pragma unroll
+          for (int w = 0; w < kRunWarps; ++w) {
+            const uint32_t x = wh[w][threadIdx.x];
+            wh[w][threadIdx.x] = run;
+            run += x;
+          }
+          base[threadIdx.x] = run;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRunItems; ++r) {
+          const bool valid = seg + 32 * r < c;
+          const uint32_t digit = valid ? (v[r] >> shift) & 0xffu : 0x100u;
+          const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+          uint32_t pos = 0;
+          if (valid) pos = wh[warp][digit] + __popc(peers & lower);
+          __syncwarp();
+          if (valid && lane == 31 - __clz(peers)) wh[warp][digit] += __popc(peers);
+          __syncwarp();
+          if (valid) dst[pos] = v[r];
+        }
+        __syncthreads();
+      }
+      uint32_t *x = src;
+      src = dst;
+      dst = x;
+    }
+    if (rec)
+      for (uint32_t t = threadIdx.x; t < c; t += kRunThreads) rec[a + t] = rec_user[src[t]];
   }
 }
 
@@ -290,32 +400,24 @@ int launch_blocks(int64_t work, int threads, int per_sm) {
 }
 
 size_t scan_temp_elems(int64_t n) {
-  size_t total = 0;
-  int64_t m = n;
-  while (m > kScanTile) {
-    m = (m + kScanTile - 1) / kScanTile;
-    total += (size_t)m + 64;
-  }
-  return total + 64;
+  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+  return (size_t)(tiles < kScanChunks ? tiles : kScanChunks) + 64;
 }
 
-gbg_status exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *tmp,
-                              cudaStream_t stream, const uint32_t *gate) {
+gbg_status exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *tmp, cudaStream_t stream) {
   if (n <= 0) return GBG_OK;
-  const int64_t nb = (n + kScanTile - 1) / kScanTile;
-  if (nb == 1) {
-    k_scan_tile<<<1, kScanThreads, 0, stream>>>(in, out, n, nullptr, gate);
+  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+  if (tiles == 1) {
+    k_scan_chunks<<<1, kScanThreads, 0, stream>>>(in, out, n, kScanTile, nullptr);
     note_launch();
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;
   }
-  uint32_t *sums = tmp;
-  uint32_t *rest = tmp + nb + 64;
-  k_block_sums<<<(unsigned)nb, kScanThreads, 0, stream>>>(in, n, sums, gate);
+  const int64_t per = (tiles + kScanChunks - 1) / kScanChunks, chunk = per * kScanTile;
+  const unsigned blocks = (unsigned)((tiles + per - 1) / per);
+  k_chunk_sums<<<blocks, kScanThreads, 0, stream>>>(in, n, chunk, tmp);
   note_launch();
-  GBG_CUDA_TRY(cudaGetLastError());
-  GBG_TRY(exclusive_scan_u32(sums, sums, nb, rest, stream, gate));
-  k_scan_tile<<<(unsigned)nb, kScanThreads, 0, stream>>>(in, out, n, sums, gate);
+  k_scan_chunks<<<blocks, kScanThreads, 0, stream>>>(in, out, n, chunk, tmp);
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
   return GBG_OK;
@@ -333,7 +435,7 @@ size_t radix_sort_temp_bytes(int64_t n) {
 
 gbg_status radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
                             uint32_t *vals_out, int64_t n, int key_bits, void *temp,
-                            cudaStream_t stream, const uint32_t *gate) {
+                            cudaStream_t stream) {
   if (n <= 0) return GBG_OK;
   if (n > 0x7fffffffLL) return set_error(GBG_EUNSUPPORTED, "radix sort: more than 2^31-1 points");
   const int64_t nb = (n + kRsTile - 1) / kRsTile;
@@ -351,11 +453,11 @@ gbg_status radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, ui
     const bool to_out = ((passes - 1 - p) % 2) == 0;
     uint32_t *kout = to_out ? keys_out : kt;
     uint32_t *vout = to_out ? vals_out : vt;
-    k_rs_hist<<<(unsigned)nb, kRsThreads, 0, stream>>>(kin, n, 8 * p, hist, nb, gate);
+    k_rs_hist<<<(unsigned)nb, kRsThreads, 0, stream>>>(kin, n, 8 * p, hist, nb);
     note_launch();
     GBG_CUDA_TRY(cudaGetLastError());
-    GBG_TRY(exclusive_scan_u32(hist, hist, kRsBins * nb, scan_tmp, stream, gate));
-    k_rs_scatter<<<(unsigned)nb, kRsThreads, 0, stream>>>(kin, vin, n, 8 * p, hist, nb, kout, vout, gate);
+    GBG_TRY(exclusive_scan_u32(hist, hist, kRsBins * nb, scan_tmp, stream));
+    k_rs_scatter<<<(unsigned)nb, kRsThreads, 0, stream>>>(kin, vin, n, 8 * p, hist, nb, kout, vout);
     note_launch();
     GBG_CUDA_TRY(cudaGetLastError());
     kin = kout;
@@ -365,21 +467,26 @@ gbg_status radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, ui
 }
 
 
-gbg_status stable_counting_sort(const uint32_t *keys, const uint32_t *rank, const uint32_t *starts, int64_t n,
-                                int key_bits, uint32_t *perm, uint32_t *skeys, uint32_t *big, void *temp,
-                                cudaStream_t stream, const float4 *rec_user, float4 *rec) {
+gbg_status stable_counting_sort(const uint32_t *keys, uint32_t *rank, const uint32_t *starts, int64_t n, uint32_t *perm,
+                                uint32_t *big, uint32_t *temp, cudaStream_t stream, const float4 *rec_user,
+                                float4 *rec) {
   if (n <= 0) return GBG_OK;
   if (n > 0x7fffffffLL) return set_error(GBG_EUNSUPPORTED, "counting sort: more than 2^31-1 points");
-  // the unstable placement lives at the start of the radix sort's scratch, which only the
-  // fallback (after the stable pass has read it) writes
-  uint32_t *perm_u = static_cast<uint32_t *>(temp);
   const int blocks = launch_blocks(n, 256);
-  k_place_unstable<<<blocks, 256, 0, stream>>>(keys, rank, starts, n, perm_u);
+  k_place_unstable<<<blocks, 256, 0, stream>>>(keys, rank, starts, n, temp);
   note_launch();
-  k_place_stable<<<blocks, 256, 0, stream>>>(keys, starts, perm_u, n, perm, big, rec_user, rec);
+  // the ranks are read no more: their array takes the list of long runs
+  k_place_stable<<<blocks, 256, 0, stream>>>(keys, starts, temp, n, perm, big, rank, rec_user, rec);
   note_launch();
+  int bits = 1;
+  while ((uint64_t)(n - 1) >> bits) ++bits;
+  if (n > (int64_t)kPlaceMaxRun) {  // fewer points hold no long run
+    k_sort_runs<<<launch_blocks(n / kPlaceMaxRun, 1, 1), kRunThreads, 0, stream>>>(big, rank, keys, starts, temp, perm,
+                                                                                  bits, rec_user, rec);
+    note_launch();
+  }
   GBG_CUDA_TRY(cudaGetLastError());
-  return radix_sort_pairs(keys, nullptr, skeys, perm, n, key_bits, temp, stream, big);
+  return GBG_OK;
 }
 
 }  // namespace gbg

@@ -219,3 +219,48 @@ def test_wrap_around_every_bound(gbg, oracle, dev, T, origin):
     assert np.array_equal(got.view(np.uint64 if T is np.float64 else np.uint32)[~np.isnan(want)],
                           want.view(np.uint64 if T is np.float64 else np.uint32)[~np.isnan(want)])
     assert np.array_equal(np.isnan(got), np.isnan(want))
+
+
+# cells at and above the longest run that the placement sorts itself (1024), of one tile of the run sort
+# (2048) and of several, alone and together; index widths of one to three passes
+@pytest.mark.parametrize("runs", [(1024,), (1025,), (2048, 2049), (1500, 9000, 1025, 70_001)])
+@pytest.mark.parametrize("spread", [0, 300, 200_000])
+def test_bins_order_with_long_runs(gbg, dev, runs, spread):
+    from gbgperiodicfields_gb300 import resident
+    n, brick = np.array((20, 18, 16)), np.array((11, 8, 8))
+    rng = np.random.default_rng(sum(runs) + spread)
+    grid = gbg.Grid3D(tuple(n), tuple(float(v) for v in n))  # cells of edge 1
+    pos = [rng.random((spread, 3)) * n]
+    for k, c in enumerate(runs):
+        pos.append(np.array([3 * k + 1, 17 - 2 * k, k]) + rng.random((c, 3)))
+    pos = np.concatenate(pos)
+    pos = np.asfortranarray(pos[rng.permutation(len(pos))])
+    bins = resident.PointBins(grid, len(pos), brick=tuple(brick)).build(to_dev(pos, dev))
+    c = np.floor(pos).astype(np.int64) % n
+    nb, br = -(-n // brick), c // brick
+    loc = c - br * brick
+    key = ((br[:, 2] * nb[1] + br[:, 1]) * nb[0] + br[:, 0]) * brick.prod() + (loc[:, 2] * brick[1] + loc[:, 1]) * brick[0] + loc[:, 0]
+    assert np.array_equal(bins.order().cpu().numpy(), np.argsort(key, kind="stable") + 1)
+    # the records follow: a linear field is reproduced by the cubic spline inside the box
+    x = torch.arange(int(n[0]), dtype=torch.float64, device=dev)[:, None, None].expand(*[int(v) for v in n])
+    field = resident.ResidentField(grid, 1, 4).load(gbg.colmajor(x.contiguous()[..., None]))
+    got = resident.interpolate_binned(field, bins, gbg.CatmullRom).cpu().numpy()[:, 0]
+    inner = (pos[:, 0] >= 2) & (pos[:, 0] < n[0] - 3)
+    assert np.abs(got - pos[:, 0])[inner].max(initial=0.0) <= 1e-5 * n[0]
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 2047, 2048, 2049, 4096 * 19, 1216 * 2048 + 5, 3 * 1216 * 2048 - 1])
+def test_cell_starts_at_every_scan_length(gbg, dev, n):
+    # grids of n cells in a row of bricks: the bins' order is the points' order by cell
+    from gbgperiodicfields_gb300 import resident
+    edge = 1 if n <= 64 else 64
+    rows = -(-n // edge)
+    ny = next(v for v in range(min(rows, 64), 0, -1) if rows % v == 0)
+    grid = gbg.Grid3D((edge, ny, rows // ny), (float(edge), float(ny), float(rows // ny)))
+    rng = np.random.default_rng(n)
+    m = 5000
+    pos = np.asfortranarray(rng.random((m, 3)) * np.array(grid.grid_size))
+    bins = resident.PointBins(grid, m, brick=(edge, 1, 1)).build(to_dev(pos, dev))
+    c = np.floor(pos).astype(np.int64)
+    key = (c[:, 2] * ny + c[:, 1]) * edge + c[:, 0]
+    assert np.array_equal(bins.order().cpu().numpy(), np.argsort(key, kind="stable") + 1)
