@@ -264,3 +264,40 @@ def test_cell_starts_at_every_scan_length(gbg, dev, n):
     c = np.floor(pos).astype(np.int64)
     key = (c[:, 2] * ny + c[:, 1]) * edge + c[:, 0]
     assert np.array_equal(bins.order().cpu().numpy(), np.argsort(key, kind="stable") + 1)
+
+
+# a group of lanes per point: points no multiple of a CTA's groups, axes shorter than the stencil (which
+# wraps more than once), component counts of every chunk, powers fewer than nodes, a bad traversal entry
+@pytest.mark.parametrize("n", [(3, 5, 2), (33, 8, 9)])
+@pytest.mark.parametrize("m", [1, 3, 65, 4097])
+@pytest.mark.parametrize("ncomp", [1, 2, 3, 9])
+@pytest.mark.parametrize("name", ["C4", "L6m1", "L6", "G8"])
+def test_fp32_gather_rows(gbg, oracle, dev, n, m, ncomp, name):
+    from gbgperiodicfields_gb300 import _lib
+    scheme = {"C4": gbg.CatmullRom, "L6m1": gbg.LalescuSpline(6, 1), "L6": gbg.LalescuSpline(6),
+              "G8": gbg.LagrangeSpline(8)}[name]
+    rng = np.random.default_rng(m + ncomp)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, origin=(0.25, -2.0, 1.0), dtype=torch.float32)
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin, dtype=np.float32)
+    pos = np.asfortranarray((np.array(grid.origin) + TWO_PI * (rng.random((m, 3)) * 3 - 1)).astype(np.float32))
+    f = np.asfortranarray(rng.standard_normal(n + (ncomp,)).astype(np.float32))
+    fd, pd = to_dev(f, dev), to_dev(pos, dev)
+    trav = torch.from_numpy((rng.permutation(m) + 1).astype(np.int32)).to(dev)
+    got = []
+    for t in (None, trav):
+        out = gbg.zeros_colmajor((m, ncomp), torch.float32, dev)
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
+        st = _lib.load().gbg_interpolate(grid.c(), _lib.GBG_F32, ncomp, fd.data_ptr(), pd.data_ptr(), m,
+                                         t.data_ptr() if t is not None else None, scheme.c(), out.data_ptr(),
+                                         status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        _lib.check(st, "gather")
+        assert int(status.item()) == 0
+        got.append(out.cpu().numpy())
+    assert np.array_equal(got[0], got[1])
+    assert relerr(got[0], oracle.gather(g, f, pos, scheme.coefficients)) <= 2e-5
+    trav[m // 2] = m + 1
+    out, status = gbg.zeros_colmajor((m, ncomp), torch.float32, dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    _lib.check(_lib.load().gbg_interpolate(grid.c(), _lib.GBG_F32, ncomp, fd.data_ptr(), pd.data_ptr(), m, trav.data_ptr(),
+                                           scheme.c(), out.data_ptr(), status.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream), "gather")
+    assert int(status.item()) == _lib.GBG_DEV_TRAVERSAL
