@@ -57,12 +57,18 @@ __device__ __forceinline__ double quiet_nan<double>() { return __longlong_as_dou
 template <>
 __device__ __forceinline__ float quiet_nan<float>() { return __int_as_float(0x7fc00000); }
 
+// mod(c, n), the remainder taken only outside the grid.
+__device__ __forceinline__ int64_t wrap_cell(int64_t c, int64_t n) {
+  return (uint64_t)c < (uint64_t)n ? c : imod(c, n);
+}
+
 // The wrapped node offsets visited along one axis: the reference's wrapped start
 // mod(base - n, N) followed by its step rule (Interpolation.jl:1000, 1025-1027).
-template <int N2>
+template <typename T, int N2>
 __device__ __forceinline__ void walk_offsets(int64_t base, int64_t extent, int64_t stride,
                                              int64_t (&off)[N2]) {
-  int64_t node = imod(base - (N2 - 2) / 2, extent);
+  // (the branch of wrap_cell costs the FP32 gather, which hides the remainder behind its loads, 10%)
+  int64_t node = sizeof(T) == 8 ? wrap_cell(base - (N2 - 2) / 2, extent) : imod(base - (N2 - 2) / 2, extent);
 #pragma unroll
   for (int i = 0; i < N2; ++i) {
     off[i] = node * stride;
@@ -87,11 +93,6 @@ __device__ __forceinline__ bool locate3(const GridT<T> &g, const T *__restrict__
   return ok;
 }
 
-// mod(c, n), the remainder taken only outside the grid.
-__device__ __forceinline__ int64_t wrap_cell(int64_t c, int64_t n) {
-  return (uint64_t)c < (uint64_t)n ? c : imod(c, n);
-}
-
 // _visit (Interpolation.jl:618-619), bounds-checked instead of trusted.
 __device__ __forceinline__ bool visit(const int32_t *__restrict__ trav, int64_t w, int64_t m,
                                       int64_t &p, int32_t *status) {
@@ -104,6 +105,57 @@ __device__ __forceinline__ bool visit(const int32_t *__restrict__ trav, int64_t 
   }
   p = v;
   return true;
+}
+
+// The reference's _locate with the quotient from the reciprocal of the spacing, r = RN(1/d): q =
+// RN(a r), then q + r (a - q d) with the residual exact by a fused multiply-add (Markstein's
+// correction).  Before its rounding the corrected quotient is within 2^-104 of a/d, so it is the
+// correctly rounded one of _locate unless a/d lies that close to a midpoint.  The floor is taken on
+// the bits: GB300 starts an FP64 operation of a warp every 76 clocks per scheduler and these points
+// need five instead of about seventeen.  False where floor(Int, q) throws in the reference.
+__device__ __forceinline__ bool locate_recip(double x, double o, double d, double r, int64_t &base, double &t) {
+  const double a = x - o;
+  const double q0 = a * r;
+  const double q = fma(fma(-q0, d, a), r, q0);
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(q);
+  const unsigned long long mag = bits & 0x7fffffffffffffffull;
+  const bool ok = mag < 0x43df399b1438a100ull;  // the bits of 9.0e18; NaN and infinities order above
+  const int ex = (int)(mag >> 52) - 1023;
+  unsigned long long whole = 0ull, cut = 0ull;  // |trunc q|, and the fraction's bits
+  unsigned long long tb = bits & 0x8000000000000000ull;
+  if (ex >= 0 && ok) {
+    const unsigned long long man = (mag & 0xfffffffffffffull) | 0x10000000000000ull;
+    const unsigned long long low = ex < 52 ? (1ull << (52 - ex)) - 1ull : 0ull;
+    cut = bits & low;
+    tb = bits & ~low;
+    whole = ex <= 52 ? man >> (52 - ex) : man << (ex - 52);
+  } else if (ok) {
+    cut = mag;
+  }
+  double fl = __longlong_as_double((long long)tb);
+  base = (long long)whole;
+  if (bits >> 63) {
+    base = -base;
+    if (cut) {
+      base -= 1;
+      fl -= 1.0;
+    }
+  }
+  if (!ok) base = 0;
+  t = q - fl;
+  return ok;
+}
+__device__ __forceinline__ bool locate_recip(float x, float o, float d, float, int64_t &base, float &t) {
+  return locate(x, o, d, base, t);  // FP32 divides at full rate
+}
+
+template <typename T>
+__device__ __forceinline__ bool locate3_recip(const GridT<T> &g, const T *__restrict__ pos, int64_t p, int64_t m,
+                                              int64_t (&b)[3], T (&t)[3]) {
+  bool ok = locate_recip(__ldg(pos + p), g.ox, g.dx, g.rx, b[0], t[0]);
+  ok &= locate_recip(__ldg(pos + p + m), g.oy, g.dy, g.ry, b[1], t[1]);
+  ok &= locate_recip(__ldg(pos + p + 2 * m), g.oz, g.dz, g.rz, b[2], t[2]);
+  return ok;
 }
 
 // ---------------------------------------------------------------- gather
@@ -133,15 +185,19 @@ __device__ __forceinline__ void axis_weights_fma(const SchemeT<T, N2> &s, T t, T
   }
 }
 
-// Compile-time width N2: the (j, i) stencil plane is unrolled, z advances by the
-// reference's running walk.  The x direction is contracted first, per (j, k) and
-// component, s = sum_i w1[i] f, then acc += (w2[j] w3[k]) s: 22 FP64 operations per
-// (j, k) at width 6 and 3 components instead of 25 -- this kernel is FP64-pipe-bound.
+// Compile-time width N2: the (j, i) stencil plane is unrolled, z advances by the reference's running
+// walk.  In FP64 this kernel is bound by the FP64 pipe (an operation of a warp every 76 clocks of a
+// scheduler), so it counts operations: x is contracted first, then y over the plane, then z -- N2^3 +
+// N2^2 + N2 a component and no weight products, 774 at width 6 and 3 components beside 90 for the
+// weights and 15 for the locate; the product form (w2[j] w3[k] once per plane row) took 792 + 90 + 50.
+// 256^3 x 3, 1e7 points, width 6: 15.75 -> 14.98 ms.
 template <typename T, int N2, int M2, int CC>
 __global__ void __launch_bounds__(kThreads)
     k_gather_plain(GridT<T> g, SchemeT<T, N2> s, int ncomp, const T *__restrict__ field,
                    const T *__restrict__ pos, int64_t m, const int32_t *__restrict__ trav,
                    T *__restrict__ out, int32_t *status) {
+  // FP32 (whose bound is its loads) and nine components keep the product form: fewer sums to hold
+  constexpr bool kPlane = sizeof(T) == 8 && CC < 9;
   const int64_t nxny = g.nx * g.ny;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < m;
        w += (int64_t)gridDim.x * blockDim.x) {
@@ -149,16 +205,16 @@ __global__ void __launch_bounds__(kThreads)
     if (!visit(trav, w, m, p, status)) continue;
     int64_t b[3];
     T t[3];
-    const bool ok = locate3(g, pos, p, m, b, t);
+    const bool ok = locate3_recip(g, pos, p, m, b, t);
     if (!ok && status) atomicOr(status, GBG_DEV_NONFINITE);
     T w1[N2], w2[N2], w3[N2];
     axis_weights_fma<T, N2, M2>(s, t[0], w1);
     axis_weights_fma<T, N2, M2>(s, t[1], w2);
     axis_weights_fma<T, N2, M2>(s, t[2], w3);
     int64_t ix[N2], iy[N2];
-    walk_offsets<N2>(b[0], g.nx, 1, ix);
-    walk_offsets<N2>(b[1], g.ny, g.nx, iy);
-    const int64_t z0 = imod(b[2] - (N2 - 2) / 2, g.nz);
+    walk_offsets<T, N2>(b[0], g.nx, 1, ix);
+    walk_offsets<T, N2>(b[1], g.ny, g.nx, iy);
+    const int64_t z0 = sizeof(T) == 8 ? wrap_cell(b[2] - (N2 - 2) / 2, g.nz) : imod(b[2] - (N2 - 2) / 2, g.nz);
     for (int c0 = 0; c0 < ncomp; c0 += CC) {
       T acc[CC];
 #pragma unroll
@@ -172,9 +228,9 @@ __global__ void __launch_bounds__(kThreads)
         for (int q = 1; q < N2; ++q)
           if (q == k) w3k = w3[q];
         const T *plane = fc + node_z * nxny;
+        [[maybe_unused]] T sy[CC];
 #pragma unroll
         for (int j = 0; j < N2; ++j) {
-          const T wyz = mul_rn(w2[j], w3k);
           const T *row = plane + iy[j];
           T sx[CC];
 #pragma unroll
@@ -185,8 +241,18 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
             for (int c = 0; c < CC; ++c) sx[c] = fma_rn(w1[i], __ldg(f + g.npf * c), sx[c]);
           }
+          if constexpr (kPlane) {
 #pragma unroll
-          for (int c = 0; c < CC; ++c) acc[c] = fma_rn(wyz, sx[c], acc[c]);
+            for (int c = 0; c < CC; ++c) sy[c] = j ? fma_rn(w2[j], sx[c], sy[c]) : mul_rn(w2[0], sx[c]);
+          } else {
+            const T wyz = mul_rn(w2[j], w3k);
+#pragma unroll
+            for (int c = 0; c < CC; ++c) acc[c] = fma_rn(wyz, sx[c], acc[c]);
+          }
+        }
+        if constexpr (kPlane) {
+#pragma unroll
+          for (int c = 0; c < CC; ++c) acc[c] = fma_rn(w3k, sy[c], acc[c]);
         }
         node_z = step_up(node_z, g.nz);
       }
@@ -517,57 +583,6 @@ struct BrickGeo {
   int32_t eb[3];  // the bricks that the largest quantity exponents are kept for
   int64_t enb[3];
 };
-
-// The reference's _locate with the quotient from the reciprocal of the spacing, r = RN(1/d): q =
-// RN(a r), then q + r (a - q d) with the residual exact by a fused multiply-add (Markstein's
-// correction).  Before its rounding the corrected quotient is within 2^-104 of a/d, so it is the
-// correctly rounded one of _locate unless a/d lies that close to a midpoint.  The floor is taken on
-// the bits: GB300 starts an FP64 operation of a warp every 76 clocks per scheduler and these points
-// need five instead of about seventeen.  False where floor(Int, q) throws in the reference.
-__device__ __forceinline__ bool locate_recip(double x, double o, double d, double r, int64_t &base, double &t) {
-  const double a = x - o;
-  const double q0 = a * r;
-  const double q = fma(fma(-q0, d, a), r, q0);
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(q);
-  const unsigned long long mag = bits & 0x7fffffffffffffffull;
-  const bool ok = mag < 0x43df399b1438a100ull;  // the bits of 9.0e18; NaN and infinities order above
-  const int ex = (int)(mag >> 52) - 1023;
-  unsigned long long whole = 0ull, cut = 0ull;  // |trunc q|, and the fraction's bits
-  unsigned long long tb = bits & 0x8000000000000000ull;
-  if (ex >= 0 && ok) {
-    const unsigned long long man = (mag & 0xfffffffffffffull) | 0x10000000000000ull;
-    const unsigned long long low = ex < 52 ? (1ull << (52 - ex)) - 1ull : 0ull;
-    cut = bits & low;
-    tb = bits & ~low;
-    whole = ex <= 52 ? man >> (52 - ex) : man << (ex - 52);
-  } else if (ok) {
-    cut = mag;
-  }
-  double fl = __longlong_as_double((long long)tb);
-  base = (long long)whole;
-  if (bits >> 63) {
-    base = -base;
-    if (cut) {
-      base -= 1;
-      fl -= 1.0;
-    }
-  }
-  if (!ok) base = 0;
-  t = q - fl;
-  return ok;
-}
-__device__ __forceinline__ bool locate_recip(float x, float o, float d, float, int64_t &base, float &t) {
-  return locate(x, o, d, base, t);  // FP32 divides at full rate
-}
-
-template <typename T>
-__device__ __forceinline__ bool locate3_recip(const GridT<T> &g, const T *__restrict__ pos, int64_t p, int64_t m,
-                                              int64_t (&b)[3], T (&t)[3]) {
-  bool ok = locate_recip(__ldg(pos + p), g.ox, g.dx, g.rx, b[0], t[0]);
-  ok &= locate_recip(__ldg(pos + p + m), g.oy, g.dy, g.ry, b[1], t[1]);
-  ok &= locate_recip(__ldg(pos + p + 2 * m), g.oz, g.dz, g.rz, b[2], t[2]);
-  return ok;
-}
 
 // A quantity as an exact integer mantissa and a binary exponent, from its bits: v = mq 2^(e - 62)
 // with 2^61 <= |mq| < 2^62.  The exponent is kept biased so that 0 means zero and kENonFinite (above
