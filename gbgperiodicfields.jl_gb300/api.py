@@ -17,7 +17,10 @@ There is no CPU path: host tensors are refused.
 """
 from __future__ import annotations
 
+import contextlib
+import ctypes
 import math
+import threading
 from typing import Optional, Sequence
 
 import numpy as np
@@ -565,12 +568,46 @@ def _check_traversal(traversal, m: int, device):
     return traversal.indices
 
 
-def _status_buffer(device):
-    return torch.zeros(1, dtype=torch.int32, device=device)
+class _StatusWord:
+    """A word of pinned host memory that the kernels of a synchronous call report into (GBG_DEV_*
+    bits): no fill before the launch and no copy back after it, only the call's own wait for its
+    stream.  One per thread; a thread has one such call in flight at a time."""
+
+    def __init__(self):
+        self.word = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        self.value = self.word.numpy()
+
+    def data_ptr(self):
+        return self.word.data_ptr()
 
 
-def _raise_device_status(status: torch.Tensor):
-    v = int(status.item())
+_status_words = threading.local()
+
+
+def _status_word() -> _StatusWord:
+    """This thread's status word, cleared."""
+    word = getattr(_status_words, "word", None)
+    if word is None:
+        word = _status_words.word = _StatusWord()
+    word.value[0] = 0
+    return word
+
+
+def _on_device(t: torch.Tensor):
+    """A context in which t's device is current (none where it is already)."""
+    return torch.cuda.device(t.device) if t.device.index != torch.cuda.current_device() else contextlib.nullcontext()
+
+
+def _check_launched(st: int, what: str, stream):
+    """_lib.check; a call that failed half-way is waited for first, as its kernels hold the status word."""
+    if st != _lib.GBG_OK:
+        stream.synchronize()
+    _lib.check(st, what)
+
+
+def _raise_device_status(status: _StatusWord):
+    """The device's report, read after the call's stream has been waited for."""
+    v = int(status.value[0])
     if v & _lib.GBG_DEV_NONFINITE:
         raise InexactError("a non-finite or out-of-range position reached the locate step "
                            "(floor(Int, x) of a non-finite coordinate)")
@@ -593,14 +630,14 @@ def interpolate_(out: AbstractPointValues, field: AbstractFieldPhysical, points:
     trav = _check_traversal(traversal, m, field.data.device)
     if m == 0:
         return out
-    status = _status_buffer(field.data.device)
-    with torch.cuda.device(field.data.device):
+    status = _status_word()
+    with _on_device(field.data):
         stream = torch.cuda.current_stream()
         st = _lib.load().gbg_interpolate(
             field.grid.c(), _DTYPE_CODE[field.data.dtype], field.ncomp, field.data.data_ptr(),
             points.positions.data_ptr(), m, trav.data_ptr() if trav is not None else None,
             scheme.c(), out.data.data_ptr(), status.data_ptr(), stream.cuda_stream)
-        _lib.check(st, "interpolate!")
+        _check_launched(st, "interpolate!", stream)
         stream.synchronize()
     _raise_device_status(status)
     return out
@@ -633,15 +670,14 @@ def anterpolate_(field: AbstractFieldPhysical, points: PointSet, quantities: Abs
     _check_colocation(field, points, quantities)
     m = points.npoints
     trav = _check_traversal(traversal, m, field.data.device)
-    status = _status_buffer(field.data.device)
-    import ctypes
+    status = _status_word()
     nbytes = ctypes.c_size_t()
     lib = _lib.load()
     _lib.check(lib.gbg_anterpolate_workspace_size(field.grid.c(), _DTYPE_CODE[field.data.dtype], field.ncomp,
                                                   m, scheme.c(), ctypes.byref(nbytes)), "anterpolate!")
     # scratch from torch's caching allocator, so repeated calls do not re-allocate
     ws = torch.empty(max(int(nbytes.value), 1), dtype=torch.uint8, device=field.data.device)
-    with torch.cuda.device(field.data.device):
+    with _on_device(field.data):
         stream = torch.cuda.current_stream()
         st = lib.gbg_anterpolate(
             field.grid.c(), _DTYPE_CODE[field.data.dtype], field.ncomp, field.data.data_ptr(),
@@ -649,7 +685,7 @@ def anterpolate_(field: AbstractFieldPhysical, points: PointSet, quantities: Abs
             quantities.data.data_ptr() if m else None, trav.data_ptr() if trav is not None else None,
             scheme.c(), float(alpha), float(beta), ws.data_ptr(), ws.numel(), status.data_ptr(),
             stream.cuda_stream)
-        _lib.check(st, "anterpolate!")
+        _check_launched(st, "anterpolate!", stream)
         stream.synchronize()
     _raise_device_status(status)
     return field

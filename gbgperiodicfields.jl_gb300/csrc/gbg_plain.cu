@@ -1484,11 +1484,14 @@ struct ScatterLayout {
 
 ScatterLayout scatter_layout(Arena &a, int64_t m, const ScatterPlan &P, int ncomp, int n2, size_t esize) {
   ScatterLayout L;
-  L.keys = a.take<uint32_t>((size_t)m);
+  // the words that start at zero stand together (scatter_clear)
+  const size_t nexp = P.bricked ? (size_t)(P.bg.enb[0] * P.bg.enb[1] * P.bg.enb[2]) : 0;
+  L.flag = a.take<uint32_t>(4);
+  L.ebrick = P.bricked ? a.take<uint32_t>(nexp * ncomp) : nullptr;
   L.counts = a.take<uint32_t>((size_t)P.nkeys + 1);
+  L.keys = a.take<uint32_t>((size_t)m);
   L.rank = a.take<uint32_t>((size_t)m);
   L.perm = a.take<uint32_t>((size_t)m);
-  L.flag = a.take<uint32_t>(4);
   L.sort_tmp = P.bricked ? nullptr : a.take<uint32_t>((size_t)m);
   L.scan_tmp = a.take<uint32_t>(scan_temp_elems(P.nkeys + 1));
   const size_t rec_bytes = 3 * (size_t)n2 * (P.bricked ? sizeof(long long) : esize);
@@ -1496,9 +1499,14 @@ ScatterLayout scatter_layout(Arena &a, int64_t m, const ScatterPlan &P, int ncom
   L.qs = P.bricked ? nullptr : a.take<char>((size_t)m * ncomp * esize);
   L.qi = P.bricked ? a.take<long long>((size_t)m * ncomp) : nullptr;
   L.qe = P.bricked ? a.take<int16_t>((size_t)m * ncomp) : nullptr;
-  const int64_t nexp = P.bricked ? P.bg.enb[0] * P.bg.enb[1] * P.bg.enb[2] : 0;
-  L.ebrick = P.bricked ? a.take<uint32_t>((size_t)nexp * ncomp) : nullptr;
   return L;
+}
+
+// Clears the flag, the exponent bricks and the counts.
+gbg_status scatter_clear(const ScatterLayout &L, const ScatterPlan &P, cudaStream_t st) {
+  const char *from = reinterpret_cast<const char *>(L.flag), *to = reinterpret_cast<const char *>(L.counts + P.nkeys + 1);
+  GBG_CUDA_TRY(cudaMemsetAsync(L.flag, 0, (size_t)(to - from), st));
+  return GBG_OK;
 }
 
 int bits_for(uint64_t max_value) {
@@ -1524,12 +1532,9 @@ gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int 
   auto kernel = k_scatter_owner<T, N2, CC>;
   GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  int dev = 0, sms = 1, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem);
+  // two CTAs per SM, by the launch bounds and the shared memory's share (more would find no ticket left)
   const int64_t nbricks = bg.nb[0] * bg.nb[1] * bg.nb[2];
-  const int blocks = (int)std::min<int64_t>(nbricks, (int64_t)sms * std::max(per_sm, 1));
+  const int blocks = launch_blocks(nbricks, 1, 2);
   mark_main_start(st);
   kernel<<<blocks, kThreads, smem, st>>>(g, bg, ncomp, chunk, chunk1, (int)sums, L.counts,
                                          static_cast<const long long *>(L.rec), L.qi, L.qe, L.ebrick, wexp, field,
@@ -1547,9 +1552,6 @@ gbg_status launch_bricked(const GridT<T> &g, const ScatterPlan &P, const gbg_sch
   const SchemeT<T, N2> s = make_scheme<T, N2>(sch);
   const int wexp = fixed_weight_exp(sch);
   const int blocks_m = launch_blocks(m, kThreads);
-  const int64_t nexp = P.bg.enb[0] * P.bg.enb[1] * P.bg.enb[2];
-  GBG_CUDA_TRY(cudaMemsetAsync(L.ebrick, 0, sizeof(uint32_t) * (size_t)nexp * ncomp, st));
-  GBG_CUDA_TRY(cudaMemsetAsync(L.flag, 0, sizeof(uint32_t), st));
   k_brick_keys<T><<<blocks_m, kThreads, 0, st>>>(g, P.bg, x, m, L.keys, L.counts, L.rank, q, ncomp, T(alpha),
                                                  L.ebrick, status);
   note_launch();
@@ -1577,7 +1579,7 @@ gbg_status dispatch_scatter(const gbg_grid &grid, const gbg_scheme &sch, int nco
   const GridT<T> g = make_grid<T>(grid);
   const T *x = static_cast<const T *>(pos);
   T *f = static_cast<T *>(field);
-  GBG_CUDA_TRY(cudaMemsetAsync(L.counts, 0, sizeof(uint32_t) * (size_t)(P.nkeys + 1), st));
+  GBG_TRY(scatter_clear(L, P, st));
   if (P.bricked) {
     const T *qq = static_cast<const T *>(q);
     const int w = sch.stencil_width;
@@ -1592,7 +1594,6 @@ gbg_status dispatch_scatter(const gbg_grid &grid, const gbg_scheme &sch, int nco
 #undef GBG_BRICKED
   }
   const int64_t ncells = g.npf;
-  GBG_CUDA_TRY(cudaMemsetAsync(L.flag, 0, sizeof(uint32_t), st));
   const SchemeT<T, GBG_MAX_NODES> s = make_scheme<T, GBG_MAX_NODES>(sch);
   k_cell_keys<T><<<launch_blocks(m, kThreads), kThreads, 0, st>>>(g, x, m, L.keys, L.counts, L.rank, status);
   note_launch();
