@@ -301,3 +301,58 @@ def test_fp32_gather_rows(gbg, oracle, dev, n, m, ncomp, name):
                                            scheme.c(), out.data_ptr(), status.data_ptr(),
                                            torch.cuda.current_stream().cuda_stream), "gather")
     assert int(status.item()) == _lib.GBG_DEV_TRAVERSAL
+
+
+# every window width: odd and even, powers of two and not, held node tables (to 8) and not; grids no
+# longer than the window; the oracle's windowed transform with the same window
+@pytest.mark.parametrize("width", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 13, 16])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("comps", [1, 4])
+def test_window_gather_and_spread(gbg, dev, width, dtype, comps):
+    from gbgperiodicfields_gb300 import _lib
+    T = np.float64 if dtype == torch.float64 else np.float32
+    n, m = (9, 16, 12), 700
+    rng = np.random.default_rng(width)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, origin=(0.5, 0.0, -1.0), dtype=dtype)
+    pos = np.asfortranarray((np.array(grid.origin) + TWO_PI * (rng.random((m, 3)) * 2 - 0.5)).astype(T))
+    pos[:20] = np.array(grid.origin, T) + np.array(grid.grid_spacing, T) * rng.integers(0, 9, (20, 3)).astype(T)
+    f = np.asfortranarray(rng.standard_normal(n + (comps,)).astype(T))
+    q = np.asfortranarray(rng.standard_normal((m, comps)).astype(T))
+    beta = float(T(2.3) * T(width))
+    # the window's weights in the grid's type, as the reference rounds them, then 64-bit sums
+    o, d = np.array(grid.origin, T), np.array(grid.grid_spacing, T)
+    ci = (pos - o) / d
+    base = np.floor(ci).astype(np.int64)
+    t = ci - np.floor(ci)
+    half = np.where(t < T(0.5), (width + 1) // 2, width // 2) if width % 2 else np.full(t.shape, width // 2)
+    off = np.arange(1, width + 1) - half[..., None]
+    z = T(2) * (t[..., None] - off.astype(T)) / T(width)
+    w = np.exp(T(beta) * (np.sqrt(np.maximum(T(1) - z * z, T(0))) - T(1))).astype(np.float64)
+    at = (base[..., None] + off) % np.array(n)[:, None]
+    want, spread = np.zeros((m, comps)), np.zeros(n + (comps,))
+    for k in range(width):
+        for j in range(width):
+            for i in range(width):
+                x, y, zz = at[:, 0, i], at[:, 1, j], at[:, 2, k]
+                wt = w[:, 0, i] * w[:, 1, j] * w[:, 2, k]
+                want += wt[:, None] * f[x, y, zz]
+                np.add.at(spread, (x, y, zz), wt[:, None] * q)
+    lib, code = _lib.load(), _lib.GBG_F64 if dtype == torch.float64 else _lib.GBG_F32
+    import ctypes
+    stream, need = torch.cuda.current_stream().cuda_stream, ctypes.c_size_t()
+    fd, pd, qd = to_dev(f, dev), to_dev(pos, dev), to_dev(q, dev)
+    out, field = gbg.zeros_colmajor((m, comps), dtype, dev), gbg.zeros_colmajor(n + (comps,), dtype, dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    _lib.check(lib.gbg_nufft_interp_workspace_size(grid.c(), code, comps, m, width, ctypes.byref(need)))
+    ws = torch.empty(need.value, dtype=torch.uint8, device=dev)
+    _lib.check(lib.gbg_nufft_interp(grid.c(), code, comps, fd.data_ptr(), pd.data_ptr(), m, None, width, beta, out.data_ptr(),
+                                    ws.data_ptr(), ws.numel(), status.data_ptr(), stream))
+    _lib.check(lib.gbg_nufft_spread_workspace_size(grid.c(), code, comps, m, width, ctypes.byref(need)))
+    ws2 = torch.empty(need.value, dtype=torch.uint8, device=dev)
+    _lib.check(lib.gbg_nufft_spread(grid.c(), code, comps, field.data_ptr(), pd.data_ptr(), m, qd.data_ptr(), None, width,
+                                    beta, ws2.data_ptr(), ws2.numel(), status.data_ptr(), stream))
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    bar = 1e-12 if dtype == torch.float64 else 1e-5
+    assert relerr(out.cpu().numpy(), want) <= bar
+    assert relerr(field.cpu().numpy(), spread) <= bar
