@@ -356,3 +356,22 @@ def test_window_gather_and_spread(gbg, dev, width, dtype, comps):
     bar = 1e-12 if dtype == torch.float64 else 1e-5
     assert relerr(out.cpu().numpy(), want) <= bar
     assert relerr(field.cpu().numpy(), spread) <= bar
+
+
+# rows below, at and above a warp's width; a scatter of nothing with beta = 1 refreshes the ghosts of the
+# bricks it reaches and leaves every value
+@pytest.mark.parametrize("ncomp", [1, 3, 9, 12])
+@pytest.mark.parametrize("n", [(8, 9, 33), (65, 8, 10), (32, 33, 8)])
+def test_export_rows_and_refreshed_ghosts(gbg, dev, ncomp, n):
+    from gbgperiodicfields_gb300 import resident
+    rng = np.random.default_rng(3 * ncomp + n[0])
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    data = to_dev(np.asfortranarray(rng.standard_normal(n + (ncomp,))), dev).to(torch.float32)
+    field = resident.ResidentField(grid, ncomp, max_stencil_width=8).load(data)
+    pos = to_dev(np.asfortranarray(TWO_PI * rng.random((500, 3))), dev)
+    bins, scheme = resident.PointBins(grid, 500).build(pos), gbg.LalescuSpline(8)
+    before = resident.interpolate_binned(field, bins, scheme)
+    resident.anterpolate_binned(field, bins, scheme, torch.zeros_like(before), beta=1.0)
+    assert torch.equal(field.read(torch.float32), data)
+    assert torch.equal(field.read(torch.float64), data.double())
+    assert torch.equal(resident.interpolate_binned(field, bins, scheme), before)
