@@ -11,7 +11,7 @@
 // Bins: each position is split into a cell and a fraction.  For Float64 positions this
 // is done in FP64 (the precision form keeps FP64 only here): u = x*(N/L)*2^32 -
 // o*(N/L)*2^32 in one FMA, floor to int64, cell = (u >> 32) mod N, fraction = the low 32
-// bits.  Points are then stably radix-sorted by (brick, cell within brick).
+// bits.  Points are then sorted by (brick, cell within brick), in index order within a cell.
 //
 // Gather: one CTA per brick (persistent; the brick's TMA halo tile double-buffered when
 // that keeps as many CTAs per SM), a point per quarter-warp: lane (i, jj) owns the
@@ -1708,6 +1708,7 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
   }
   // a region that fits at once stages over the running sums' space too
   const bool one = count <= (uint32_t)g.chunk1;
+  constexpr uint32_t kVotePoints = 1024;  // the most points whose trips are voted (see there)
   const int P = one ? g.chunk1 : g.chunk;
   float *sq = one ? sacc : sacc + bvol * CP;
   float *sw = sq + P * CP;
@@ -1912,7 +1913,7 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
                 if (max(off[e0], c0) < min(off[e0 + N2], c1)) rows |= 1ull << (kk * 8 + jj);
               }
         }
-        if constexpr (CP > 4) {
+        if (CP > 4 && count <= kVotePoints) {
           const uint32_t weights = smem_addr(sw), quantities = smem_addr(sq);
           uint32_t wp = 0, wx = 0, wy = 0, wz = 0, qp = 0;  // the point's record, its weights, its quantities
           int left = 0, jj = 0, kk = 0;
@@ -1934,9 +1935,13 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
           // Twelve components: pairs of multiply-adds (24 issue slots a point instead of 48, the same bits),
           // and trips that are the warp's, held together by the vote: each takes one point of every lane
           // that has one left, and a lane whose row is done moves on within the trip.  512^3 x 12, 3.2e7
-          // points: 10.35 ms, 11.85 with the loop below.  With four components the loop below wins (128^3 x
-          // 3, 5e5 points, width 6: 336 us, 387 this way): a point's 16 multiply-adds are too few to pay for
-          // the pairs' weights and the vote.
+          // points: 10.15 ms, 11.85 with the loop below.  With more points in the region the rows are long
+          // enough for the loop below, and lanes in different rows cost more than they gain: 128^3 x 9 at
+          // width 4, mean points a region and us this way and below: 410, 193 and 231; 810, 346 and 395;
+          // 1620, 902 and 863; 3230, 1796 and 1581 -- at width 6: 650, 530 and 618; 1290, 1197 and 1183;
+          // 2580, 2296 and 2013.  With four components the loop below wins (128^3 x 3, 5e5 points, width 6:
+          // 336 us, 387 this way): a point's 16 multiply-adds are too few to pay for the pairs' weights and
+          // the vote.
           unsigned long long acc2[BY * BZ][CP / 2];
 #pragma unroll
           for (int n = 0; n < BY * BZ; ++n)

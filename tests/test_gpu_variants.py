@@ -375,3 +375,22 @@ def test_export_rows_and_refreshed_ghosts(gbg, dev, ncomp, n):
     assert torch.equal(field.read(torch.float32), data)
     assert torch.equal(field.read(torch.float64), data.double())
     assert torch.equal(resident.interpolate_binned(field, bins, scheme), before)
+
+
+# a brick's region with as many points as are taken in voted trips, one more, and several stagings
+@pytest.mark.parametrize("m", [1023, 1024, 1025, 4000])
+@pytest.mark.parametrize("ncomp,name", [(9, "cubic"), (12, "quintic"), (5, "octic")])
+def test_wide_scatter_either_side_of_the_vote(gbg, oracle, dev, m, ncomp, name):
+    from gbgperiodicfields_gb300 import resident
+    rng = np.random.default_rng(m + ncomp)
+    grid = gbg.Grid3D((32, 32, 32), (TWO_PI,) * 3)
+    scheme = {"cubic": gbg.CatmullRom, "quintic": gbg.LalescuSpline(6), "octic": gbg.LalescuSpline(8)}[name]
+    # all of them inside the second brick of every axis, cells 12 to 15
+    pos = np.asfortranarray(TWO_PI / 32 * (12 + 3.9 * rng.random((m, 3))))
+    q = np.asfortranarray(rng.standard_normal((m, ncomp)))
+    field = resident.ResidentField(grid, ncomp, max_stencil_width=8)
+    bins = resident.PointBins(grid, m).build(to_dev(pos, dev))
+    resident.anterpolate_binned(field, bins, scheme, to_dev(q, dev))
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    want = oracle.scatter(g, np.zeros((32, 32, 32, ncomp), order="F"), pos, q, scheme.coefficients)
+    assert relerr(field.read(torch.float64).cpu().numpy(), want) <= 1e-5
