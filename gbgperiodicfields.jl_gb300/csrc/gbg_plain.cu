@@ -1438,8 +1438,8 @@ gbg_status dispatch_gather(const gbg_grid &grid, const gbg_scheme &sch, int ncom
 
 // Which scatter runs, and its bricks: a thread per node of a brick whenever every axis is at least
 // a stencil wide, else the node pull (which also handles a stencil wider than the grid, reached
-// several times per node).  More than 22 components keep the pull, as their quantities' mantissas
-// and exponents would need more workspace than the pull's own copy of them.
+// several times per node).  More than 22 components (21 from width 7) keep the pull, as their
+// quantities' mantissas and exponents would need more workspace than the pull's own copy of them.
 struct ScatterPlan {
   bool bricked = false;
   BrickGeo bg{};
@@ -1453,7 +1453,7 @@ ScatterPlan plan_scatter(const gbg_grid &g, int ncomp, size_t esize, int n2) {
   // 14.5 ms where these took 12.8 (256^3 x 3, 1e7 points, 30% in blobs): more regions go in passes.
   const int base[3] = {8, 8, 4};
   const int ebase[3] = {(size_t)ncomp * esize > 24 ? 8 : 16, 8, 8};
-  bool wide_enough = n2 <= 8 && ncomp <= 22;
+  bool wide_enough = n2 <= 8 && ncomp <= (n2 < 7 ? 22 : 21);
   int64_t nbricks = 1;
   for (int d = 0; d < 3; ++d) {
     p.bg.b[d] = (int32_t)std::min<int64_t>(base[d], g.n[d]);
