@@ -305,7 +305,7 @@ def run_gb300(args, rank, world):
     avg = {k: float(np.mean(v)) for k, v in calls.items()}
     kavg = {k: float(np.mean(v)) for k, v in kernels.items()}
     alg = algorithmic_bytes(M3, C3, int(np.prod(N3)), 4)
-    kname = {"gather": "k_gather_staged4<4, 12, float>", "scatter": "k_scatter_nodes<4, 1, 12>"}
+    kname = {"gather": "k_gather_staged<4, 4, 12, float>", "scatter": "k_scatter_nodes<4, 1, 12>"}
     per_kernel = {k: {"kernel": kname[k], "ms": kavg[k], "algorithmic_bytes": alg[k],
                       "achieved": alg[k] / (kavg[k] / 1e3) / 1e9,
                       "frac": alg[k] / (kavg[k] / 1e3) / 1e9 / peak} for k in kavg}

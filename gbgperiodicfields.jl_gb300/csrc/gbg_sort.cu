@@ -1,10 +1,11 @@
-// Device prefix sum and stable LSD radix sort (sm_103a).
+// Device prefix sum, stable counting sort and stable LSD radix sort (sm_103a).
 //
 // The reference's traversal order is a counting sort whose placement goes through
 // atomics, so points within a tile land in an unspecified order
-// (Interpolation.jl:672-684).  Here the placement is a stable LSD radix sort of
-// (key, point index) pairs: within a key the points keep their index order, which makes
-// the order -- and every float sum that follows it -- identical run to run.
+// (Interpolation.jl:672-684).  Here both sorts are stable -- the traversal order's an LSD radix
+// sort of (key, point index) pairs, the bins' and the FP64 scatter's a counting sort: within a key
+// the points keep their index order, which makes the order -- and every float sum that follows it --
+// identical run to run.
 #include "gbg_common.cuh"
 
 namespace gbg {

@@ -134,7 +134,7 @@ gbg_status gbg_interpolate(const gbg_grid *grid, gbg_dtype dtype, int32_t ncomp,
  * field = alpha * W^T q + beta * field, with beta == 0 overwriting (NaN-safe).
  * Deterministic: the result is bitwise identical run to run and independent of the
  * traversal (points are sorted by brick and cell on the device and every brick sums its
- * nodes' contributions as 64-bit fixed-point integers, whose sum does not depend on the
+ * nodes' contributions as wide fixed-point integers, whose sum does not depend on the
  * order of the additions; no float atomics).  workspace: device scratch
  * of at least gbg_anterpolate_workspace_size bytes, or NULL (the library then takes
  * stream-ordered scratch with cudaMallocAsync and releases it before returning). */
@@ -447,7 +447,7 @@ gbg_status gbg_nufft_interp(const gbg_grid *fine, gbg_dtype dtype, int32_t ncomp
                             double beta, void *out, void *workspace, size_t workspace_bytes,
                             int32_t *device_status, void *stream);
 /* Device bytes of the spread's workspace: int64 node sums, the points' tiles, ranks and
- * window weights (about npf*ncomp*8 + npoints*(24 + 3*width*sizeof(dtype)) bytes). */
+ * FP64 window weights (about npf*ncomp*8 + npoints*24 bytes, and 24*width a point for FP64). */
 gbg_status gbg_nufft_spread_workspace_size(const gbg_grid *fine, gbg_dtype dtype, int32_t ncomp, int64_t npoints,
                                            int32_t width, size_t *bytes);
 /* Type 1 window spread -- _nufft_spread_kernel! (Interpolation.jl:1919-1950): field (on
