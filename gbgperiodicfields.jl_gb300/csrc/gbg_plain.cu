@@ -341,12 +341,17 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Fixed-point exponent P of the scatter's weights, w * 2^P: |w| <= L (the scheme's
-// Bernstein bound with evaluation slack) <= 1.5 * 2^lb, P = 61 - lb.  Then |w * 2^P| < 1.5 *
-// 2^61 (its high digit of 31 bits fits an int32), a product of two less its low 62 bits stays
-// below 2.25 * 2^60 and of three below 3.375 * 2^59.
-int fixed_weight_exp(const gbg_scheme &sch) {
-  const double L = weight_bound(sch, std::ldexp(1.0, -40));
+// The largest |w| of a scheme as a kernel in T evaluates it: the Bernstein bound, and the evaluation's
+// roundings (about two a power, each of sum |c| at most).
+template <typename T>
+double evaluated_weight_bound(const gbg_scheme &sch) {
+  return weight_bound(sch, sizeof(T) == 8 ? std::ldexp(1.0, -40) : std::ldexp((double)sch.num_powers, -23));
+}
+
+// Fixed-point exponent P of the scatter's weights, w * 2^P: |w| <= L (evaluated_weight_bound)
+// <= 1.5 * 2^lb, P = 61 - lb.  Then |w * 2^P| < 1.5 * 2^61 (its high digit of 31 bits fits an int32), a
+// product of two less its low 62 bits stays below 2.25 * 2^60 and of three below 3.375 * 2^59.
+int fixed_weight_exp(double L) {
   int lb = 0;
   while (1.5 * std::ldexp(1.0, lb) < L && lb < 60) ++lb;
   return 61 - lb;
@@ -845,8 +850,9 @@ constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 // lb, |w| <= 1.5 * 2^lb from the scheme's Bernstein bound), each product less its low 62 bits: w1 w2 w3
 // * 2^(3P - 124), to a few units of 2^-59 and below 2^61.  Cut in two digits, of 30 bits and the signed
 // rest, it meets the quantity's digits in
-// 2 ND products below 2^54, each added by one multiply-add to an accumulator of its own: no shifts
-// and no carries per contribution, and up to 511 points before one could overflow.  The accumulators
+// 2 ND products, each added by one multiply-add to an accumulator of its own: no shifts
+// and no carries per contribution, and no accumulator can overflow over the points of one staging
+// (owner_points).  The accumulators
 // are folded at their weights into a 192-bit sum, which holds any number of contributions exactly;
 // the only roundings of a node are those of its weights, the last window's end (2^-155 of the
 // region's largest contribution, or less) and the final conversion.  A non-finite quantity marks
@@ -857,7 +863,18 @@ constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 // a point and added to 128-bit sums in shared memory by four dependent atomics per contribution; 256^3
 // x 3, 1e7 points with 30% in blobs, cubic: 21.4 ms, now 10.5.  Three CTAs per SM (80 registers, which
 // spill) take 12.0.
-constexpr int kOwnerPoints = 508;  // staged points: at most 511 trips between folds
+constexpr int kOwnerPoints = 508;  // staged points, at most
+
+// The points that one staging may hold for weights up to L in P bits: a node adds each of them once to an
+// accumulator between folds.  The node weight, below L^3 2^(3P - 124), has a low digit below 2^30 and a high
+// one below h = L^3 2^(3P - 154) + 1, and meets digits below 2^24: no accumulator passes 2^63 in 2^39 / h
+// points.  508 for L <= 1.25 * 2^lb (the Lalescu and Lagrange splines, whose weights are at most one or a
+// little above), 300 for the largest weights of a caller's own scheme (and never below 256: weights past
+// 1.5 * 2^60, which no P holds, must not leave a staging without points).
+int owner_points(double L, int wexp) {
+  const double h = 1.001 * L * L * L * std::ldexp(1.0, 3 * wexp - 154) + 2.0;
+  return (int)std::max(256.0, std::min<double>(kOwnerPoints, std::ldexp(1.0, 39) / h)) & ~3;
+}
 
 // Shared words of a staged point: the digits of CC components and the meta word, in 16-byte units of
 // an odd count (or one), so that lanes reading neighbouring points meet different banks.
@@ -1518,8 +1535,8 @@ int bits_for(uint64_t max_value) {
 
 // The owner kernel for CC components at a time.
 template <typename T, int N2, int CC>
-gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int wexp, const ScatterLayout &L,
-                        T *field, double beta, cudaStream_t st) {
+gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int wexp, int points,
+                        const ScatterLayout &L, T *field, double beta, cudaStream_t st) {
   constexpr size_t per = kDigitWords<CC, kDigits<T>> * 4 + kWeightWords<N2> * 8 + 4;
   const BrickGeo &bg = P.bg;
   const size_t e[3] = {(size_t)bg.b[0] + N2 - 1, (size_t)bg.b[1] + N2 - 1, (size_t)bg.b[2] + N2 - 1};
@@ -1527,8 +1544,8 @@ gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int 
   const size_t sums = ((size_t)bg.bvol * CC * 24 + 15) & ~size_t(15);
   // an SM's 228 KB over the CTAs that the launch bounds ask for, less 1 KB reserved and the static part
   const size_t budget = 228 * 1024 / 2 - 1024 - 512;
-  const int chunk = (int)(std::min<size_t>(kOwnerPoints, (budget - tables - sums) / per) & ~size_t(3));
-  const int chunk1 = (int)(std::min<size_t>(kOwnerPoints, (budget - tables) / per) & ~size_t(3));
+  const int chunk = (int)(std::min<size_t>(points, (budget - tables - sums) / per) & ~size_t(3));
+  const int chunk1 = (int)(std::min<size_t>(points, (budget - tables) / per) & ~size_t(3));
   const size_t smem = std::max(sums + chunk * per, chunk1 * per) + tables;
   auto kernel = k_scatter_owner<T, N2, CC>;
   GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1551,7 +1568,8 @@ gbg_status launch_bricked(const GridT<T> &g, const ScatterPlan &P, const gbg_sch
                           const T *x, const T *q, int64_t m, double alpha, const ScatterLayout &L, T *field,
                           double beta, int32_t *status, cudaStream_t st) {
   const SchemeT<T, N2> s = make_scheme<T, N2>(sch);
-  const int wexp = fixed_weight_exp(sch);
+  const double bound = evaluated_weight_bound<T>(sch);
+  const int wexp = fixed_weight_exp(bound), points = owner_points(bound, wexp);
   const int blocks_m = launch_blocks(m, kThreads);
   k_brick_keys<T><<<blocks_m, kThreads, 0, st>>>(g, P.bg, x, m, L.keys, L.counts, L.rank, q, ncomp, T(alpha),
                                                  L.ebrick, status);
@@ -1565,8 +1583,8 @@ gbg_status launch_bricked(const GridT<T> &g, const ScatterPlan &P, const gbg_sch
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
   // three components share a point's weights and its trip; other counts go one at a time
-  return ncomp % 3 == 0 ? launch_owner<T, N2, 3>(g, P, ncomp, wexp, L, field, beta, st)
-                        : launch_owner<T, N2, 1>(g, P, ncomp, wexp, L, field, beta, st);
+  return ncomp % 3 == 0 ? launch_owner<T, N2, 3>(g, P, ncomp, wexp, points, L, field, beta, st)
+                        : launch_owner<T, N2, 1>(g, P, ncomp, wexp, points, L, field, beta, st);
 }
 
 // The deterministic scatter.  The brick scatter (integer sums, FP64-grade per node)

@@ -1,6 +1,10 @@
 """Edges of the kernels' variants: sizes around a tile, a word or a chunk, and the calls that a
 dispatch sends another way than their neighbours.  Integers are compared bitwise; the bars of
 computed values are the ones of the path's own parity tests."""
+import ctypes
+import math
+from fractions import Fraction
+
 import numpy as np
 import pytest
 import torch
@@ -394,3 +398,39 @@ def test_wide_scatter_either_side_of_the_vote(gbg, oracle, dev, m, ncomp, name):
     g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
     want = oracle.scatter(g, np.zeros((32, 32, 32, ncomp), order="F"), pos, q, scheme.coefficients)
     assert relerr(field.read(torch.float64).cpu().numpy(), want) <= 1e-5
+
+
+def _custom_scheme(gbg, coefficients):
+    """gbg_scheme_custom: a caller's own (nodes, powers) coefficient matrix."""
+    from gbgperiodicfields_gb300 import _lib, api
+    coef = np.asarray(coefficients, dtype=np.float64)
+    c = _lib.SchemeC()
+    flat = np.ascontiguousarray(coef.T).ravel()
+    _lib.check(_lib.load().gbg_scheme_custom(coef.shape[0], coef.shape[1],
+                                             flat.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), ctypes.byref(c)), "custom")
+    return api._SplineScheme(c)
+
+
+# Weights above one in the scatter's digit sums: as many equal points in one stencil as a staging, or a pass
+# of a crowded cell, can hold, on both sides of those sizes; sums that no rounding hides
+@pytest.mark.parametrize("width", [2, 4])
+@pytest.mark.parametrize("weight", [1.25, 1.3, 1.4, 1.5, 1.51, 2.9])
+@pytest.mark.parametrize("m", [300, 508, 600, 3000])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_scatter_sums_of_large_weights(gbg, dev, width, weight, m, dtype):
+    T = np.float64 if dtype == torch.float64 else np.float32
+    n = (8, 9, 10)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, dtype=dtype)
+    scheme = _custom_scheme(gbg, np.full((width, 1), weight))
+    pos = np.asfortranarray(np.full((m, 3), 2.0, dtype=T))
+    w = Fraction(float(T(weight)))
+    at = [(int(np.floor(2.0 / (TWO_PI / k))) - (width // 2 - 1) + np.arange(width)) % k for k in n]
+    for value in (0.3, -0.1, 0.7, 1.0 - 2.0 ** -40):
+        q = np.asfortranarray(np.full((m, 3), value, dtype=T))
+        got = _scatter_abi(gbg, grid, dev, np.zeros(n + (3,), T, order="F"), pos, q, scheme, 1.0, 0.0)
+        want = np.zeros(n + (3,))
+        want[np.ix_(*at, range(3))] = float(w ** 3 * Fraction(float(T(value))) * m)
+        # the sum of exact products rounded once; a weight's and the node weight's fixed point are below 2^-55
+        assert np.abs(got - want).max() <= (2.0 ** -51 if dtype == torch.float64 else 2.0 ** -23) * np.abs(want).max()
+
+
