@@ -834,8 +834,20 @@ __device__ __forceinline__ int2 lds64(uint32_t a) {
 // quantity of the region, window 0 holds q / 2^(e_r + 1 - 24 ND) down to its whole part (a signed top
 // digit, the others unsigned), window k the next 24 ND k bits below it.  Three digits keep a double
 // whole unless it is below 2^-18 of the region's largest, two a float below 2^-23: what is left
-// then makes further windows, up to kWindows, that are summed apart.
-constexpr int kDigit = 24, kWindows = 3;
+// then makes further windows, that are summed apart.  The last bit kept of any quantity is 2^(e_r + 1 - D),
+// to which it is rounded first (sum_depth): a region's sums are exact whole numbers of one unit.
+constexpr int kDigit = 24, kDepth = 144;
+
+// D for a region of count points: a node's sum of products of node weights (below 2^61) and quantities
+// (at most 2^(D - 1) units) has to fit 224 bits.
+__device__ __forceinline__ int sum_depth(uint32_t count) { return min(kDepth, 163 - (32 - __clz((int)count))); }
+
+// mq rounded to a multiple of 2^rc (ties up).
+__device__ __forceinline__ long long round_quantity(long long mq, int rc) {
+  if (rc <= 0) return mq;
+  return rc > 62 ? 0ll : ((mq + (1ll << (rc - 1))) >> rc) << rc;
+}
+
 template <typename T>
 constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 
@@ -853,9 +865,12 @@ constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 // 2 ND products, each added by one multiply-add to an accumulator of its own: no shifts
 // and no carries per contribution, and no accumulator can overflow over the points of one staging
 // (owner_points).  The accumulators
-// are folded at their weights into a 192-bit sum, which holds any number of contributions exactly;
-// the only roundings of a node are those of its weights, the last window's end (2^-155 of the
-// region's largest contribution, or less) and the final conversion.  A non-finite quantity marks
+// are folded at their weights into a 192-bit sum; where a region goes in several stagings or windows, these
+// are added, each shifted to the unit of the last bit kept, in 224 bits a node.  No bit is dropped between
+// the products and the final conversion, so the results depend neither on the order of the points nor on
+// how a region is cut.  The only roundings of a node are those of its weights, the quantities' last bit
+// (2^-143 of the region's largest, and a bit more for each doubling of a region past half a million points)
+// and the final conversion.  A non-finite quantity marks
 // every node its stencil reaches, which is written as NaN (the reference's 0 * NaN included).
 //
 // Bound by issue and by the latency of a brick's phases (at 256^3 x 3 and 6e6 uniform points half of its
@@ -960,6 +975,49 @@ __device__ __forceinline__ Int192 owner_fold(const long long (&A)[2 * ND]) {
   return s;
 }
 
+// A node's 224-bit sum (words at[0], at[plane], at[2 plane] and the signed top) += v * 2^shift; with shift
+// < 0 the bits that leave are zeros, the quantities having been rounded above them.
+__device__ __forceinline__ void add_sum(unsigned long long *at, int plane, uint32_t *top, Int192 v, int shift) {
+  unsigned long long s3 = (unsigned long long)((long long)v.s2 >> 63);
+  if (shift >= 64) {
+    s3 = v.s2;
+    v.s2 = v.s1;
+    v.s1 = v.s0;
+    v.s0 = 0ull;
+    shift -= 64;
+  }
+  if (shift > 0) {
+    s3 = (s3 << shift) | (v.s2 >> (64 - shift));
+    v.s2 = (v.s2 << shift) | (v.s1 >> (64 - shift));
+    v.s1 = (v.s1 << shift) | (v.s0 >> (64 - shift));
+    v.s0 <<= shift;
+  } else if (shift < 0) {
+    const int d = -shift;
+    v.s0 = (v.s0 >> d) | (v.s1 << (64 - d));
+    v.s1 = (v.s1 >> d) | (v.s2 << (64 - d));
+    v.s2 = (v.s2 >> d) | (s3 << (64 - d));
+  }
+  const unsigned long long a0 = at[0] + v.s0, c0 = a0 < v.s0;
+  const unsigned long long h1 = v.s1 + c0, a1 = at[plane] + h1, c1 = (unsigned long long)(h1 < c0) + (a1 < h1);
+  const unsigned long long h2 = v.s2 + c1, a2 = at[2 * plane] + h2, c2 = (unsigned long long)(h2 < c1) + (a2 < h2);
+  at[0] = a0;
+  at[plane] = a1;
+  at[2 * plane] = a2;
+  *top += (uint32_t)s3 + (uint32_t)c2;
+}
+
+// Such a sum as 192 bits: whole where it fits, else without its lowest 64 bits (bits -= 64), their
+// being there kept in the lowest one for the rounding.
+__device__ __forceinline__ Int192 leading_bits(const unsigned long long *at, int plane, uint32_t top, int &bits) {
+  Int192 s{at[0], at[plane], at[2 * plane]};
+  const long long s3 = (long long)(int)top;
+  if (s3 != ((long long)s.s2 >> 63)) {
+    s = Int192{s.s1 | (unsigned long long)(s.s0 != 0ull), s.s2, (unsigned long long)s3};
+    bits -= 64;
+  }
+  return s;
+}
+
 template <typename T, int N2, int CC>
 __global__ void __launch_bounds__(kThreads, 2)
     k_scatter_owner(GridT<T> g, BrickGeo bg, int ncomp, int chunk, int chunk1, int sums_bytes,
@@ -985,7 +1043,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint32_t *xe = kz + E2, *ye = xe + E0, *ze = ye + E1;                // per-axis exponent brick tables
   uint32_t *marked = ze + E2;                                          // bvol nodes' non-finite marks
   uint32_t *ereg = marked + bvol;                                      // ncomp region scales
-  unsigned long long *sums = reinterpret_cast<unsigned long long *>(smem_owner);  // bvol * CC 192-bit sums
+  // bvol * CC sums of 224 bits: three planes of 64 a component, then the signed tops
+  unsigned long long *sums = reinterpret_cast<unsigned long long *>(smem_owner);
+  uint32_t *tops = reinterpret_cast<uint32_t *>(sums + (size_t)3 * CC * bvol);
   const uint32_t nbricks = (uint32_t)(bg.nb[0] * bg.nb[1] * bg.nb[2]);
   const int n[3] = {(int)g.nx, (int)g.ny, (int)g.nz};
   const int tid = (int)threadIdx.x;
@@ -1049,24 +1109,27 @@ __global__ void __launch_bounds__(kThreads, 2)
     __syncthreads();
     const uint32_t count = block_scan_counts(off, ecount, warp_tot);
     if (tid == 0) off[ecount] = count;
+    const int depth = sum_depth(count);
     for (int cc0 = 0; cc0 < ncomp; cc0 += CC) {
       long long A[CC][2 * ND] = {};  // the products' accumulators, [weight digit * ND + quantity digit]
       auto inside = [&](int lx, int ly, int lz) -> bool {
         return bc[0] * B0 + lx < n[0] && bc[1] * B1 + ly < n[1] && bc[2] * B2 + lz < n[2];
       };
-      auto write = [&](int c, int lx, int ly, int lz, const Int192 &s, uint32_t marks) {
+      // a node's sum, in units of 2^(e_r + 1 - bits) times the node weight's
+      auto write = [&](int c, int lx, int ly, int lz, const Int192 &s, int bits, uint32_t marks) {
         const int e = (int)ereg[cc0 + c];
-        T v = e ? (T)to_double(s, (e - kEBias) + 1 - kDigit * ND + 124 - 3 * wexp) : T(0);
+        T v = e ? (T)to_double(s, (e - kEBias) + 1 - bits + 124 - 3 * wexp) : T(0);
         if ((marks >> c) & 1u) v = quiet_nan<T>();
         T *f = field + (bc[0] * B0 + lx) + g.nx * ((bc[1] * B1 + ly) + g.ny * (bc[2] * B2 + lz)) + g.npf * (cc0 + c);
         *f = beta_zero ? v : add_rn(mul_rn(beta, *f), v);
       };
-      // staging room for the whole region at once, or pieces beside the 192-bit sums
+      // staging room for the whole region at once, or pieces beside the nodes' sums
       bool multi = count > (uint32_t)chunk1, again;
       do {
         again = false;
         if (multi) {
           for (int i = tid; i < 3 * CC * bvol; i += blockDim.x) sums[i] = 0ull;
+          for (int i = tid; i < CC * bvol; i += blockDim.x) tops[i] = 0u;
           for (int i = tid; i < bvol; i += blockDim.x) marked[i] = 0u;
         }
         const int P = multi ? chunk : chunk1;
@@ -1104,7 +1167,7 @@ __global__ void __launch_bounds__(kThreads, 2)
           for (uint32_t c0 = 0; (c0 < total || (c0 == 0 && !multi)) && !again; c0 += (uint32_t)P) {
             const uint32_t c1 = min(total, c0 + (uint32_t)P);
             const int np = (int)(c1 - c0);
-            for (int win = 0; win < kWindows; ++win) {
+            for (int win = 0; win < kDepth / (kDigit * ND); ++win) {
               __syncthreads();  // the previous points are summed (and the offsets' end is set)
               if (win == 0) {
                 for (int e = tid, ex = ex0; e < ecount; e += blockDim.x) {
@@ -1135,9 +1198,11 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
                 for (int c = 0; c < CC; ++c) {
                   const int e = __ldg(qe + q0 + c);
-                  const long long mq = __ldg(qi + q0 + c);  // 0 for a zero or non-finite quantity
                   if (e == kENonFinite) meta |= 256u << c;
-                  const int r0 = 63 + (e ? max((int)ereg[cc0 + c] - e, 0) : 0) - kDigit * ND * (win + 1);
+                  const int drop = 63 + (e ? max((int)ereg[cc0 + c] - e, 0) : 0);  // bits of q below 2^(e_r + 1) in mq
+                  const int r0 = drop - kDigit * ND * (win + 1);
+                  // 0 for a zero or non-finite quantity
+                  const long long mq = round_quantity(__ldg(qi + q0 + c), drop - depth);
                   if (win == 0) {
                     // the mantissa's bits from r0 up: 24 (ND - 1) of them, and the signed rest above
                     const int rt = r0 + kDigit * (ND - 1);  // >= 39
@@ -1190,7 +1255,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const uint32_t marks = owner_walk<N2, CC, ND>(rows, po, ebase, E0, E1, nx0 + N2 - 1, c0, c1, digits, weights, A);
                 if (node)
 #pragma unroll
-                  for (int c = 0; c < CC; ++c) write(c, nx0, ny0, nz0, owner_fold<ND>(A[c]), marks >> 8);
+                  for (int c = 0; c < CC; ++c) write(c, nx0, ny0, nz0, owner_fold<ND>(A[c]), kDigit * ND, marks >> 8);
                 break;  // no window is left
               }
               // A crowded region's nodes differ much in their points (at a blob's edge tenfold within a
@@ -1239,31 +1304,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                 if (node && part < CC) {
                   const int nl = (lz * B1 + ly) * B0 + lx;
                   if (part == 0 && (marks >> 8)) marked[nl] |= marks >> 8;
-                  Int192 s = owner_fold<ND>(mine);
-                  for (int j = 0; j < win; ++j) {  // down to window 0's weight: 24 ND bits each
-                    constexpr int D = kDigit * ND;
-                    if constexpr (D >= 64) {
-                      s.s0 = (s.s1 >> (D - 64)) | (s.s2 << (128 - D));
-                      s.s1 = (unsigned long long)((long long)s.s2 >> (D - 64));
-                      s.s2 = (unsigned long long)((long long)s.s2 >> 63);
-                    } else {
-                      s.s0 = (s.s0 >> D) | (s.s1 << (64 - D));
-                      s.s1 = (s.s1 >> D) | (s.s2 << (64 - D));
-                      s.s2 = (unsigned long long)((long long)s.s2 >> D);
-                    }
-                  }
-                  unsigned long long *at = sums + (size_t)3 * part * bvol + nl;
-                  Int192 t{at[0], at[bvol], at[2 * bvol]};
-                  t.s0 += s.s0;
-                  unsigned long long cy = t.s0 < s.s0;
-                  const unsigned long long h = s.s1 + cy;
-                  cy = h < cy;
-                  t.s1 += h;
-                  cy += t.s1 < h;
-                  t.s2 += s.s2 + cy;
-                  at[0] = t.s0;
-                  at[bvol] = t.s1;
-                  at[2 * bvol] = t.s2;
+                  add_sum(sums + (size_t)3 * part * bvol + nl, bvol, tops + part * bvol + nl, owner_fold<ND>(mine),
+                          depth - kDigit * ND * (win + 1));
                 }
               }
               if (!left) break;
@@ -1278,8 +1320,9 @@ __global__ void __launch_bounds__(kThreads, 2)
           const int nl = (nz0 * B1 + ny0) * B0 + nx0;
 #pragma unroll
           for (int c = 0; c < CC; ++c) {
-            const unsigned long long *at = sums + (size_t)3 * c * bvol + nl;
-            write(c, nx0, ny0, nz0, Int192{at[0], at[bvol], at[2 * bvol]}, marked[nl]);
+            int bits = depth;
+            const Int192 sum = leading_bits(sums + (size_t)3 * c * bvol + nl, bvol, tops[c * bvol + nl], bits);
+            write(c, nx0, ny0, nz0, sum, bits, marked[nl]);
           }
         }
       }
@@ -1541,7 +1584,7 @@ gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int 
   const BrickGeo &bg = P.bg;
   const size_t e[3] = {(size_t)bg.b[0] + N2 - 1, (size_t)bg.b[1] + N2 - 1, (size_t)bg.b[2] + N2 - 1};
   const size_t tables = sizeof(uint32_t) * (4 * e[0] * e[1] * e[2] + 2 + 2 * (e[0] + e[1] + e[2]) + (size_t)bg.bvol + (size_t)ncomp);
-  const size_t sums = ((size_t)bg.bvol * CC * 24 + 15) & ~size_t(15);
+  const size_t sums = ((size_t)bg.bvol * CC * 28 + 15) & ~size_t(15);
   // an SM's 228 KB over the CTAs that the launch bounds ask for, less 1 KB reserved and the static part
   const size_t budget = 228 * 1024 / 2 - 1024 - 512;
   const int chunk = (int)(std::min<size_t>(points, (budget - tables - sums) / per) & ~size_t(3));

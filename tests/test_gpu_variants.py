@@ -434,3 +434,46 @@ def test_scatter_sums_of_large_weights(gbg, dev, width, weight, m, dtype):
         assert np.abs(got - want).max() <= (2.0 ** -51 if dtype == torch.float64 else 2.0 ** -23) * np.abs(want).max()
 
 
+# A region with one large quantity whose other nodes hold small ones only: those below the first window of
+# digits (2^-18 in FP64, 2^-23 in FP32 of the region's largest) and crowded ones, in any order of the points
+@pytest.mark.parametrize("small", [-20, -60, -90, -110])
+@pytest.mark.parametrize("m", [40, 300, 1500, 6000])
+@pytest.mark.parametrize("comps", [1, 3])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_scatter_of_small_quantities_beside_a_large_one(gbg, dev, small, m, comps, dtype):
+    T = np.float64 if dtype == torch.float64 else np.float32
+    n = (16, 16, 8)
+    rng = np.random.default_rng(m - small)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, dtype=dtype)
+    spacing = TWO_PI / np.array(n)
+    pos = np.concatenate([(1 + rng.random((m, 3))), [[6.5, 6.5, 2.5]]]) * spacing
+    q = np.concatenate([rng.standard_normal((m, comps)) * 2.0 ** small, np.ones((1, comps))])
+    pos, q = np.asfortranarray(pos.astype(T)), np.asfortranarray(q.astype(T))
+    zero = np.zeros(n + (comps,), T, order="F")
+    got = _scatter_abi(gbg, grid, dev, zero, pos, q, gbg.CatmullRom, 1.0, 0.0)
+    for _ in range(4):
+        order = rng.permutation(m + 1)
+        again = _scatter_abi(gbg, grid, dev, zero, pos[order], q[order], gbg.CatmullRom, 1.0, 0.0)
+        assert np.array_equal(got, again)
+    want = np.zeros(n + (comps,))
+    size, reach = _contribution_sizes(gbg.CatmullRom.coefficients, n, pos.astype(np.float64), q.astype(np.float64), spacing)
+    w = np.zeros((m + 1, 3, 4))
+    ci = pos.astype(np.float64) / spacing
+    base = np.floor(ci).astype(np.int64)
+    for p in range(3, -1, -1):
+        w = w * (ci - base)[..., None] + gbg.CatmullRom.coefficients[:, p]
+    parts = {}
+    for k in range(4):
+        for j in range(4):
+            for i in range(4):
+                wt = w[:, 0, i] * w[:, 1, j] * w[:, 2, k]
+                for p in range(m + 1):
+                    node = tuple((base[p, d] - 1 + s) % n[d] for d, s in enumerate((i, j, k)))
+                    parts.setdefault(node, []).append(wt[p] * q[p].astype(np.float64))
+    for node, terms in parts.items():
+        want[node] = [math.fsum(t[c] for t in terms) for c in range(comps)]
+    # the weights' own roundings (a dozen of T's per contribution, the locate's among them), the node weight's
+    # fixed point (its unit 2^-59, a few of them) and the quantities' last kept bit, 2^-143 of the largest
+    eps = 2.0 ** -53 if dtype == torch.float64 else 2.0 ** -24
+    bar = 64 * eps * (size + reach) + 4 * 2.0 ** -59 * reach + 2.0 ** -143 * (m + 1)
+    assert np.all(np.abs(got - want) <= bar)
