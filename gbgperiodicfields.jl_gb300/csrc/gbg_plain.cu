@@ -1496,10 +1496,33 @@ gbg_status dispatch_gather(const gbg_grid &grid, const gbg_scheme &sch, int ncom
   }
 }
 
+// Whether the brick scatter takes so many components.  Its quantities' mantissas and exponents need up to
+// twice the workspace of the pull's own copy of them, so the line is a part of the call's contract: a set
+// below it has integer sums whatever its type, a set above it the pull's workspace.  It is where the nodes
+// of an 8x8x8 brick, clipped to the grid, with 16 bytes a component and the tables of their region fill
+// 200 KB: 21 or 22 components on a grid of full bricks, 46 where an axis has 4 nodes.
+bool brick_takes(const gbg_grid &g, int ncomp, int n2) {
+  if (ncomp <= 20) return true;
+  size_t b[3], e[3];
+  for (int d = 0; d < 3; ++d) {
+    b[d] = (size_t)std::min<int64_t>(8, g.n[d]);
+    e[d] = b[d] + n2 - 1;
+  }
+  // the most stretches of consecutive cells along x in a row of any brick's region
+  size_t most = 1;
+  for (int64_t x0 = 0; x0 < g.n[0]; x0 += (int64_t)b[0]) {
+    size_t stretches = 0;
+    for (size_t i = 0; i < e[0]; ++i) stretches += i == 0 || imod(x0 - n2 / 2 + (int64_t)i, g.n[0]) % (int64_t)b[0] == 0;
+    most = std::max(most, stretches);
+  }
+  const size_t nodes = b[0] * b[1] * b[2], words = e[0] * e[1] * e[2] + e[1] * e[2] * most + 2 * 1024 + 2 * e[0] + e[1] +
+                                                   e[2] + nodes + 1 + most + (size_t)ncomp;
+  return nodes * ((size_t)ncomp * 16 + 4) + 4 * words <= 200 * 1024;
+}
+
 // Which scatter runs, and its bricks: a thread per node of a brick whenever every axis is at least
-// a stencil wide, else the node pull (which also handles a stencil wider than the grid, reached
-// several times per node).  More than 22 components (21 from width 7) keep the pull, as their
-// quantities' mantissas and exponents would need more workspace than the pull's own copy of them.
+// a stencil wide and the components are not too many (brick_takes), else the node pull (which also handles
+// a stencil wider than the grid, reached several times per node).
 struct ScatterPlan {
   bool bricked = false;
   BrickGeo bg{};
@@ -1513,7 +1536,7 @@ ScatterPlan plan_scatter(const gbg_grid &g, int ncomp, size_t esize, int n2) {
   // 14.5 ms where these took 12.8 (256^3 x 3, 1e7 points, 30% in blobs): more regions go in passes.
   const int base[3] = {8, 8, 4};
   const int ebase[3] = {(size_t)ncomp * esize > 24 ? 8 : 16, 8, 8};
-  bool wide_enough = n2 <= 8 && ncomp <= (n2 < 7 ? 22 : 21);
+  bool wide_enough = n2 <= 8;
   int64_t nbricks = 1;
   for (int d = 0; d < 3; ++d) {
     p.bg.b[d] = (int32_t)std::min<int64_t>(base[d], g.n[d]);
@@ -1524,7 +1547,7 @@ ScatterPlan plan_scatter(const gbg_grid &g, int ncomp, size_t esize, int n2) {
     if (g.n[d] < n2 || g.n[d] >= (int64_t(1) << 31)) wide_enough = false;
   }
   p.bg.bvol = (int64_t)p.bg.b[0] * p.bg.b[1] * p.bg.b[2];
-  p.bricked = wide_enough && nbricks * p.bg.bvol < (int64_t(1) << 32) - 1;
+  p.bricked = wide_enough && nbricks * p.bg.bvol < (int64_t(1) << 32) - 1 && brick_takes(g, ncomp, n2);
   p.nkeys = p.bricked ? nbricks * p.bg.bvol : g.n[0] * g.n[1] * g.n[2];
   return p;
 }

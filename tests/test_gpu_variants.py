@@ -477,3 +477,23 @@ def test_scatter_of_small_quantities_beside_a_large_one(gbg, dev, small, m, comp
     eps = 2.0 ** -53 if dtype == torch.float64 else 2.0 ** -24
     bar = 64 * eps * (size + reach) + 4 * 2.0 ** -59 * reach + 2.0 ** -143 * (m + 1)
     assert np.all(np.abs(got - want) <= bar)
+
+
+# more components than a full brick's line takes, on grids whose clipped bricks let them in: the integer sums do
+# not depend on how many components there are, so the first three are those of a deposit of three
+@pytest.mark.parametrize("n,width,comps", [((64, 64, 4), 4, 27), ((33, 4, 9), 4, 45), ((40, 2, 2), 2, 81), ((6, 7, 30), 6, 27),
+                                           ((64, 64, 4), 4, 23), ((30, 6, 50), 6, 24)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_scatter_of_many_components_on_thin_grids(gbg, dev, n, width, comps, dtype):
+    T = np.float64 if dtype == torch.float64 else np.float32
+    rng = np.random.default_rng(comps)
+    m = 20_000
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, dtype=dtype)
+    scheme = gbg.LalescuSpline(width) if width > 2 else gbg.LagrangeSpline(2)
+    pos = np.asfortranarray((TWO_PI * rng.random((m, 3))).astype(T))
+    q = np.asfortranarray((0.5 + rng.random((m, comps))).astype(T))
+    got = _scatter_abi(gbg, grid, dev, np.zeros(n + (comps,), T, order="F"), pos, q, scheme, 1.0, 0.0)
+    for c in range(0, comps, 3):
+        some = q[:, c:c + 3]
+        few = _scatter_abi(gbg, grid, dev, np.zeros(n + some.shape[1:], T, order="F"), pos, some, scheme, 1.0, 0.0)
+        assert np.array_equal(got[..., c:c + 3], few)
