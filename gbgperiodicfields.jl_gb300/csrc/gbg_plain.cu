@@ -29,7 +29,16 @@ struct GridT {
   T ox, oy, oz;  // T.(grid.origin)
   T dx, dy, dz;  // T.(grid.grid_spacing)
   T rx, ry, rz;  // their reciprocals, rounded once
+  bool recip;    // locate_recip's quotients are the divisions' (reciprocal_locates)
 };
+
+// Spacings whose reciprocal, and the products and residuals of locate_recip with it, stay in the normal range.
+// (2^-900 and 2^900: a quotient that matters, between 2^-53 and 2^63, has a residual above 2^-1022 there.)
+bool reciprocal_locates(const gbg_grid &g) {
+  for (int d = 0; d < 3; ++d)
+    if (!(g.spacing[d] >= std::ldexp(1.0, -900) && g.spacing[d] <= std::ldexp(1.0, 900))) return false;
+  return true;
+}
 
 template <typename T>
 GridT<T> make_grid(const gbg_grid &g) {
@@ -47,6 +56,7 @@ GridT<T> make_grid(const gbg_grid &g) {
   r.rx = T(1) / r.dx;
   r.ry = T(1) / r.dy;
   r.rz = T(1) / r.dz;
+  r.recip = reciprocal_locates(g);
   return r;
 }
 
@@ -646,7 +656,7 @@ __global__ void __launch_bounds__(kThreads)
        p += (int64_t)gridDim.x * blockDim.x) {
     int64_t b[3];
     T t[3];
-    const bool ok = locate3_recip(g, pos, p, m, b, t);
+    const bool ok = g.recip ? locate3_recip(g, pos, p, m, b, t) : locate3(g, pos, p, m, b, t);
     if (!ok && status) atomicOr(status, GBG_DEV_NONFINITE);
     // cells, bricks and keys fit 32 bits (fewer than 2^32 keys)
     uint32_t brick = 0, local = 0, eb = 0;
@@ -722,7 +732,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     int64_t b[3];
     T t[3];
-    const bool ok = locate3_recip(g, pos, p, m, b, t);
+    const bool ok = g.recip ? locate3_recip(g, pos, p, m, b, t) : locate3(g, pos, p, m, b, t);
     longlong2 *dst = reinterpret_cast<longlong2 *>(wts + sl * (3 * N2));  // 48, 96, 144 or 192 bytes a point
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -1478,7 +1488,8 @@ template <typename T>
 gbg_status dispatch_gather(const gbg_grid &grid, const gbg_scheme &sch, int ncomp, const void *field,
                            const void *pos, int64_t m, const int32_t *trav, void *out,
                            int32_t *status, cudaStream_t st) {
-  switch (sch.stencil_width) {
+  // the compiled widths' FP64 locate multiplies by the spacing's reciprocal; the run-time width's divides
+  switch (sizeof(T) == 4 || reciprocal_locates(grid) ? sch.stencil_width : 0) {
     case 2: return launch_gather<T, 2>(grid, sch, ncomp, field, pos, m, trav, out, status, st);
     case 4: return launch_gather<T, 4>(grid, sch, ncomp, field, pos, m, trav, out, status, st);
     case 6: return launch_gather<T, 6>(grid, sch, ncomp, field, pos, m, trav, out, status, st);

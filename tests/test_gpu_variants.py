@@ -497,3 +497,27 @@ def test_scatter_of_many_components_on_thin_grids(gbg, dev, n, width, comps, dty
         some = q[:, c:c + 3]
         few = _scatter_abi(gbg, grid, dev, np.zeros(n + some.shape[1:], T, order="F"), pos, some, scheme, 1.0, 0.0)
         assert np.array_equal(got[..., c:c + 3], few)
+
+
+# spacings whose reciprocal is no normal number: the same cells and fractions as on the grid scaled by a power
+# of two, so the same transfers
+@pytest.mark.parametrize("scale", [2.0 ** -1030, 2.0 ** -1010, 2.0 ** -880, 2.0 ** 880, 2.0 ** 1016])
+@pytest.mark.parametrize("width", [2, 4, 8])
+def test_spacings_without_a_normal_reciprocal(gbg, dev, scale, width):
+    n, m = (8, 9, 12), 500
+    rng = np.random.default_rng(width)
+    # positions and domain of few bits, whole at every scale
+    domain = (16.0, 18.0, 12.0)
+    pos = np.asfortranarray(rng.integers(-512, 1024, (m, 3)) / 64.0)
+    f = np.asfortranarray(rng.standard_normal(n + (3,)))
+    q = np.asfortranarray(rng.standard_normal((m, 3)))
+    scheme = gbg.LalescuSpline(width) if width > 2 else gbg.LagrangeSpline(2)
+    got = {}
+    for s in (1.0, scale):
+        grid = gbg.Grid3D(n, tuple(s * d for d in domain))
+        points = gbg.PointSet(to_dev(np.asfortranarray(pos * s), dev))
+        values = gbg.interpolate(gbg.VectorFieldPhysical(to_dev(f, dev), grid), points, scheme).data.cpu().numpy()
+        deposit = gbg.anterpolate(grid, points, gbg.VectorPointValues(to_dev(q, dev)), scheme).data.cpu().numpy()
+        got[s] = values, deposit
+    assert relerr(got[scale][0], got[1.0][0]) <= 1e-13  # another kernel's order of the same sums
+    assert np.array_equal(got[scale][1], got[1.0][1])
