@@ -600,6 +600,15 @@ struct BrickGeo {
   int64_t enb[3];
 };
 
+// A cell's key: the cells brick by brick, each brick's own x fastest, with no room for what a last brick
+// lacks (so that the counts of a grid take its cells' number of words, however thin it is).  Along an axis
+// cell c is cell l = c % b of its brick, the first of which is c - l, in an extent of v = min(b, n - c + l)
+// cells: the cells before the brick are v2 (v1 (c0 - l0) + (c1 - l1) n0) + (c2 - l2) n0 n1.
+__device__ __forceinline__ uint32_t cell_key(uint32_t n0, uint32_t n01, uint32_t f0, uint32_t f1, uint32_t f2, uint32_t l0,
+                                             uint32_t l1, uint32_t l2, uint32_t v0, uint32_t v1, uint32_t v2) {
+  return f2 * n01 + v2 * (f1 * n0 + v1 * f0) + (l2 * v1 + l1) * v0 + l0;
+}
+
 // A quantity as an exact integer mantissa and a binary exponent, from its bits: v = mq 2^(e - 62)
 // with 2^61 <= |mq| < 2^62.  The exponent is kept biased so that 0 means zero and kENonFinite (above
 // every finite one) a NaN or an infinity.
@@ -659,16 +668,17 @@ __global__ void __launch_bounds__(kThreads)
     const bool ok = g.recip ? locate3_recip(g, pos, p, m, b, t) : locate3(g, pos, p, m, b, t);
     if (!ok && status) atomicOr(status, GBG_DEV_NONFINITE);
     // cells, bricks and keys fit 32 bits (fewer than 2^32 keys)
-    uint32_t brick = 0, local = 0, eb = 0;
+    uint32_t f[3], l[3], v[3], eb = 0;
 #pragma unroll
     for (int d = 2; d >= 0; --d) {
-      const uint32_t c = (uint32_t)wrap_cell(b[d], n[d]);
-      const uint32_t bd = c / (uint32_t)bg.b[d];
-      brick = brick * (uint32_t)bg.nb[d] + bd;
-      local = local * (uint32_t)bg.b[d] + (c - bd * (uint32_t)bg.b[d]);
+      const uint32_t c = (uint32_t)wrap_cell(b[d], n[d]), bd = (uint32_t)bg.b[d];
+      f[d] = c / bd * bd;
+      l[d] = c - f[d];
+      v[d] = min(bd, (uint32_t)n[d] - f[d]);
       eb = eb * (uint32_t)bg.enb[d] + c / (uint32_t)bg.eb[d];
     }
-    const uint32_t key = brick * (uint32_t)bg.bvol + local;
+    const uint32_t key = cell_key((uint32_t)n[0], (uint32_t)n[0] * (uint32_t)n[1], f[0], f[1], f[2], l[0], l[1], l[2],
+                                  v[0], v[1], v[2]);
     keys[p] = key;
     rank[p] = atomicAdd(counts + key, 1u);
     for (int c = 0; c < ncomp; ++c) {
@@ -1049,8 +1059,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint32_t *r0s = off + ecount + 1;                                    // the cells' first slots
   uint32_t *poff = r0s + ecount;                                       // the same of one pass's share
   uint32_t *pr0 = poff + ecount + 1;
-  uint32_t *kx = pr0 + ecount, *ky = kx + E0, *kz = ky + E1;           // per-axis key tables
-  uint32_t *xe = kz + E2, *ye = xe + E0, *ze = ye + E1;                // per-axis exponent brick tables
+  uint32_t *fx = pr0 + ecount, *fy = fx + E0, *fz = fy + E1;           // per axis the first cell of a cell's brick
+  uint32_t *vx = fz + E2, *vy = vx + E0, *vz = vy + E1;                // its place in it, and the brick's extent
+  uint32_t *xe = vz + E2, *ye = xe + E0, *ze = ye + E1;                // per-axis exponent brick tables
   uint32_t *marked = ze + E2;                                          // bvol nodes' non-finite marks
   uint32_t *ereg = marked + bvol;                                      // ncomp region scales
   // bvol * CC sums of 224 bits: three planes of 64 a component, then the signed tops
@@ -1058,6 +1069,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint32_t *tops = reinterpret_cast<uint32_t *>(sums + (size_t)3 * CC * bvol);
   const uint32_t nbricks = (uint32_t)(bg.nb[0] * bg.nb[1] * bg.nb[2]);
   const int n[3] = {(int)g.nx, (int)g.ny, (int)g.nz};
+  const uint32_t n0 = (uint32_t)n[0], n01 = n0 * (uint32_t)n[1];
   const int tid = (int)threadIdx.x;
   // a thread's node; a warp's are a block of 4x4x2 in a full brick, so that its lanes' stencils overlap
   // and their point counts differ little
@@ -1089,10 +1101,9 @@ __global__ void __launch_bounds__(kThreads, 2)
       const int e = t - (d == 0 ? 0 : (d == 1 ? E0 : E0 + E1));
       int c = (bc[d] * bg.b[d] - half + e) % n[d];
       if (c < 0) c += n[d];
-      const uint32_t cb = (uint32_t)c / (uint32_t)bg.b[d], cl = (uint32_t)c - cb * (uint32_t)bg.b[d];
-      if (d == 0) kx[e] = cb * (uint32_t)bvol + cl;
-      else if (d == 1) ky[e] = cb * (uint32_t)bg.nb[0] * (uint32_t)bvol + cl * (uint32_t)B0;
-      else kz[e] = cb * (uint32_t)(bg.nb[1] * bg.nb[0]) * (uint32_t)bvol + cl * (uint32_t)(B0 * B1);
+      const uint32_t cl = (uint32_t)c % (uint32_t)bg.b[d];
+      fx[t] = (uint32_t)c - cl;
+      vx[t] = cl | (uint32_t)min(bg.b[d], n[d] - c + (int)cl) << 8;
       // the exponent brick of the cell, marked where the axis enters one
       const uint32_t eb = (uint32_t)c / (uint32_t)bg.eb[d], before = (uint32_t)(c ? c - 1 : n[d] - 1) / (uint32_t)bg.eb[d];
       const uint32_t step = d == 0 ? 1u : (uint32_t)(d == 1 ? bg.enb[0] : bg.enb[0] * bg.enb[1]);
@@ -1102,7 +1113,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     // the cells, and each component's scale: the largest exponent of the exponent bricks that hold a
     // cell of the region
     for (int e = tid, ex = ex0, ey = ey0, ez = ez0; e < ecount; e += blockDim.x) {
-      const uint32_t key = kx[ex] + ky[ey] + kz[ez];
+      const uint32_t lx = vx[ex], ly = vy[ey], lz = vz[ez];
+      const uint32_t key = cell_key(n0, n01, fx[ex], fy[ey], fz[ez], lx & 0xffu, ly & 0xffu, lz & 0xffu, lx >> 8, ly >> 8, lz >> 8);
       const uint32_t a = __ldg(cell_start + key);
       r0s[e] = a;
       off[e] = __ldg(cell_start + key + 1) - a;
@@ -1519,11 +1531,14 @@ bool brick_takes(const gbg_grid &g, int ncomp, int n2) {
     b[d] = (size_t)std::min<int64_t>(8, g.n[d]);
     e[d] = b[d] + n2 - 1;
   }
-  // the most stretches of consecutive cells along x in a row of any brick's region
+  // the most stretches of consecutive cells along x in a row of any brick's region (only the first and the
+  // last two bricks' regions reach over the grid's end; the others are alike)
   size_t most = 1;
-  for (int64_t x0 = 0; x0 < g.n[0]; x0 += (int64_t)b[0]) {
+  const int64_t bricks = (g.n[0] + (int64_t)b[0] - 1) / (int64_t)b[0];
+  for (int64_t k = 0; k < bricks; k = (k == 3 ? std::max<int64_t>(4, bricks - 3) : k + 1)) {
     size_t stretches = 0;
-    for (size_t i = 0; i < e[0]; ++i) stretches += i == 0 || imod(x0 - n2 / 2 + (int64_t)i, g.n[0]) % (int64_t)b[0] == 0;
+    for (size_t i = 0; i < e[0]; ++i)
+      stretches += i == 0 || imod(k * (int64_t)b[0] - n2 / 2 + (int64_t)i, g.n[0]) % (int64_t)b[0] == 0;
     most = std::max(most, stretches);
   }
   const size_t nodes = b[0] * b[1] * b[2], words = e[0] * e[1] * e[2] + e[1] * e[2] * most + 2 * 1024 + 2 * e[0] + e[1] +
@@ -1547,19 +1562,16 @@ ScatterPlan plan_scatter(const gbg_grid &g, int ncomp, size_t esize, int n2) {
   // 14.5 ms where these took 12.8 (256^3 x 3, 1e7 points, 30% in blobs): more regions go in passes.
   const int base[3] = {8, 8, 4};
   const int ebase[3] = {(size_t)ncomp * esize > 24 ? 8 : 16, 8, 8};
-  bool wide_enough = n2 <= 8;
-  int64_t nbricks = 1;
+  p.nkeys = g.n[0] * g.n[1] * g.n[2];
+  p.bricked = n2 <= 8 && p.nkeys < (int64_t(1) << 32) - 1 && brick_takes(g, ncomp, n2);
   for (int d = 0; d < 3; ++d) {
     p.bg.b[d] = (int32_t)std::min<int64_t>(base[d], g.n[d]);
     p.bg.nb[d] = (g.n[d] + p.bg.b[d] - 1) / p.bg.b[d];
     p.bg.eb[d] = (int32_t)std::min<int64_t>(ebase[d], g.n[d]);
     p.bg.enb[d] = (g.n[d] + p.bg.eb[d] - 1) / p.bg.eb[d];
-    nbricks *= p.bg.nb[d];
-    if (g.n[d] < n2 || g.n[d] >= (int64_t(1) << 31)) wide_enough = false;
+    if (g.n[d] < n2 || g.n[d] >= (int64_t(1) << 31)) p.bricked = false;
   }
   p.bg.bvol = (int64_t)p.bg.b[0] * p.bg.b[1] * p.bg.b[2];
-  p.bricked = wide_enough && nbricks * p.bg.bvol < (int64_t(1) << 32) - 1 && brick_takes(g, ncomp, n2);
-  p.nkeys = p.bricked ? nbricks * p.bg.bvol : g.n[0] * g.n[1] * g.n[2];
   return p;
 }
 
@@ -1617,7 +1629,7 @@ gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int 
   constexpr size_t per = kDigitWords<CC, kDigits<T>> * 4 + kWeightWords<N2> * 8 + 4;
   const BrickGeo &bg = P.bg;
   const size_t e[3] = {(size_t)bg.b[0] + N2 - 1, (size_t)bg.b[1] + N2 - 1, (size_t)bg.b[2] + N2 - 1};
-  const size_t tables = sizeof(uint32_t) * (4 * e[0] * e[1] * e[2] + 2 + 2 * (e[0] + e[1] + e[2]) + (size_t)bg.bvol + (size_t)ncomp);
+  const size_t tables = sizeof(uint32_t) * (4 * e[0] * e[1] * e[2] + 2 + 3 * (e[0] + e[1] + e[2]) + (size_t)bg.bvol + (size_t)ncomp);
   const size_t sums = ((size_t)bg.bvol * CC * 28 + 15) & ~size_t(15);
   // an SM's 228 KB over the CTAs that the launch bounds ask for, less 1 KB reserved and the static part
   const size_t budget = 228 * 1024 / 2 - 1024 - 512;

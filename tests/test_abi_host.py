@@ -182,3 +182,21 @@ def test_displacement_refusals(gbg):
     bad.domain[1] = -1.0
     assert lib.gbg_points_displace(bad, 2, 1, 1, 10, 0, None, None, None) == gbg._lib.GBG_EARG
     assert lib.gbg_points_displace(None, 2, 1, 1, 0, 0, None, None, None) == gbg._lib.GBG_OK
+
+
+@pytest.mark.parametrize("n", [(1700, 1700, 5), (1500, 1500, 7), (13, 1100, 1100), (1100, 9, 1300), (2500, 2500, 2), (251, 251, 251)])
+@pytest.mark.parametrize("m", [1, 500])
+def test_scatter_workspace_of_thin_grids(gbg, n, m):
+    # a word a cell however little of its last brick an axis fills, so that few points on 14 million cells fit the
+    # fixed scratch of the allocation-free form
+    nbytes = ctypes.c_size_t()
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    lib = gbg._lib.load()
+    width = 2 if min(n) < 4 else 4
+    gbg._lib.check(lib.gbg_anterpolate_workspace_size(grid.c(), gbg._lib.GBG_F64, 3, m, gbg.LagrangeSpline(width).c(),
+                                                      ctypes.byref(nbytes)), "workspace")
+    cells = np.prod(n)
+    # the counts, the largest exponent of 3 components per 16x8x8 cells, a point's records, and the alignment of each part
+    exponents = 3 * np.prod([-(-a // min(a, b)) for a, b in zip(n, (16, 8, 8))])
+    assert nbytes.value <= 4 * (cells + 1 + exponents) + m * 256 + 16 * 1024
+    assert nbytes.value <= 64 << 20
