@@ -17,7 +17,6 @@ There is no CPU path: host tensors are refused.
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes
 import math
 import threading
@@ -569,50 +568,74 @@ def _check_traversal(traversal, m: int, device):
 
 
 class _StatusWord:
-    """A word of pinned host memory that the kernels of a synchronous call report into (GBG_DEV_*
-    bits): no fill before the launch and no copy back after it, only the call's own wait for its
-    stream.  One per thread; a thread has one such call in flight at a time."""
+    """A word of pinned host memory that kernels report into (GBG_DEV_* bits): no fill before a launch and no
+    copy back after it.  stream: the one whose kernels hold the word, or None; a word given up while it is held
+    (its call cut short by a signal's exception) is waited for before its memory can serve another."""
 
     def __init__(self):
+        self.stream = None
         self.word = torch.zeros(1, dtype=torch.int32, pin_memory=True)
         self.value = self.word.numpy()
+        self.address = self.word.data_ptr()
 
-    def data_ptr(self):
-        return self.word.data_ptr()
-
-
-_status_words = threading.local()
-
-
-def _status_word() -> _StatusWord:
-    """This thread's status word, cleared."""
-    word = getattr(_status_words, "word", None)
-    if word is None:
-        word = _status_words.word = _StatusWord()
-    word.value[0] = 0
-    return word
+    def __del__(self):
+        if self.stream is not None:
+            try:
+                self.stream.synchronize()
+            except Exception:
+                pass
 
 
-def _on_device(t: torch.Tensor):
-    """A context in which t's device is current (none where it is already)."""
-    return torch.cuda.device(t.device) if t.device.index != torch.cuda.current_device() else contextlib.nullcontext()
+class _FreeWords(threading.local):
+    """The status words that are free, thread by thread (one, unless a call ran inside another)."""
+
+    def __init__(self):
+        self.free = []
 
 
-def _check_launched(st: int, what: str, stream):
-    """_lib.check; a call that failed half-way is waited for first, as its kernels hold the status word."""
-    if st != _lib.GBG_OK:
-        stream.synchronize()
-    _lib.check(st, what)
+_status_words = _FreeWords()
 
 
-def _raise_device_status(status: _StatusWord):
-    """The device's report, read after the call's stream has been waited for."""
-    v = int(status.value[0])
-    if v & _lib.GBG_DEV_NONFINITE:
-        raise InexactError("a non-finite or out-of-range position reached the locate step "
-                           "(floor(Int, x) of a non-finite coordinate)")
-    if v & _lib.GBG_DEV_TRAVERSAL:
-        raise ArgumentError("a traversal entry outside 1:M reached the device")
+class _launched_on:
+    """A synchronous call's launches, as a context: t's device is current, `stream` is its current stream,
+    `status` the address of a cleared word of the call's own.  The context ends when the stream has been waited
+    for, however its body ended, and raise_status() tells what the kernels reported."""
+
+    __slots__ = ("device", "stream", "word", "status", "reported")
+
+    def __init__(self, t: torch.Tensor):
+        if t.device.index == torch.cuda.current_device():
+            self.device, self.stream = None, torch.cuda.current_stream()
+        else:
+            self.device, self.stream = torch.cuda.device(t.device), torch.cuda.current_stream(t.device)
+
+    def __enter__(self):
+        free = _status_words.free
+        word = self.word = free.pop() if free else _StatusWord()
+        word.value[0] = 0
+        word.stream = self.stream
+        self.status = word.address
+        if self.device is not None:
+            self.device.__enter__()
+        return self
+
+    def __exit__(self, *error):
+        word = self.word
+        try:
+            self.stream.synchronize()
+            self.reported = int(word.value[0])
+            word.stream = None
+            _status_words.free.append(word)
+        finally:
+            if self.device is not None:
+                self.device.__exit__(*error)
+
+    def raise_status(self):
+        if self.reported & _lib.GBG_DEV_NONFINITE:
+            raise InexactError("a non-finite or out-of-range position reached the locate step "
+                               "(floor(Int, x) of a non-finite coordinate)")
+        if self.reported & _lib.GBG_DEV_TRAVERSAL:
+            raise ArgumentError("a traversal entry outside 1:M reached the device")
 
 
 def interpolate_(out: AbstractPointValues, field: AbstractFieldPhysical, points: PointSet, scheme,
@@ -630,16 +653,13 @@ def interpolate_(out: AbstractPointValues, field: AbstractFieldPhysical, points:
     trav = _check_traversal(traversal, m, field.data.device)
     if m == 0:
         return out
-    status = _status_word()
-    with _on_device(field.data):
-        stream = torch.cuda.current_stream()
+    with _launched_on(field.data) as call:
         st = _lib.load().gbg_interpolate(
             field.grid.c(), _DTYPE_CODE[field.data.dtype], field.ncomp, field.data.data_ptr(),
             points.positions.data_ptr(), m, trav.data_ptr() if trav is not None else None,
-            scheme.c(), out.data.data_ptr(), status.data_ptr(), stream.cuda_stream)
-        _check_launched(st, "interpolate!", stream)
-        stream.synchronize()
-    _raise_device_status(status)
+            scheme.c(), out.data.data_ptr(), call.status, call.stream.cuda_stream)
+        _lib.check(st, "interpolate!")
+    call.raise_status()
     return out
 
 
@@ -670,24 +690,21 @@ def anterpolate_(field: AbstractFieldPhysical, points: PointSet, quantities: Abs
     _check_colocation(field, points, quantities)
     m = points.npoints
     trav = _check_traversal(traversal, m, field.data.device)
-    status = _status_word()
     nbytes = ctypes.c_size_t()
     lib = _lib.load()
     _lib.check(lib.gbg_anterpolate_workspace_size(field.grid.c(), _DTYPE_CODE[field.data.dtype], field.ncomp,
                                                   m, scheme.c(), ctypes.byref(nbytes)), "anterpolate!")
     # scratch from torch's caching allocator, so repeated calls do not re-allocate
     ws = torch.empty(max(int(nbytes.value), 1), dtype=torch.uint8, device=field.data.device)
-    with _on_device(field.data):
-        stream = torch.cuda.current_stream()
+    with _launched_on(field.data) as call:
         st = lib.gbg_anterpolate(
             field.grid.c(), _DTYPE_CODE[field.data.dtype], field.ncomp, field.data.data_ptr(),
             points.positions.data_ptr() if m else None, m,
             quantities.data.data_ptr() if m else None, trav.data_ptr() if trav is not None else None,
-            scheme.c(), float(alpha), float(beta), ws.data_ptr(), ws.numel(), status.data_ptr(),
-            stream.cuda_stream)
-        _check_launched(st, "anterpolate!", stream)
-        stream.synchronize()
-    _raise_device_status(status)
+            scheme.c(), float(alpha), float(beta), ws.data_ptr(), ws.numel(), call.status,
+            call.stream.cuda_stream)
+        _lib.check(st, "anterpolate!")
+    call.raise_status()
     return field
 
 

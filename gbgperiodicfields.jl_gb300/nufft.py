@@ -29,8 +29,8 @@ import torch
 
 from . import _lib
 from ._lib import ArgumentError, DimensionMismatch, MethodError
-from .api import (AbstractPointValues, AbstractTransferScheme, Grid3D, PointSet, PointTraversalOrder, _DTYPE_CODE, _check_launched,
-                  _check_npoints_match, _check_traversal, _on_device, _raise_device_status, _require_cuda, _status_word, colmajor, empty_colmajor)
+from .api import (AbstractPointValues, AbstractTransferScheme, Grid3D, PointSet, PointTraversalOrder, _DTYPE_CODE,
+                  _check_npoints_match, _check_traversal, _launched_on, _require_cuda, colmajor, empty_colmajor)
 
 _COMPLEX = {torch.float32: torch.complex64, torch.float64: torch.complex128}
 _REAL = {torch.complex64: torch.float32, torch.complex128: torch.float64}
@@ -466,22 +466,19 @@ def interpolate_nufft_(out: AbstractPointValues, field: AbstractFieldSpectral, p
     phys = _fft_inverse(spec, fine.grid_size, layout)
     if m == 0:
         return out
-    status = _status_word()
     lib = _lib.load()
     nbytes = ctypes.c_size_t()
     _lib.check(lib.gbg_nufft_interp_workspace_size(fine.c(), _DTYPE_CODE[fine.dtype], field.ncomp, m, scheme.width,
                                                    ctypes.byref(nbytes)), "interpolate!")
     ws = torch.empty(int(nbytes.value), dtype=torch.uint8, device=field.data.device)
-    with _on_device(field.data):
-        stream = torch.cuda.current_stream()
+    with _launched_on(field.data) as call:
         st = lib.gbg_nufft_interp(fine.c(), _DTYPE_CODE[fine.dtype], field.ncomp, phys.data_ptr(),
                                   points.positions.data_ptr(), m,
                                   trav.data_ptr() if trav is not None else None, scheme.width, scheme.beta,
-                                  out.data.data_ptr(), ws.data_ptr(), ws.numel(), status.data_ptr(),
-                                  stream.cuda_stream)
-        _check_launched(st, "interpolate!", stream)
-        stream.synchronize()
-    _raise_device_status(status)
+                                  out.data.data_ptr(), ws.data_ptr(), ws.numel(), call.status,
+                                  call.stream.cuda_stream)
+        _lib.check(st, "interpolate!")
+    call.raise_status()
     return out
 
 
@@ -506,17 +503,14 @@ def anterpolate_nufft_(field: AbstractFieldSpectral, points: PointSet, quantitie
     _lib.check(lib.gbg_nufft_spread_workspace_size(fine.c(), _DTYPE_CODE[fine.dtype], field.ncomp, m, scheme.width,
                                                    ctypes.byref(nbytes)), "anterpolate!")
     ws = torch.empty(int(nbytes.value), dtype=torch.uint8, device=dev)
-    status = _status_word()
-    with _on_device(field.data):
-        stream = torch.cuda.current_stream()
+    with _launched_on(field.data) as call:
         st = lib.gbg_nufft_spread(fine.c(), _DTYPE_CODE[fine.dtype], field.ncomp, phys.data_ptr(),
                                   points.positions.data_ptr() if m else None, m,
                                   quantities.data.data_ptr() if m else None,
                                   trav.data_ptr() if trav is not None else None, scheme.width, scheme.beta,
-                                  ws.data_ptr(), ws.numel(), status.data_ptr(), stream.cuda_stream)
-        _check_launched(st, "anterpolate!", stream)
-        stream.synchronize()
-    _raise_device_status(status)
+                                  ws.data_ptr(), ws.numel(), call.status, call.stream.cuda_stream)
+        _lib.check(st, "anterpolate!")
+    call.raise_status()
     spec = _fft_forward(phys, layout)
     coarse = torch.zeros(field_spectral_shape(scheme.reference_grid, layout, R), dtype=field.data.dtype, device=dev)
     px, py, pz = scheme._pairs()

@@ -521,3 +521,77 @@ def test_spacings_without_a_normal_reciprocal(gbg, dev, scale, width):
         got[s] = values, deposit
     assert relerr(got[scale][0], got[1.0][0]) <= 1e-13  # another kernel's order of the same sums
     assert np.array_equal(got[scale][1], got[1.0][1])
+
+
+def _bad_and_good(gbg, dev, m):
+    """A gather whose every position is non-finite, and one of a single point."""
+    grid = gbg.Grid3D((16, 16, 16), (TWO_PI,) * 3)
+    field = gbg.ScalarFieldPhysical(to_dev(np.ones((16, 16, 16)), dev), grid)
+    bad = gbg.PointSet(to_dev(np.full((m, 3), np.nan), dev))
+    good = gbg.PointSet(to_dev(np.full((1, 3), 1.0), dev))
+    out = {p: gbg.ScalarPointValues(gbg.empty_colmajor((p.npoints,), torch.float64, dev)) for p in (bad, good)}
+    return [lambda p=p: gbg.interpolate_(out[p], field, p, gbg.CatmullRom) for p in (bad, good)]
+
+
+def test_status_of_a_call_cut_short_reaches_no_later_call(gbg, dev, monkeypatch):
+    from gbgperiodicfields_gb300 import _lib
+    bad, good = _bad_and_good(gbg, dev, 3_000_000)
+    good()
+    check = _lib.check
+
+    def interrupted(st, what):
+        monkeypatch.setattr(_lib, "check", check)
+        raise KeyboardInterrupt  # as a signal between the launch and the wait
+
+    for _ in range(5):
+        monkeypatch.setattr(_lib, "check", interrupted)
+        with pytest.raises(KeyboardInterrupt):
+            bad()
+        good()
+        with pytest.raises(gbg.InexactError):
+            bad()
+        good()
+
+
+def test_status_of_a_call_inside_another(gbg, dev, monkeypatch):
+    from gbgperiodicfields_gb300 import _lib
+    bad, good = _bad_and_good(gbg, dev, 100)
+    check = _lib.check
+
+    def nested(inner):
+        def run(st, what):
+            monkeypatch.setattr(_lib, "check", check)
+            torch.cuda.synchronize()
+            inner()
+            return check(st, what)
+        return run
+
+    monkeypatch.setattr(_lib, "check", nested(good))
+    with pytest.raises(gbg.InexactError):
+        bad()
+    good()
+
+
+def test_status_by_thread(gbg, dev):
+    import threading
+    calls = [_bad_and_good(gbg, dev, 50_000) for _ in range(4)]
+    wrong = []
+
+    def work(k):
+        bad, good = calls[k]
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(40):
+                try:
+                    (bad if (i + k) % 2 else good)()
+                    reported = False
+                except gbg.InexactError:
+                    reported = True
+                if reported != bool((i + k) % 2):
+                    wrong.append((k, i))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
