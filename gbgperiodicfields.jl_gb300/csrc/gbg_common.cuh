@@ -73,6 +73,16 @@ __device__ __forceinline__ long long fixed_rn(double x, int e) {
   return (b >> 63) ? -(long long)r : (long long)r;
 }
 
+// Reports bits into a caller's status word (or nowhere).  The word may lie in host memory, so the lanes that
+// report together send one atomic, and none where the bits are there already: a deposit whose every point is bad
+// reads the word once a warp instead of sending a million atomics over the host's link (1e7 points with three
+// non-finite quantities, deposited: 22.9 ms with an atomic each).
+__device__ __forceinline__ void report(int32_t *status, int32_t bits) {
+  if (!status) return;
+  const int first = __ffs((int)__activemask()) - 1;
+  if ((int)(threadIdx.x & 31u) == first && (*static_cast<volatile int32_t *>(status) & bits) != bits) atomicOr(status, bits);
+}
+
 // Adds v to a 64-bit integer kept in shared memory as two 32-bit words, lo[i] and hi[i],
 // with native 32-bit atomics: the low word's add returns the old value, whose wrap is the
 // carry into the high word.  Each add wraps the low word at most once, so after all adds

@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kThreads)
     int64_t b[3];
     T t[3];
     const bool ok = g.recip ? locate3_recip(g, pos, p, m, b, t) : locate3(g, pos, p, m, b, t);
-    if (!ok && status) atomicOr(status, GBG_DEV_NONFINITE);
+    if (!ok) report(status, GBG_DEV_NONFINITE);
     // cells, bricks and keys fit 32 bits (fewer than 2^32 keys)
     uint32_t f[3], l[3], v[3], eb = 0;
 #pragma unroll
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(kThreads)
       long long mq;
       const int e = split_quantity(mul_rn(alpha, __ldg(q + p + m * c)), mq);  // quantity = T(alpha)*q
       if (e == kENonFinite) {
-        if (status) atomicOr(status, GBG_DEV_NONFINITE);
+        report(status, GBG_DEV_NONFINITE);
       } else if (e) {
         // most points find their brick's exponent at least as large already
         uint32_t *at = ebrick + (size_t)eb * ncomp + c;

@@ -595,3 +595,17 @@ def test_status_by_thread(gbg, dev):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("bad", ["positions", "quantities"])
+def test_deposit_of_bad_points_only(gbg, dev, bad):
+    # every lane of every warp reports
+    m = 200_000
+    rng = np.random.default_rng(3)
+    grid = gbg.Grid3D((32, 32, 32), (TWO_PI,) * 3)
+    pos, q = TWO_PI * rng.random((m, 3)), rng.standard_normal((m, 3))
+    (pos if bad == "positions" else q)[:] = np.nan
+    points, values = gbg.PointSet(to_dev(pos, dev)), gbg.VectorPointValues(to_dev(q, dev))
+    for _ in range(2):
+        with pytest.raises(gbg.InexactError):
+            gbg.anterpolate(grid, points, values, gbg.CatmullRom)
