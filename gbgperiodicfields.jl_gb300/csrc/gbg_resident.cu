@@ -1458,28 +1458,33 @@ void scatter_nodes_chunk(FixGeo &g, int cp, int n2, size_t budget) {
   g.chunk1 = g.chunk + (int32_t)(((size_t)g.bvol * cp * sizeof(float) / per) & ~size_t(3));
 }
 
+// Shared memory per scatter CTA: its share of an SM's, with `ctas` on it, less the block's reserved
+// and static share, or more when a region of 512 points would not fit one chunk (a brick's
+// region holds a few hundred at the usual densities, and each extra chunk re-stages and
+// re-walks the rows; a single chunk may also use the running sums' space).
+size_t scatter_nodes_share(int ctas) { return 228 * 1024 / ctas - 4096; }
+size_t scatter_nodes_want(const FixGeo &g, int cp, int n2) {
+  const size_t per = sizeof(float) * (cp + scatter_wstride(n2));
+  const size_t sums = sizeof(float) * (size_t)g.bvol * cp;
+  return scatter_nodes_fixed(g, cp) + (512 * per > sums ? 512 * per - sums : 0) + 4 * per;
+}
+size_t scatter_nodes_budget(const FixGeo &g, int cp, int n2, int ctas) {
+  const size_t share = scatter_nodes_share(ctas);
+  return scatter_nodes_want(g, cp, n2) <= share ? share : std::min<size_t>(200 * 1024, 228 * 1024 - 4096);
+}
+
 // Scatter CTAs per SM that registers and shared memory are shared out for.  The setup of a brick is a
 // chain of short phases with barriers between them, so a third CTA pays where a region still fits
 // one staging: width 4 or less and four components (256^3 x 3, 6e6 points: 1.80 ms with two, 1.53 with
 // three, 1.99 with four; at width 6 a region of 644 points takes two stagings and 128^3 x 3 goes from
-// 388 to 648 us).
-constexpr int scatter_ctas(int n2, int cp) { return cp == 4 && n2 <= 4 ? 3 : 2; }
-template <int N2, int CP>
-constexpr int kScatterCtas = scatter_ctas(N2, CP);
-
-// Shared memory per scatter CTA: its share of an SM's less the block's reserved
-// and static share, or more when a region of 512 points would not fit one chunk (a brick's
-// region holds a few hundred at the usual densities, and each extra chunk re-stages and
-// re-walks the rows; a single chunk may also use the running sums' space).  It depends on
-// the brick's geometry alone, never on the launch shape: the chunks are where the
+// 388 to 648 us), with the brick's tables within a third of the memory (of 16x8x8, 20x10x10 and 32x8x8
+// cells they are not: 128^3 x 3, width 4, a point a cell, with two CTAs an SM 504, 610 and 577 us, with the one
+// that would fit 555, 932 and 850).
+// It depends on the brick's geometry alone, never on the launch shape: the chunks are where the
 // compensated summation folds its partial sums, so the same chunks for every launch keep
 // the results bitwise independent of the threads per CTA and of batching.
-size_t scatter_nodes_budget(const FixGeo &g, int cp, int n2) {
-  const size_t per = sizeof(float) * (cp + scatter_wstride(n2));
-  const size_t sums = sizeof(float) * (size_t)g.bvol * cp;
-  const size_t want = scatter_nodes_fixed(g, cp) + (512 * per > sums ? 512 * per - sums : 0) + 4 * per;
-  const size_t half = 228 * 1024 / scatter_ctas(n2, cp) - 4096;
-  return want <= half ? half : std::min<size_t>(200 * 1024, 228 * 1024 - 4096);
+int scatter_ctas(const FixGeo &g, int cp, int n2) {
+  return cp == 4 && n2 <= 4 && scatter_nodes_want(g, cp, n2) <= scatter_nodes_share(3) ? 3 : 2;
 }
 
 // Few points a brick (as for the direct gather), and a region no wider than the grid on any
@@ -2124,8 +2129,8 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
   return issued;
 }
 
-template <int N2, bool FIXED, int CP>
-__global__ void __launch_bounds__(kThreads, kScatterCtas<N2, CP>)
+template <int N2, bool FIXED, int CP, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS)
     k_scatter_nodes(FixGeo g, SchemeT<float, N2> s, const uint32_t *__restrict__ cell_start,
                     const float4 *__restrict__ rec, const float *__restrict__ qs,
                     const unsigned *__restrict__ qmax_bits, float *__restrict__ field, float beta,
@@ -2535,8 +2540,15 @@ gbg_status launch_staged_scatter(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int threads = b->scatter_threads ? b->scatter_threads : kThreads;
   const bool reach = beta == 1.0 && b->reach_ok;
+  const int ctas = scatter_ctas(g, f->cp, N2);
+  scatter_nodes_chunk(g, f->cp, N2, scatter_nodes_budget(g, f->cp, N2, ctas));
+  auto nodes_kernel = [&]() -> decltype(&k_scatter_nodes<N2, FIXED, 12, 2>) {
+    if constexpr (N2 <= 4)
+      if (ctas == 3) return &k_scatter_nodes<N2, FIXED, 4, 3>;
+    if (f->cp == 4) return &k_scatter_nodes<N2, FIXED, 4, 2>;
+    return &k_scatter_nodes<N2, FIXED, 12, 2>;
+  };
   auto go = [&](auto kernel) -> gbg_status {
-    scatter_nodes_chunk(g, f->cp, N2, scatter_nodes_budget(g, f->cp, N2));
     const size_t smem = scatter_nodes_smem(g, f->cp, N2);
     if (smem > 227 * 1024) return set_error(GBG_EUNSUPPORTED, "brick too large for the scatter's shared memory");
     GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2573,7 +2585,6 @@ gbg_status launch_staged_scatter(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme
     if (f->cp == 4) GBG_TRY(sp(k_scatter_sparse<N2, FIXED, 4>, sparse_warp_smem<N2, 4>(kThreads / 32)));
     else GBG_TRY(sp(k_scatter_sparse<N2, FIXED, 12>, sparse_warp_smem<N2, 12>(kThreads / 32)));
     auto over = [&](auto kernel) -> gbg_status {
-      scatter_nodes_chunk(g, f->cp, N2, scatter_nodes_budget(g, f->cp, N2));
       const size_t smem = scatter_nodes_smem(g, f->cp, N2);
       if (smem > 227 * 1024) return set_error(GBG_EUNSUPPORTED, "brick too large for the scatter's shared memory");
       GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2587,13 +2598,11 @@ gbg_status launch_staged_scatter(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme
       GBG_CUDA_TRY(cudaGetLastError());
       return GBG_OK;
     };
-    if (f->cp == 4) GBG_TRY(over(k_scatter_nodes<N2, FIXED, 4>));
-    else GBG_TRY(over(k_scatter_nodes<N2, FIXED, 12>));
+    GBG_TRY(over(nodes_kernel()));
     mark_main_stop(st);
     return GBG_OK;
   }
-  if (f->cp == 4) return go(k_scatter_nodes<N2, FIXED, 4>);
-  return go(k_scatter_nodes<N2, FIXED, 12>);
+  return go(nodes_kernel());
 }
 
 // ------------------------------------------------------------ batched form
@@ -3622,7 +3631,7 @@ gbg_status batch_plan(const gbg_batch_item *items, int32_t count, gbg_batch_s *b
       d.fg.halo = ds->halo;
       d.fg.cp = ds->cp;
       d.fg.ncomp = ds->ncomp;
-      scatter_nodes_chunk(d.fg, ds->cp, w, scatter_nodes_budget(d.fg, ds->cp, w));
+      scatter_nodes_chunk(d.fg, ds->cp, w, scatter_nodes_budget(d.fg, ds->cp, w, scatter_ctas(d.fg, ds->cp, w)));
       scat_max = std::max(scat_max, scatter_nodes_smem(d.fg, ds->cp, w));
       bt->cstride = std::max<int64_t>(bt->cstride, b->bvol * 12);
       if (d.fg.e[0] > 255) return set_error(GBG_EUNSUPPORTED, "batch: brick too large for the scatter");

@@ -609,3 +609,33 @@ def test_deposit_of_bad_points_only(gbg, dev, bad):
     for _ in range(2):
         with pytest.raises(gbg.InexactError):
             gbg.anterpolate(grid, points, values, gbg.CatmullRom)
+
+
+# bricks whose tables take a third, half and all of an SM's memory
+@pytest.mark.parametrize("brick", [(11, 8, 8), (16, 8, 8), (20, 10, 10), (32, 8, 8), (16, 16, 8)])
+@pytest.mark.parametrize("width,ncomp", [(2, 3), (4, 4), (4, 1)])
+@pytest.mark.parametrize("density", [0.05, 1.3])
+def test_scatter_of_every_brick_share(gbg, oracle, dev, brick, width, ncomp, density):
+    _resident_scatter(gbg, oracle, dev, (40, 33, 24), brick, width, ncomp, density)
+
+
+def _resident_scatter(gbg, oracle, dev, n, brick, width, ncomp, density):
+    """A resident scatter against the oracle, and the batched form's against it bit by bit."""
+    from gbgperiodicfields_gb300 import resident
+    m = int(density * np.prod(n))
+    rng = np.random.default_rng(m + 100 * ncomp + width)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    scheme = gbg.LalescuSpline(width) if width > 2 else gbg.LagrangeSpline(2)
+    pos = np.asfortranarray(TWO_PI * rng.random((m, 3)))
+    q = np.asfortranarray(rng.standard_normal((m, ncomp)).astype(np.float32))
+    want = oracle.scatter(g, np.zeros(n + (ncomp,), order="F"), pos, q.astype(np.float64), scheme.coefficients)
+    bins = resident.PointBins(grid, m, brick=brick).build(to_dev(pos, dev))
+    dest = resident.ResidentField(grid, ncomp, max_stencil_width=width)
+    qd = to_dev(q, dev)
+    resident.anterpolate_binned(dest, bins, scheme, qd)
+    got = dest.read(torch.float32).cpu().numpy()
+    assert relerr(got, want) <= 1e-5
+    again = resident.ResidentField(grid, ncomp, max_stencil_width=width)
+    resident.Batch([dict(field=dest, bins=bins, scheme=scheme, dest=again, q=qd)]).run()
+    assert np.array_equal(again.read(torch.float32).cpu().numpy(), got)
