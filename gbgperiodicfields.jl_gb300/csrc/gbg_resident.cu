@@ -1473,18 +1473,26 @@ size_t scatter_nodes_budget(const FixGeo &g, int cp, int n2, int ctas) {
   return scatter_nodes_want(g, cp, n2) <= share ? share : std::min<size_t>(200 * 1024, 228 * 1024 - 4096);
 }
 
+// Points of a brick's region, on average.
+double scatter_region_points(const FixGeo &g, int64_t npoints) {
+  return (double)npoints * g.e[0] * g.e[1] * g.e[2] / ((double)g.n[0] * g.n[1] * g.n[2]);
+}
+
 // Scatter CTAs per SM that registers and shared memory are shared out for.  The setup of a brick is a
-// chain of short phases with barriers between them, so a third CTA pays where a region still fits
-// one staging: width 4 or less and four components (256^3 x 3, 6e6 points: 1.80 ms with two, 1.53 with
-// three, 1.99 with four; at width 6 a region of 644 points takes two stagings and 128^3 x 3 goes from
-// 388 to 648 us), with the brick's tables within a third of the memory (of 16x8x8, 20x10x10 and 32x8x8
-// cells they are not: 128^3 x 3, width 4, a point a cell, with two CTAs an SM 504, 610 and 577 us, with the one
-// that would fit 555, 932 and 850).
-// It depends on the brick's geometry alone, never on the launch shape: the chunks are where the
-// compensated summation folds its partial sums, so the same chunks for every launch keep
+// chain of short phases with barriers between them, so a third CTA pays (256^3 x 3, 6e6 points, width 4: 1.80
+// ms with two, 1.53 with three, 1.99 with four) where most regions still fit its smaller staging at once:
+// width 4 or less and four components, the brick's tables within a third of the memory, and the
+// mean region within 7/8 of the staging.  128^3 x 3 at width 4, points a cell and us with two and three: 0.36,
+// 243 and 224; 0.5 (853 points a region, a staging of 710), 298 and 344; 0.7, 429 and 475.  A third CTA at
+// width 6, whose regions of 644 points take two stagings: 128^3 x 3 goes from 388 to 648 us.
+// It depends on the bins alone (their geometry and number of points), never on the launch shape: the chunks
+// are where the compensated summation folds its partial sums, so the same chunks for every launch keep
 // the results bitwise independent of the threads per CTA and of batching.
-int scatter_ctas(const FixGeo &g, int cp, int n2) {
-  return cp == 4 && n2 <= 4 && scatter_nodes_want(g, cp, n2) <= scatter_nodes_share(3) ? 3 : 2;
+int scatter_ctas(const FixGeo &g, int cp, int n2, int64_t npoints) {
+  if (cp != 4 || n2 > 4 || scatter_nodes_want(g, cp, n2) > scatter_nodes_share(3)) return 2;
+  FixGeo third = g;
+  scatter_nodes_chunk(third, cp, n2, scatter_nodes_share(3));
+  return scatter_region_points(g, npoints) <= 0.875 * third.chunk1 ? 3 : 2;
 }
 
 // Few points a brick (as for the direct gather), and a region no wider than the grid on any
@@ -2540,7 +2548,7 @@ gbg_status launch_staged_scatter(gbg_field_s *f, gbg_bins_s *b, const gbg_scheme
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int threads = b->scatter_threads ? b->scatter_threads : kThreads;
   const bool reach = beta == 1.0 && b->reach_ok;
-  const int ctas = scatter_ctas(g, f->cp, N2);
+  const int ctas = scatter_ctas(g, f->cp, N2, b->npoints);
   scatter_nodes_chunk(g, f->cp, N2, scatter_nodes_budget(g, f->cp, N2, ctas));
   auto nodes_kernel = [&]() -> decltype(&k_scatter_nodes<N2, FIXED, 12, 2>) {
     if constexpr (N2 <= 4)
@@ -3631,7 +3639,7 @@ gbg_status batch_plan(const gbg_batch_item *items, int32_t count, gbg_batch_s *b
       d.fg.halo = ds->halo;
       d.fg.cp = ds->cp;
       d.fg.ncomp = ds->ncomp;
-      scatter_nodes_chunk(d.fg, ds->cp, w, scatter_nodes_budget(d.fg, ds->cp, w, scatter_ctas(d.fg, ds->cp, w)));
+      scatter_nodes_chunk(d.fg, ds->cp, w, scatter_nodes_budget(d.fg, ds->cp, w, scatter_ctas(d.fg, ds->cp, w, b->npoints)));
       scat_max = std::max(scat_max, scatter_nodes_smem(d.fg, ds->cp, w));
       bt->cstride = std::max<int64_t>(bt->cstride, b->bvol * 12);
       if (d.fg.e[0] > 255) return set_error(GBG_EUNSUPPORTED, "batch: brick too large for the scatter");

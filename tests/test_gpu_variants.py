@@ -639,3 +639,9 @@ def _resident_scatter(gbg, oracle, dev, n, brick, width, ncomp, density):
     again = resident.ResidentField(grid, ncomp, max_stencil_width=width)
     resident.Batch([dict(field=dest, bins=bins, scheme=scheme, dest=again, q=qd)]).run()
     assert np.array_equal(again.read(torch.float32).cpu().numpy(), got)
+
+
+# mean regions below, at and above 7/8 of the smaller staging (710 points at width 4, 1088 at width 2)
+@pytest.mark.parametrize("width,density", [(4, 0.30), (4, 0.36), (4, 0.37), (4, 0.5), (4, 0.9), (2, 0.9), (2, 0.97), (2, 0.98), (2, 1.2)])
+def test_scatter_either_side_of_the_third_share(gbg, oracle, dev, width, density):
+    _resident_scatter(gbg, oracle, dev, (44, 32, 24), (11, 8, 8), width, 3, density)
