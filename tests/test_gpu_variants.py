@@ -645,3 +645,11 @@ def _resident_scatter(gbg, oracle, dev, n, brick, width, ncomp, density):
 @pytest.mark.parametrize("width,density", [(4, 0.30), (4, 0.36), (4, 0.37), (4, 0.5), (4, 0.9), (2, 0.9), (2, 0.97), (2, 0.98), (2, 1.2)])
 def test_scatter_either_side_of_the_third_share(gbg, oracle, dev, width, density):
     _resident_scatter(gbg, oracle, dev, (44, 32, 24), (11, 8, 8), width, 3, density)
+
+
+# regions of few and of many points at the widths whose trips are never voted, and mean regions either side of
+# 1024 points at those where they are
+@pytest.mark.parametrize("width,density", [(2, 0.1), (2, 1.5), (8, 0.1), (8, 0.4), (4, 0.5), (4, 0.7), (6, 0.3), (6, 0.45)])
+@pytest.mark.parametrize("ncomp", [5, 12])
+def test_scatter_trips_at_every_width(gbg, oracle, dev, width, density, ncomp):
+    _resident_scatter(gbg, oracle, dev, (33, 24, 20), (11, 8, 8), width, ncomp, density)
