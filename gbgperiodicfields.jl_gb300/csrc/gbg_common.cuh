@@ -267,8 +267,8 @@ gbg_status radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, ui
 // Stable sort of point indices by key from a counting pass: rank[p] is what an atomic count
 // of keys[p] returned (the array is overwritten) and starts[] the exclusive scan of those counts
 // (starts[k+1] - starts[k] points per key).  perm[s] = the point in slot s, points of one key in
-// index order -- the order the stable radix sort gives.  *big must be zero on entry (keys with more
-// than 1024 points are counted there and sorted apart).  temp holds n words.  With rec_user and rec
+// index order -- the order the stable radix sort gives.  big[0] and big[4] must be zero on entry (keys with
+// more than 1024 points are counted there and sorted apart).  temp holds n words.  With rec_user and rec
 // given, rec[s] = rec_user[perm[s]] is written too.
 gbg_status stable_counting_sort(const uint32_t *keys, uint32_t *rank, const uint32_t *starts, int64_t n, uint32_t *perm,
                                 uint32_t *big, uint32_t *temp, cudaStream_t stream, const float4 *rec_user = nullptr,

@@ -1593,7 +1593,7 @@ ScatterLayout scatter_layout(Arena &a, int64_t m, const ScatterPlan &P, int ncom
   ScatterLayout L;
   // the words that start at zero stand together (scatter_clear)
   const size_t nexp = P.bricked ? (size_t)(P.bg.enb[0] * P.bg.enb[1] * P.bg.enb[2]) : 0;
-  L.flag = a.take<uint32_t>(4);
+  L.flag = a.take<uint32_t>(8);
   L.ebrick = P.bricked ? a.take<uint32_t>(nexp * ncomp) : nullptr;
   L.counts = a.take<uint32_t>((size_t)P.nkeys + 1);
   L.keys = a.take<uint32_t>((size_t)m);

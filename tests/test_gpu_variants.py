@@ -653,3 +653,35 @@ def test_scatter_either_side_of_the_third_share(gbg, oracle, dev, width, density
 @pytest.mark.parametrize("ncomp", [5, 12])
 def test_scatter_trips_at_every_width(gbg, oracle, dev, width, density, ncomp):
     _resident_scatter(gbg, oracle, dev, (33, 24, 20), (11, 8, 8), width, ncomp, density)
+
+
+# runs at and above the longest that one CTA sorts (16384, or a 255th of the points), alone, beside shorter
+# ones and nearly as many as there can be, shares of the points that end within a tile
+@pytest.mark.parametrize("runs,spread", [((16384,), 0), ((16385,), 0), ((16384, 16385, 1025, 40_000, 1024, 2500), 30_001),
+                                         ((200_000,), 1), ((20_000,) * 200, 77), ((16_500,) * 240, 300_000)])
+def test_bins_order_with_huge_runs(gbg, dev, runs, spread):
+    from gbgperiodicfields_gb300 import resident
+    n = np.array((24, 24, 24))
+    rng = np.random.default_rng(len(runs) + spread)
+    grid = gbg.Grid3D(tuple(n), tuple(float(v) for v in n))  # cells of edge 1
+    cells = rng.choice(24 ** 3, len(runs), replace=False)
+    pos = [24 * rng.random((spread, 3))]
+    for k, c in zip(cells, runs):
+        pos.append(np.array([k % 24, (k // 24) % 24, k // 576]) + rng.random((c, 3)))
+    pos = np.concatenate(pos)
+    pos = np.asfortranarray(pos[rng.permutation(len(pos))])
+    bins = resident.PointBins(grid, len(pos), brick=(8, 8, 8))
+    c = np.floor(pos).astype(np.int64) % n
+    br = c // 8
+    loc = c - 8 * br
+    key = ((br[:, 2] * 3 + br[:, 1]) * 3 + br[:, 0]) * 512 + (loc[:, 2] * 8 + loc[:, 1]) * 8 + loc[:, 0]
+    want = np.argsort(key, kind="stable") + 1
+    for _ in range(2):
+        bins.build(to_dev(pos, dev))
+        assert np.array_equal(bins.order().cpu().numpy(), want)
+    # the records follow: a linear field is reproduced by the cubic spline inside the box
+    x = torch.arange(24, dtype=torch.float64, device=dev)[:, None, None].expand(24, 24, 24)
+    field = resident.ResidentField(grid, 1, 4).load(gbg.colmajor(x.contiguous()[..., None]))
+    got = resident.interpolate_binned(field, bins, gbg.CatmullRom).cpu().numpy()[:, 0]
+    inner = (pos[:, 0] >= 2) & (pos[:, 0] < 21)
+    assert np.abs(got - pos[:, 0])[inner].max(initial=0.0) <= 24e-5
