@@ -914,9 +914,9 @@ int owner_points(double L, int wexp) {
 }
 
 // Shared words of a staged point: the digits of CC components and the meta word, in 16-byte units of
-// an odd count (or one), so that lanes reading neighbouring points meet different banks.
+// an odd count, so that lanes reading neighbouring points meet different banks.
 template <int CC, int ND>
-constexpr int kDigitWords = CC * ND + 1 <= 4 ? 4 : 12;
+constexpr int kDigitWords = 4 * (((CC * ND + 4) / 4) | 1);
 template <int N2>
 constexpr int kWeightWords = 3 * N2 + 1;  // 64-bit words, odd
 
@@ -952,7 +952,7 @@ __device__ __forceinline__ uint32_t owner_walk(unsigned long long rows, const ui
     for (int j = 0; j < 2 * ND; ++j) A[c][j] = 0ll;
   while (__any_sync(0xffffffffu, todo > 0)) {
     if (todo > 0) {
-      uint32_t d[12];
+      uint32_t d[(CC * ND + 4) / 4 * 4];
 #pragma unroll
       for (int j = 0; j < (CC * ND + 4) / 4; ++j) {
         const uint4 v = lds128(dp + 16 * j);
@@ -1063,22 +1063,22 @@ __device__ __forceinline__ Int192 leading_bits(const unsigned long long *at, int
   return s;
 }
 
-template <typename T, int N2, int CC>
+// The components from cfrom up to cto, CMAX at a time and the last REST of them by themselves.
+template <typename T, int N2, int CMAX, int REST>
 __global__ void __launch_bounds__(kThreads, 2)
-    k_scatter_owner(GridT<T> g, BrickGeo bg, int ncomp, int chunk, int chunk1, int sums_bytes,
+    k_scatter_owner(GridT<T> g, BrickGeo bg, int ncomp, int cfrom, int cto, int chunk, int chunk1, int sums_bytes,
                     const uint32_t *__restrict__ cell_start, const long long *__restrict__ wts,
                     const long long *__restrict__ qi, const int16_t *__restrict__ qe,
                     const uint32_t *__restrict__ ebrick, int wexp, T *__restrict__ field, T beta, int beta_zero,
                     uint32_t *__restrict__ ticket) {
-  constexpr int ND = kDigits<T>, DW = kDigitWords<CC, ND>, WW = kWeightWords<N2>, half = N2 / 2;
-  static_assert(CC * ND + 1 <= DW, "");
+  constexpr int ND = kDigits<T>, WW = kWeightWords<N2>, half = N2 / 2;
   extern __shared__ __align__(16) unsigned char smem_owner[];
   __shared__ uint32_t warp_tot[32];
   __shared__ uint32_t s_brick[2], s_unit;
   const int B0 = bg.b[0], B1 = bg.b[1], B2 = bg.b[2];
   const int E0 = B0 + N2 - 1, E1 = B1 + N2 - 1, E2 = B2 + N2 - 1, ecount = E0 * E1 * E2;
   const int bvol = (int)bg.bvol;
-  const size_t per = DW * 4 + WW * 8 + 4;
+  const size_t per = kDigitWords<(REST > CMAX ? REST : CMAX), ND> * 4 + WW * 8 + 4;
   const size_t staging = max((size_t)sums_bytes + (size_t)chunk * per, (size_t)chunk1 * per);
   uint32_t *off = reinterpret_cast<uint32_t *>(smem_owner + staging);  // ecount + 1 offsets
   uint32_t *r0s = off + ecount + 1;                                    // the cells' first slots
@@ -1089,9 +1089,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint32_t *xe = vz + E2, *ye = xe + E0, *ze = ye + E1;                // per-axis exponent brick tables
   uint32_t *marked = ze + E2;                                          // bvol nodes' non-finite marks
   uint32_t *ereg = marked + bvol;                                      // ncomp region scales
-  // bvol * CC sums of 224 bits: three planes of 64 a component, then the signed tops
+  // the nodes' sums of 224 bits: three planes of 64 a component, then the signed tops
   unsigned long long *sums = reinterpret_cast<unsigned long long *>(smem_owner);
-  uint32_t *tops = reinterpret_cast<uint32_t *>(sums + (size_t)3 * CC * bvol);
   const uint32_t nbricks = (uint32_t)(bg.nb[0] * bg.nb[1] * bg.nb[2]);
   const int n[3] = {(int)g.nx, (int)g.ny, (int)g.nz};
   const uint32_t n0 = (uint32_t)n[0], n01 = n0 * (uint32_t)n[1];
@@ -1157,7 +1156,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint32_t count = block_scan_counts(off, ecount, warp_tot);
     if (tid == 0) off[ecount] = count;
     const int depth = sum_depth(count);
-    for (int cc0 = 0; cc0 < ncomp; cc0 += CC) {
+    auto components = [&](auto some, int cc0) {  // `some` components from cc0 on
+      constexpr int CC = decltype(some)::value, DW = kDigitWords<CC, ND>;
+      uint32_t *tops = reinterpret_cast<uint32_t *>(sums + (size_t)3 * CC * bvol);
       long long A[CC][2 * ND] = {};  // the products' accumulators, [weight digit * ND + quantity digit]
       auto inside = [&](int lx, int ly, int lz) -> bool {
         return bc[0] * B0 + lx < n[0] && bc[1] * B1 + ly < n[1] && bc[2] * B2 + lz < n[2];
@@ -1383,7 +1384,10 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
       }
       __syncthreads();  // the sums and the staging are free for the next components
-    }
+    };
+    int cc0 = cfrom;
+    for (; cc0 + CMAX + REST <= cto; cc0 += CMAX) components(std::integral_constant<int, CMAX>{}, cc0);
+    if constexpr (REST > 0) components(std::integral_constant<int, REST>{}, cc0);
   }
 }
 
@@ -1656,10 +1660,10 @@ int bits_for(uint64_t max_value) {
   return b;
 }
 
-// The owner kernel for CC components at a time.
-template <typename T, int N2, int CC>
-gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int wexp, int points,
+template <typename T, int N2, int CMAX, int REST = 0>
+gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int cfrom, int cto, int wexp, int points,
                         const ScatterLayout &L, T *field, double beta, cudaStream_t st) {
+  constexpr int CC = REST > CMAX ? REST : CMAX;
   constexpr size_t per = kDigitWords<CC, kDigits<T>> * 4 + kWeightWords<N2> * 8 + 4;
   const BrickGeo &bg = P.bg;
   const size_t e[3] = {(size_t)bg.b[0] + N2 - 1, (size_t)bg.b[1] + N2 - 1, (size_t)bg.b[2] + N2 - 1};
@@ -1670,20 +1674,45 @@ gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int 
   const int chunk = (int)(std::min<size_t>(points, (budget - tables - sums) / per) & ~size_t(3));
   const int chunk1 = (int)(std::min<size_t>(points, (budget - tables) / per) & ~size_t(3));
   const size_t smem = std::max(sums + chunk * per, chunk1 * per) + tables;
-  auto kernel = k_scatter_owner<T, N2, CC>;
+  auto kernel = k_scatter_owner<T, N2, CMAX, REST>;
   GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GBG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   // two CTAs per SM, by the launch bounds and the shared memory's share (more would find no ticket left)
   const int64_t nbricks = bg.nb[0] * bg.nb[1] * bg.nb[2];
   const int blocks = launch_blocks(nbricks, 1, 2);
-  mark_main_start(st);
-  kernel<<<blocks, kThreads, smem, st>>>(g, bg, ncomp, chunk, chunk1, (int)sums, L.counts,
+  kernel<<<blocks, kThreads, smem, st>>>(g, bg, ncomp, cfrom, cto, chunk, chunk1, (int)sums, L.counts,
                                          static_cast<const long long *>(L.rec), L.qi, L.qe, L.ebrick, wexp, field,
-                                         T(beta), beta == 0.0, L.flag);
-  mark_main_stop(st);
+                                         T(beta), beta == 0.0, L.flag + (cfrom > 0));
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
   return GBG_OK;
+}
+
+// The owner kernel over all components, three to a trip and the last one, two or four by themselves: in the
+// same launch up to width 4, whose bricks' listing costs more than the registers that a kernel of two
+// sizes spills, in a second one from width 6.  96^3, 885k points, FP64, for 3, 4 and 5 components: width
+// 4, 1.21, 1.64 and 2.18 ms (one at a time 2.82 and 3.47 for the last two), width 8, 8.4, 10.7 and 14.7 (18.7 and
+// 23.1).
+template <typename T, int N2>
+gbg_status launch_owners(const GridT<T> &g, const ScatterPlan &P, int ncomp, int wexp, int points, const ScatterLayout &L,
+                         T *field, double beta, cudaStream_t st) {
+  auto go = [&](auto cmax, auto rest, int cfrom, int cto) {
+    return launch_owner<T, N2, decltype(cmax)::value, decltype(rest)::value>(g, P, ncomp, cfrom, cto, wexp, points, L,
+                                                                             field, beta, st);
+  };
+  constexpr std::integral_constant<int, 0> none{};
+  constexpr std::integral_constant<int, 1> one{};
+  constexpr std::integral_constant<int, 2> two{};
+  constexpr std::integral_constant<int, 3> three{};
+  constexpr std::integral_constant<int, 4> four{};
+  if (ncomp == 1) return go(one, none, 0, 1);
+  if (ncomp == 2) return go(two, none, 0, 2);
+  if (ncomp == 4) return go(four, none, 0, 4);
+  if (ncomp % 3 == 0) return go(three, none, 0, ncomp);
+  if constexpr (N2 <= 4) return ncomp % 3 == 1 ? go(three, four, 0, ncomp) : go(three, two, 0, ncomp);
+  const int main = ncomp % 3 == 1 ? ncomp - 4 : ncomp - 2;
+  GBG_TRY(go(three, none, 0, main));
+  return ncomp % 3 == 1 ? go(four, none, main, ncomp) : go(two, none, main, ncomp);
 }
 
 template <typename T, int N2, bool FIXED>
@@ -1705,9 +1734,10 @@ gbg_status launch_bricked(const GridT<T> &g, const ScatterPlan &P, const gbg_sch
       g, s, x, L.perm, m, wexp, static_cast<long long *>(L.rec), q, ncomp, T(alpha), L.qi, L.qe);
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
-  // three components share a point's weights and its trip; other counts go one at a time
-  return ncomp % 3 == 0 ? launch_owner<T, N2, 3>(g, P, ncomp, wexp, points, L, field, beta, st)
-                        : launch_owner<T, N2, 1>(g, P, ncomp, wexp, points, L, field, beta, st);
+  mark_main_start(st);
+  GBG_TRY((launch_owners<T, N2>(g, P, ncomp, wexp, points, L, field, beta, st)));
+  mark_main_stop(st);
+  return GBG_OK;
 }
 
 // The deterministic scatter.  The brick scatter (integer sums, FP64-grade per node)

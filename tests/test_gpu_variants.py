@@ -685,3 +685,26 @@ def test_bins_order_with_huge_runs(gbg, dev, runs, spread):
     got = resident.interpolate_binned(field, bins, gbg.CatmullRom).cpu().numpy()[:, 0]
     inner = (pos[:, 0] >= 2) & (pos[:, 0] < 21)
     assert np.abs(got - pos[:, 0])[inner].max(initial=0.0) <= 24e-5
+
+
+# every remainder of three: a component's sums do not depend on the others beside it, sparse and crowded, with
+# quantities of one window and of several
+@pytest.mark.parametrize("comps", [1, 2, 3, 4, 5, 7, 8, 10])
+@pytest.mark.parametrize("width", [2, 4, 6, 8])
+@pytest.mark.parametrize("m,spread", [(2000, 0), (2000, 60), (60_000, 0), (60_000, 30)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_scatter_of_every_component_count(gbg, dev, comps, width, m, spread, dtype):
+    T = np.float64 if dtype == torch.float64 else np.float32
+    n = (17, 16, 13)
+    rng = np.random.default_rng(comps + m)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3, dtype=dtype)
+    scheme = gbg.LalescuSpline(width) if width > 2 else gbg.LagrangeSpline(2)
+    pos = np.asfortranarray((TWO_PI * rng.random((m, 3))).astype(T))
+    q = (rng.standard_normal((m, comps)) * 2.0 ** (-spread * rng.random((m, 1)))).astype(T)
+    q[rng.integers(m), rng.integers(comps)] = np.nan
+    q = np.asfortranarray(q)
+    old = np.asfortranarray(rng.standard_normal(n + (comps,)).astype(T))
+    got = _scatter_abi(gbg, grid, dev, old, pos, q, scheme, 1.0, 0.5)
+    for c in range(comps):
+        alone = _scatter_abi(gbg, grid, dev, old[..., c:c + 1], pos, q[:, c:c + 1], scheme, 1.0, 0.5)
+        assert np.array_equal(got[..., c:c + 1], alone, equal_nan=True)
