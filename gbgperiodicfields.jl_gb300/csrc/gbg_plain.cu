@@ -920,14 +920,15 @@ constexpr int kDigitWords = 4 * (((CC * ND + 4) / 4) | 1);
 template <int N2>
 constexpr int kWeightWords = 3 * N2 + 1;  // 64-bit words, odd
 
-// The trips of one lane's node over the staged points: `rows` marks (bit kk * 8 + jj) the rows of cells
+// The trips of one lane's node over the points [lo, hi) of the region, staged where point p's digits and weights
+// are at digits and weights plus p of their strides: `rows` marks (bit kk * 8 + jj) the rows of cells
 // (lx..lx+N2-1, ly+jj, lz+kk) to take.  The loop is the warp's, held together by its vote: a trip takes
 // one point of every lane that has one left, and a lane whose row is done moves to its next row within
 // the trip.  (Left to itself the compiler makes this a loop over rows around a loop over their points,
 // where the lanes wait for the fullest of 32 rows at every row.)  Returns the points' meta words, or-ed.
 template <int N2, int CC, int ND>
 __device__ __forceinline__ uint32_t owner_walk(unsigned long long rows, const uint32_t *po, int ebase, int E0, int E1,
-                                               int xk, uint32_t c0, uint32_t c1, uint32_t digits, uint32_t weights,
+                                               int xk, uint32_t lo, uint32_t hi, uint32_t digits, uint32_t weights,
                                                long long (&A)[CC][2 * ND]) {
   constexpr int DW = kDigitWords<CC, ND>, WW = kWeightWords<N2>;
   int todo = 0;
@@ -937,10 +938,10 @@ __device__ __forceinline__ uint32_t owner_walk(unsigned long long rows, const ui
     rows &= rows - 1ull;
     const int kk = s >> 3, jj = s & 7;
     const int e0 = ebase + (kk * E1 + jj) * E0;
-    const uint32_t p0 = max(po[e0], c0);
-    todo = (int)(min(po[e0 + N2], c1) - p0);
-    dp = digits + (p0 - c0) * (DW * 4);
-    wp = weights + (p0 - c0) * (WW * 8);
+    const uint32_t p0 = max(po[e0], lo);
+    todo = (int)(min(po[e0 + N2], hi) - p0);
+    dp = digits + p0 * (DW * 4);
+    wp = weights + p0 * (WW * 8);
     wy = wp + 8 * (2 * N2 - 1 - jj);
     wz = wp + 8 * (3 * N2 - 1 - kk);
     wp += 8 * xk;
@@ -1074,7 +1075,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   constexpr int ND = kDigits<T>, WW = kWeightWords<N2>, half = N2 / 2;
   extern __shared__ __align__(16) unsigned char smem_owner[];
   __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t s_brick[2], s_unit;
+  __shared__ uint32_t s_brick[2], s_unit, s_lump;
   const int B0 = bg.b[0], B1 = bg.b[1], B2 = bg.b[2];
   const int E0 = B0 + N2 - 1, E1 = B1 + N2 - 1, E2 = B2 + N2 - 1, ecount = E0 * E1 * E2;
   const int bvol = (int)bg.bvol;
@@ -1107,7 +1108,11 @@ __global__ void __launch_bounds__(kThreads, 2)
   // a thread's first region cell and the step to its next, as coordinates
   const int ex0 = tid % E0, ey0 = (tid / E0) % E1, ez0 = tid / (E0 * E1);
   const int esx = (int)blockDim.x % E0, esy = ((int)blockDim.x / E0) % E1, esz = (int)blockDim.x / (E0 * E1);
-  if (tid == 0) s_brick[0] = atomicAdd(ticket, 1u);
+  if (tid == 0) {
+    s_brick[0] = atomicAdd(ticket, 1u);
+    s_lump = 0u;
+  }
+  uint32_t piece = 0u;  // stagings so far; s_lump: the last one that a cell holds a third of
   for (int it = 0;; ++it) {
     __syncthreads();
     const uint32_t brick = s_brick[it & 1];
@@ -1218,8 +1223,10 @@ __global__ void __launch_bounds__(kThreads, 2)
             for (int win = 0; win < kDepth / (kDigit * ND); ++win) {
               __syncthreads();  // the previous points are summed (and the offsets' end is set)
               if (win == 0) {
+                ++piece;
                 for (int e = tid, ex = ex0; e < ecount; e += blockDim.x) {
                   const uint32_t o0 = po[e], lo = max(o0, c0), hi = min(po[e + 1], c1);
+                  if (multi && (int)(hi - lo) > np / 3) s_lump = piece;  // a cell holds a third of the points
                   for (uint32_t t = lo; t < hi; ++t) {
                     pslot[t - c0] = pr[e] + (t - o0);
                     reinterpret_cast<uint32_t *>(dig)[(t - c0) * DW + CC * ND] = (uint32_t)ex;
@@ -1315,7 +1322,8 @@ __global__ void __launch_bounds__(kThreads, 2)
               // A crowded region's nodes differ much in their points (at a blob's edge tenfold within a
               // brick), so a node has four lanes, each with a quarter of its rows, and the warps take the
               // 2x2x2 blocks of nodes as they get free.  (A thread a node there kept a fifth of the lanes
-              // busy.)
+              // busy.)  Where one cell holds a third of the staging, a lane has all rows and a quarter of the
+              // staging instead: 64^3 x 1, 1e6 points in one cell, 83 ms, by rows 184.
               const int nu0 = (B0 + 1) / 2, nu1 = (B1 + 1) / 2, units = nu0 * nu1 * ((B2 + 1) / 2);
               const int lane = tid & 31, part = lane & 3;
               while (true) {
@@ -1327,7 +1335,16 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const bool node = lx < B0 && ly < B1 && lz < B2 && inside(lx, ly, lz);
                 const int ebase = (lz * E1 + ly) * E0 + lx;
                 unsigned long long rows = 0ull;
-                if (node) {
+                uint32_t lo = c0, hi = c1;
+                if (s_lump == piece) {
+                  lo += (uint32_t)(np * part / 4);
+                  hi = c0 + (uint32_t)(np * (part + 1) / 4);
+#pragma unroll 1
+                  for (int r = 0; node && r < N2 * N2; ++r) {
+                    const int kk = r / N2, jj = r % N2, e0 = ebase + (kk * E1 + jj) * E0;
+                    if (max(po[e0], lo) < min(po[e0 + N2], hi)) rows |= 1ull << (kk * 8 + jj);
+                  }
+                } else if (node) {
 #pragma unroll
                   for (int i = 0; i < (N2 * N2 + 3) / 4; ++i) {
                     const int r = 4 * i + part;  // rows r of this lane's quarter, turned so that each has every y
@@ -1338,7 +1355,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                     }
                   }
                 }
-                uint32_t marks = owner_walk<N2, CC, ND>(rows, po, ebase, E0, E1, lx + N2 - 1, c0, c1, digits, weights, A);
+                uint32_t marks = owner_walk<N2, CC, ND>(rows, po, ebase, E0, E1, lx + N2 - 1, lo, hi, digits - c0 * (DW * 4), weights - c0 * (WW * 8), A);
                 // the four lanes' sums, then a component a lane
                 long long mine[2 * ND];
 #pragma unroll

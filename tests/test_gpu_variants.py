@@ -708,3 +708,25 @@ def test_scatter_of_every_component_count(gbg, dev, comps, width, m, spread, dty
     for c in range(comps):
         alone = _scatter_abi(gbg, grid, dev, old[..., c:c + 1], pos, q[:, c:c + 1], scheme, 1.0, 0.5)
         assert np.array_equal(got[..., c:c + 1], alone, equal_nan=True)
+
+
+# crowded regions whose points lie in one cell, in one row of cells and in a few: a node's lanes share a row's
+# points there, with pieces whose ends cut the rows
+@pytest.mark.parametrize("extent", [(1, 1, 1), (6, 1, 1), (2, 2, 1), (5, 5, 4)])
+@pytest.mark.parametrize("m", [505, 509, 1777, 40_003])
+@pytest.mark.parametrize("width", [2, 4, 8])
+def test_scatter_of_crowded_cells(gbg, oracle, dev, extent, m, width):
+    n = (16, 11, 9)
+    rng = np.random.default_rng(m + width)
+    grid = gbg.Grid3D(n, (TWO_PI,) * 3)
+    g = oracle.grid_dict(grid.grid_size, grid.domain_size, grid.origin)
+    scheme = gbg.LalescuSpline(width) if width > 2 else gbg.LagrangeSpline(2)
+    pos = np.asfortranarray((np.array([5.0, 6.0, 3.0]) + rng.random((m, 3)) * extent) * TWO_PI / n)
+    q = np.asfortranarray(rng.standard_normal((m, 3)))
+    zero = np.zeros(n + (3,), order="F")
+    got = _scatter_abi(gbg, grid, dev, zero, pos, q, scheme, 1.0, 0.0)
+    want = oracle.scatter(g, zero.copy(order="F"), pos, q, scheme.coefficients)
+    size, reach = _contribution_sizes(scheme.coefficients, n, pos, q, TWO_PI / np.array(n))
+    assert np.all(np.abs(got - want) <= 1e-12 * size + 4 * 2.0 ** -59 * reach)
+    order = rng.permutation(m)
+    assert np.array_equal(got, _scatter_abi(gbg, grid, dev, zero, pos[order], q[order], scheme, 1.0, 0.0))
