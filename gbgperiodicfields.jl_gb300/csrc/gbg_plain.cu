@@ -78,7 +78,7 @@ template <int N2>
 __device__ __forceinline__ void walk_offsets(int64_t base, int64_t extent, int64_t stride,
                                              int64_t (&off)[N2]) {
   // (the remainder, not wrap_cell's branch around it: the FP32 gather, waiting for its loads either way,
-  // took 1.61 ms with the branch and 1.48 without, 193 x 160 x 127 x 9, 3e6 points; FP64 the same)
+  // takes 1.61 ms with the branch and 1.48 without, 193 x 160 x 127 x 9, 3e6 points; FP64 the same)
   int64_t node = imod(base - (N2 - 2) / 2, extent);
 #pragma unroll
   for (int i = 0; i < N2; ++i) {
@@ -200,8 +200,8 @@ __device__ __forceinline__ void axis_weights_fma(const SchemeT<T, N2> &s, T t, T
 // walk.  In FP64 this kernel is bound by the FP64 pipe (an operation of a warp every 76 clocks of a
 // scheduler), so it counts operations: x is contracted first, then y over the plane, then z -- N2^3 +
 // N2^2 + N2 a component and no weight products, 774 at width 6 and 3 components beside 90 for the
-// weights and 15 for the locate; the product form (w2[j] w3[k] once per plane row) took 792 + 90 + 50.
-// 256^3 x 3, 1e7 points, width 6: 15.75 -> 14.98 ms.
+// weights and 15 for the locate; the product form (w2[j] w3[k] once per plane row) with a division to
+// locate takes 792 + 90 + 50.  256^3 x 3, 1e7 points, width 6: 14.98 ms, 15.75 that way.
 template <typename T, int N2, int M2, int CC>
 __global__ void __launch_bounds__(kThreads)
     k_gather_plain(GridT<T> g, SchemeT<T, N2> s, int ncomp, const T *__restrict__ field,
@@ -277,8 +277,8 @@ __global__ void __launch_bounds__(kThreads)
 // stencil.  A row's nodes are then one contiguous read, where a thread per point has 32 lanes in 32
 // places of the cache for every node and component.  Every lane forms its own node's three weights
 // and takes the others' y and z weights by shuffles; y is contracted first, then z, and the lane's x
-// weight comes last.  96^3, 1.5e6 points, width 6, points in no order: 3 components 1.49 -> 0.68 ms, 9
-// components 9.96 -> 2.18; in traversal order 0.79 -> 0.62 and 2.73 -> 1.88.  FP64 keeps a thread per
+// weight comes last.  96^3, 1.5e6 points, width 6, a thread per point and this, points in no order: 3
+// components 1.49 and 0.68 ms, 9 components 9.96 and 2.18; in traversal order 0.79 and 0.62, 2.73 and 1.88.  FP64 keeps a thread per
 // point: it is bound by the FP64 pipe, and the weights and sums that the lanes form more than once
 // would cost it a third more operations.
 template <int N2, int CC>
@@ -887,7 +887,7 @@ constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 // (owner_points).  The accumulators
 // are folded at their weights into a 192-bit sum; where a region goes in several stagings, these are added, in
 // 192 bits a node while no quantity has bits below window 0, then shifted to the unit of the last bit kept, in
-// 224 (in 224 from the first staging on the listed 256^3 scatter took 1% longer, width 8 at a point a cell 3%).
+// 224 (in 224 from the first staging on, 256^3 x 3 with 1e7 points takes 1% longer, width 8 at a point a cell 3%).
 // No bit is dropped between
 // the products and the final conversion, so the results depend neither on the order of the points nor on
 // how a region is cut.  The only roundings of a node are those of its weights, the quantities' last bit
@@ -896,10 +896,9 @@ constexpr int kDigits = sizeof(T) == 8 ? 3 : 2;
 // every node its stencil reaches, which is written as NaN (the reference's 0 * NaN included).
 //
 // Bound by issue and by the latency of a brick's phases (at 256^3 x 3 and 6e6 uniform points half of its
-// time is the listing and staging, half the trips, at 23 of 32 lanes).  What it replaced gave each warp
-// a point and added to 128-bit sums in shared memory by four dependent atomics per contribution; 256^3
-// x 3, 1e7 points with 30% in blobs, cubic: 21.4 ms, now 10.5.  Three CTAs per SM (80 registers, which
-// spill) take 12.0.
+// time is the listing and staging, half the trips, at 23 of 32 lanes).  256^3 x 3, 1e7 points with 30% in
+// blobs, cubic: 10.5 ms; a warp to a point, which adds to 128-bit sums in shared memory by four dependent
+// atomics per contribution, takes 21.4, and three CTAs per SM (80 registers, which spill) 12.0.
 constexpr int kOwnerPoints = 508;  // staged points, at most
 
 // The points that one staging may hold for weights up to L in P bits: a node adds each of them once to an
@@ -1443,9 +1442,9 @@ __global__ void k_to_one_based(const uint32_t *__restrict__ perm, int32_t *__res
 
 // Bound by the bitmap's L2 atomics, one per entry: a bit per point (an eighth of a byte to clear
 // and touch instead of a word), while the span and the number of points seen first are kept per
-// thread and reach the one global triple by three atomics a block.  With three atomics per entry, all
-// on that triple, 3e6 entries took 3.9 ms; now the order's whole rebuild, this check and a 9-component
-// gather at its points take 1.80 ms (5.72 before).
+// thread and reach the one global triple by three atomics a block.  Three atomics per entry, all on that
+// triple, take 3.9 ms for 3e6 entries; with these the order's whole rebuild, this check and a 9-component
+// gather at its points take 1.80 ms.
 __global__ void __launch_bounds__(kThreads)
     k_validate(const int32_t *__restrict__ order, int64_t m, uint32_t *__restrict__ seen, unsigned long long *stats) {
   __shared__ int32_t s_lo[kThreads / 32], s_hi[kThreads / 32];

@@ -180,9 +180,9 @@ __device__ __forceinline__ int64_t div_any(int64_t a, int64_t d) {
 }
 
 // A warp per padded row: the row's y and z are wrapped once, its lanes take consecutive x, so every
-// component is read along contiguous runs and a node is written in 16-byte pieces.  Bound by HBM: a
-// thread per node, with five 64-bit divisions, took 220 us for 256^3 x 3 FP32 (470 MB; 70 us at the copy
-// rate); now 88 us.
+// component is read along contiguous runs and a node is written in 16-byte pieces.  Bound by HBM: 88 us
+// for 256^3 x 3 FP32 (470 MB; 70 us at the copy rate); a thread per node, with five 64-bit divisions, takes
+// 220.
 template <typename T, int CP>
 __global__ void __launch_bounds__(kThreads)
     k_import(float *__restrict__ dst, int ncomp, int px, int py, int pz, int halo, int nx, int ny, int nz,
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Interior nodes back to the caller's planes, a warp per row of x: the node's components in 16-byte loads,
-// each plane's stores coalesced.  Bound by HBM (512^3 x 12: 2.11 ms; 2.2 with a thread per node,
-// 64-bit divisions and 4-byte loads 48 bytes apart; 128^3 x 3 10.9 us against 14.8).
+// each plane's stores coalesced.  Bound by HBM.  512^3 x 12: 2.11 ms, 2.2 with a thread per node, 64-bit
+// divisions and 4-byte loads 48 bytes apart; 128^3 x 3: 10.9 us and 14.8.
 template <int CP>
 __global__ void k_export(const float *__restrict__ srcp, int ncomp, int64_t px, int64_t py, int halo, int64_t nx,
                          int64_t ny, int64_t nz, void *dst, int dst_f64) {
@@ -433,9 +433,9 @@ __device__ __forceinline__ uint32_t bits_of(float x) { return __float_as_uint(x)
 // non-finite (an infinity becomes NaN, mod's own image of it).  A coordinate less than one extent
 // outside the box takes mod's value directly, which is exact there: itself within [0, extent), less
 // extent within [extent, 2 extent), plus extent (rounded, as mod adds it) below zero.  The tests are on
-// the bits (FP64 compares run at the FP64 rate), and an origin of zero neither shifts nor is added: fmod
-// and those operations were a good part of the FP64 work of moving a point (4e6 points, two terms, moved
-// and keyed: 401 -> 267 us; the seven FP64 operations a coordinate keeps take 173 us of the pipe).
+// the bits (FP64 compares run at the FP64 rate), and an origin of zero neither shifts nor is added.  4e6
+// points, two terms, moved and keyed: 267 us, of which the seven FP64 operations left a coordinate take
+// 173 of the pipe; 401 with fmod and those operations.
 template <typename T>
 __device__ __forceinline__ T wrap_coordinate(T x, T extent, T extent2, T origin) {
   const auto zero = bits_of(T(0));
@@ -1555,7 +1555,7 @@ __device__ bool scatter_brick_nodes(const FixGeo &g, const float *coef, int m2, 
     __syncthreads();
   }
   constexpr int half = N2 / 2;
-  // bricks and keys fit 32 bits: divisions of 64 took 0.2 of 10.3 ms at 512^3 x 12
+  // bricks and keys fit 32 bits: divisions of 64 take 0.2 of 10.3 ms at 512^3 x 12
   const uint32_t nb0 = (uint32_t)g.nb[0], nb1 = (uint32_t)g.nb[1], b32 = (uint32_t)b;
   const int bx = (int)(b32 % nb0), by = (int)((b32 / nb0) % nb1), bz = (int)(b32 / nb0 / nb1);
   const int B0 = g.b[0], B1 = g.b[1];
