@@ -1063,6 +1063,13 @@ __device__ __forceinline__ Int192 leading_bits(const unsigned long long *at, int
   return s;
 }
 
+// Whether a pass's first slots take the place of the cells' own, each moved on by what the pass lists, so that
+// the staging has the room of a second table: from width 6, whose regions go in several passes (150 x 111 x 97
+// x 3, 0.6 points a cell, width 6, FP32: 3.29 ms, 3.54 with the second table).  Up to width 4 the staging holds
+// its most points either way, and the kernel is 3% slower without the table.
+template <int N2>
+constexpr bool kSlotsMove = N2 >= 6;
+
 // The components from cfrom up to cto, CMAX at a time and the last REST of them by themselves.
 template <typename T, int N2, int CMAX, int REST>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -1083,8 +1090,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   uint32_t *off = reinterpret_cast<uint32_t *>(smem_owner + staging);  // ecount + 1 offsets
   uint32_t *r0s = off + ecount + 1;                                    // the cells' first slots
   uint32_t *poff = r0s + ecount;                                       // the same of one pass's share
-  uint32_t *pr0 = poff + ecount + 1;
-  uint32_t *fx = pr0 + ecount, *fy = fx + E0, *fz = fy + E1;           // per axis the first cell of a cell's brick
+  uint32_t *pr0 = kSlotsMove<N2> ? r0s : poff + ecount + 1;
+  uint32_t *fx = poff + ecount + 1 + (kSlotsMove<N2> ? 0 : ecount);    // per axis the first cell of a cell's brick
+  uint32_t *fy = fx + E0, *fz = fy + E1;
   uint32_t *vx = fz + E2, *vy = vx + E0, *vz = vy + E1;                // its place in it, and the brick's extent
   uint32_t *xe = vz + E2, *ye = xe + E0, *ze = ye + E1;                // per-axis exponent brick tables
   uint32_t *marked = ze + E2;                                          // bvol nodes' non-finite marks
@@ -1206,7 +1214,7 @@ __global__ void __launch_bounds__(kThreads, 2)
               const bool big = (at1 >> 32) != 0ull;
               const uint32_t a = big ? (uint32_t)(at0 / passes) : (uint32_t)at0 / passes;
               const uint32_t b = big ? (uint32_t)(at1 / passes) : (uint32_t)at1 / passes;
-              pr0[e] = r0s[e] + a;
+              if constexpr (!kSlotsMove<N2>) pr0[e] = r0s[e] + a;
               poff[e] = b - a;
             }
             __syncthreads();
@@ -1233,6 +1241,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                   ex += esx;
                   if (ex >= E0) ex -= E0;
                 }
+                if (kSlotsMove<N2> && multi && c1 == total)  // (a cell is the same thread's in every loop over them)
+                  for (int e = tid; e < ecount; e += blockDim.x) r0s[e] += po[e + 1] - po[e];
                 __syncthreads();
               }
               int left = 0;  // some quantity has bits below this window
@@ -1387,6 +1397,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (again) multi = true;
       } while (again);
       if (multi) {
+        if constexpr (kSlotsMove<N2>)
+          for (int e = tid; e < ecount; e += blockDim.x) r0s[e] -= off[e + 1] - off[e];
         __syncthreads();
         if (tid < bvol && inside(nx0, ny0, nz0)) {
           const int nl = (nz0 * B1 + ny0) * B0 + nx0;
@@ -1683,7 +1695,7 @@ gbg_status launch_owner(const GridT<T> &g, const ScatterPlan &P, int ncomp, int 
   constexpr size_t per = kDigitWords<CC, kDigits<T>> * 4 + kWeightWords<N2> * 8 + 4;
   const BrickGeo &bg = P.bg;
   const size_t e[3] = {(size_t)bg.b[0] + N2 - 1, (size_t)bg.b[1] + N2 - 1, (size_t)bg.b[2] + N2 - 1};
-  const size_t tables = sizeof(uint32_t) * (4 * e[0] * e[1] * e[2] + 2 + 3 * (e[0] + e[1] + e[2]) + (size_t)bg.bvol + (size_t)ncomp);
+  const size_t tables = sizeof(uint32_t) * ((kSlotsMove<N2> ? 3 : 4) * e[0] * e[1] * e[2] + 2 + 3 * (e[0] + e[1] + e[2]) + (size_t)bg.bvol + (size_t)ncomp);
   const size_t sums = ((size_t)bg.bvol * CC * 28 + 15) & ~size_t(15);
   // an SM's 228 KB over the CTAs that the launch bounds ask for, less 1 KB reserved and the static part
   const size_t budget = 228 * 1024 / 2 - 1024 - 512;
