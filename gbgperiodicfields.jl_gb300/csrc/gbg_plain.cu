@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     s_brick[0] = atomicAdd(ticket, 1u);
     s_lump = 0u;
   }
-  uint32_t piece = 0u;  // stagings so far; s_lump: the last one that a cell holds a third of
+  uint32_t passed = 0u;  // passes so far; s_lump: the last one that a cell holds a third of
   for (int it = 0;; ++it) {
     __syncthreads();
     const uint32_t brick = s_brick[it & 1];
@@ -1203,11 +1203,13 @@ __global__ void __launch_bounds__(kThreads, 2)
         // remainders falling in passes of their own), so that every pass has work for every node;
         // a pass above the staging's size goes in pieces.
         const uint32_t even = (uint32_t)(P * 7 / 8), passes = multi ? (count + even - 1) / even : 1u;
+        const uint32_t third = count / passes / 3u;  // of a pass's points
         for (uint32_t pass = 0; pass < passes && !again; ++pass) {
           const uint32_t *po = off, *pr = r0s;
           uint32_t total = count;
           if (multi) {
             __syncthreads();  // the previous pass is listed no longer
+            ++passed;
             for (int e = tid; e < ecount; e += blockDim.x) {
               const unsigned long long cells = off[e + 1] - off[e], phase = (uint32_t)e * 2654435761u % passes;
               const unsigned long long at0 = cells * pass + phase, at1 = at0 + cells;
@@ -1216,6 +1218,7 @@ __global__ void __launch_bounds__(kThreads, 2)
               const uint32_t b = big ? (uint32_t)(at1 / passes) : (uint32_t)at1 / passes;
               if constexpr (!kSlotsMove<N2>) pr0[e] = r0s[e] + a;
               poff[e] = b - a;
+              if (b - a > third) s_lump = passed;
             }
             __syncthreads();
             total = block_scan_counts(poff, ecount, warp_tot);
@@ -1230,10 +1233,8 @@ __global__ void __launch_bounds__(kThreads, 2)
             for (int win = 0; win < kDepth / (kDigit * ND); ++win) {
               __syncthreads();  // the previous points are summed (and the offsets' end is set)
               if (win == 0) {
-                ++piece;
                 for (int e = tid, ex = ex0; e < ecount; e += blockDim.x) {
                   const uint32_t o0 = po[e], lo = max(o0, c0), hi = min(po[e + 1], c1);
-                  if (multi && (int)(hi - lo) > np / 3) s_lump = piece;  // a cell holds a third of the points
                   for (uint32_t t = lo; t < hi; ++t) {
                     pslot[t - c0] = pr[e] + (t - o0);
                     reinterpret_cast<uint32_t *>(dig)[(t - c0) * DW + CC * ND] = (uint32_t)ex;
@@ -1331,7 +1332,7 @@ __global__ void __launch_bounds__(kThreads, 2)
               // A crowded region's nodes differ much in their points (at a blob's edge tenfold within a
               // brick), so a node has four lanes, each with a quarter of its rows, and the warps take the
               // 2x2x2 blocks of nodes as they get free.  (A thread a node there kept a fifth of the lanes
-              // busy.)  Where one cell holds a third of the staging, a lane has all rows and a quarter of the
+              // busy.)  Where one cell holds a third of the pass, a lane has all rows and a quarter of the
               // staging instead: 64^3 x 1, 1e6 points in one cell, 83 ms, by rows 184.
               const int nu0 = (B0 + 1) / 2, nu1 = (B1 + 1) / 2, units = nu0 * nu1 * ((B2 + 1) / 2);
               const int lane = tid & 31, part = lane & 3;
@@ -1345,7 +1346,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const int ebase = (lz * E1 + ly) * E0 + lx;
                 unsigned long long rows = 0ull;
                 uint32_t lo = c0, hi = c1;
-                if (s_lump == piece) {
+                if (s_lump == passed) {
                   lo += (uint32_t)(np * part / 4);
                   hi = c0 + (uint32_t)(np * (part + 1) / 4);
 #pragma unroll 1
