@@ -1081,7 +1081,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   constexpr int ND = kDigits<T>, WW = kWeightWords<N2>, half = N2 / 2;
   extern __shared__ __align__(16) unsigned char smem_owner[];
   __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t s_brick[2], s_unit, s_lump;
+  __shared__ uint32_t s_brick[2], s_unit;
   const int B0 = bg.b[0], B1 = bg.b[1], B2 = bg.b[2];
   const int E0 = B0 + N2 - 1, E1 = B1 + N2 - 1, E2 = B2 + N2 - 1, ecount = E0 * E1 * E2;
   const int bvol = (int)bg.bvol;
@@ -1115,11 +1115,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   // a thread's first region cell and the step to its next, as coordinates
   const int ex0 = tid % E0, ey0 = (tid / E0) % E1, ez0 = tid / (E0 * E1);
   const int esx = (int)blockDim.x % E0, esy = ((int)blockDim.x / E0) % E1, esz = (int)blockDim.x / (E0 * E1);
-  if (tid == 0) {
-    s_brick[0] = atomicAdd(ticket, 1u);
-    s_lump = 0u;
-  }
-  uint32_t passed = 0u;  // passes so far; s_lump: the last one that a cell holds a third of
+  if (tid == 0) s_brick[0] = atomicAdd(ticket, 1u);
   for (int it = 0;; ++it) {
     __syncthreads();
     const uint32_t brick = s_brick[it & 1];
@@ -1203,13 +1199,16 @@ __global__ void __launch_bounds__(kThreads, 2)
         // remainders falling in passes of their own), so that every pass has work for every node;
         // a pass above the staging's size goes in pieces.
         const uint32_t even = (uint32_t)(P * 7 / 8), passes = multi ? (count + even - 1) / even : 1u;
-        const uint32_t third = count / passes / 3u;  // of a pass's points
+        bool lump = false;  // a row of cells holds a third of the points
         for (uint32_t pass = 0; pass < passes && !again; ++pass) {
           const uint32_t *po = off, *pr = r0s;
           uint32_t total = count;
           if (multi) {
             __syncthreads();  // the previous pass is listed no longer
-            ++passed;
+            if (pass == 0) {
+              for (int r = tid; r < E1 * E2; r += blockDim.x) lump |= off[(r + 1) * E0] - off[r * E0] > count / 3u;
+              lump = __syncthreads_or(lump);
+            }
             for (int e = tid; e < ecount; e += blockDim.x) {
               const unsigned long long cells = off[e + 1] - off[e], phase = (uint32_t)e * 2654435761u % passes;
               const unsigned long long at0 = cells * pass + phase, at1 = at0 + cells;
@@ -1218,7 +1217,6 @@ __global__ void __launch_bounds__(kThreads, 2)
               const uint32_t b = big ? (uint32_t)(at1 / passes) : (uint32_t)at1 / passes;
               if constexpr (!kSlotsMove<N2>) pr0[e] = r0s[e] + a;
               poff[e] = b - a;
-              if (b - a > third) s_lump = passed;
             }
             __syncthreads();
             total = block_scan_counts(poff, ecount, warp_tot);
@@ -1332,8 +1330,8 @@ __global__ void __launch_bounds__(kThreads, 2)
               // A crowded region's nodes differ much in their points (at a blob's edge tenfold within a
               // brick), so a node has four lanes, each with a quarter of its rows, and the warps take the
               // 2x2x2 blocks of nodes as they get free.  (A thread a node there kept a fifth of the lanes
-              // busy.)  Where one cell holds a third of the pass, a lane has all rows and a quarter of the
-              // staging instead: 64^3 x 1, 1e6 points in one cell, 83 ms, by rows 184.
+              // busy.)  Where one row holds a third of the points, a lane has all rows and a quarter of the
+              // staging instead: 64^3 x 1, 1e6 points in one cell, 83 ms, by rows 184; in six along x, 105 and 205.
               const int nu0 = (B0 + 1) / 2, nu1 = (B1 + 1) / 2, units = nu0 * nu1 * ((B2 + 1) / 2);
               const int lane = tid & 31, part = lane & 3;
               while (true) {
@@ -1346,7 +1344,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const int ebase = (lz * E1 + ly) * E0 + lx;
                 unsigned long long rows = 0ull;
                 uint32_t lo = c0, hi = c1;
-                if (s_lump == passed) {
+                if (lump) {
                   lo += (uint32_t)(np * part / 4);
                   hi = c0 + (uint32_t)(np * (part + 1) / 4);
 #pragma unroll 1
