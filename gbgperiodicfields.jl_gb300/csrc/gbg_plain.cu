@@ -1081,7 +1081,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   constexpr int ND = kDigits<T>, WW = kWeightWords<N2>, half = N2 / 2;
   extern __shared__ __align__(16) unsigned char smem_owner[];
   __shared__ uint32_t warp_tot[32];
-  __shared__ uint32_t s_brick[2], s_unit;
+  __shared__ uint32_t s_brick[2], s_unit, s_lump;
   const int B0 = bg.b[0], B1 = bg.b[1], B2 = bg.b[2];
   const int E0 = B0 + N2 - 1, E1 = B1 + N2 - 1, E2 = B2 + N2 - 1, ecount = E0 * E1 * E2;
   const int bvol = (int)bg.bvol;
@@ -1115,7 +1115,11 @@ __global__ void __launch_bounds__(kThreads, 2)
   // a thread's first region cell and the step to its next, as coordinates
   const int ex0 = tid % E0, ey0 = (tid / E0) % E1, ez0 = tid / (E0 * E1);
   const int esx = (int)blockDim.x % E0, esy = ((int)blockDim.x / E0) % E1, esz = (int)blockDim.x / (E0 * E1);
-  if (tid == 0) s_brick[0] = atomicAdd(ticket, 1u);
+  if (tid == 0) {
+    s_brick[0] = atomicAdd(ticket, 1u);
+    s_lump = 0u;
+  }
+  uint32_t passed = 0u;  // passes so far; s_lump: the last one of a region with such cells in one row
   for (int it = 0;; ++it) {
     __syncthreads();
     const uint32_t brick = s_brick[it & 1];
@@ -1199,16 +1203,13 @@ __global__ void __launch_bounds__(kThreads, 2)
         // remainders falling in passes of their own), so that every pass has work for every node;
         // a pass above the staging's size goes in pieces.
         const uint32_t even = (uint32_t)(P * 7 / 8), passes = multi ? (count + even - 1) / even : 1u;
-        bool lump = false;  // a row of cells holds a third of the points
+        const uint32_t third = count / 3u;
         for (uint32_t pass = 0; pass < passes && !again; ++pass) {
           const uint32_t *po = off, *pr = r0s;
           uint32_t total = count;
           if (multi) {
             __syncthreads();  // the previous pass is listed no longer
-            if (pass == 0) {
-              for (int r = tid; r < E1 * E2; r += blockDim.x) lump |= off[(r + 1) * E0] - off[r * E0] > count / 3u;
-              lump = __syncthreads_or(lump);
-            }
+            ++passed;
             for (int e = tid; e < ecount; e += blockDim.x) {
               const unsigned long long cells = off[e + 1] - off[e], phase = (uint32_t)e * 2654435761u % passes;
               const unsigned long long at0 = cells * pass + phase, at1 = at0 + cells;
@@ -1217,6 +1218,9 @@ __global__ void __launch_bounds__(kThreads, 2)
               const uint32_t b = big ? (uint32_t)(at1 / passes) : (uint32_t)at1 / passes;
               if constexpr (!kSlotsMove<N2>) pr0[e] = r0s[e] + a;
               poff[e] = b - a;
+              // a node's cells in one row hold a third of the points (seen anew in every pass: found once a brick
+              // or a region, the trips came out 0.5 to 1% slower at width 4)
+              if (off[min(e + N2, ecount)] - off[e] > third) s_lump = passed;
             }
             __syncthreads();
             total = block_scan_counts(poff, ecount, warp_tot);
@@ -1344,7 +1348,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const int ebase = (lz * E1 + ly) * E0 + lx;
                 unsigned long long rows = 0ull;
                 uint32_t lo = c0, hi = c1;
-                if (lump) {
+                if (s_lump == passed) {
                   lo += (uint32_t)(np * part / 4);
                   hi = c0 + (uint32_t)(np * (part + 1) / 4);
 #pragma unroll 1
