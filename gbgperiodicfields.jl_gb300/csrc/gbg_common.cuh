@@ -269,10 +269,12 @@ gbg_status radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, ui
 // (starts[k+1] - starts[k] points per key).  perm[s] = the point in slot s, points of one key in
 // index order -- the order the stable radix sort gives.  big[0] and big[4] must be zero on entry (keys with
 // more than 1024 points are counted there and sorted apart).  temp holds n words.  With rec_user and rec
-// given, rec[s] = rec_user[perm[s]] is written too.
+// given, rec[s] = rec_user[perm[s]] is written too.  With rest given, the longest runs are left to the caller's
+// next launch (place_huge in gbg_sort.cuh), which saves one.
+struct HugeRuns;
 gbg_status stable_counting_sort(const uint32_t *keys, uint32_t *rank, const uint32_t *starts, int64_t n, uint32_t *perm,
                                 uint32_t *big, uint32_t *temp, cudaStream_t stream, const float4 *rec_user = nullptr,
-                                float4 *rec = nullptr);
+                                float4 *rec = nullptr, HugeRuns *rest = nullptr);
 
 // Grid-stride launch shape: a multiple of the SM count.
 int launch_blocks(int64_t work, int threads, int per_sm = 8);

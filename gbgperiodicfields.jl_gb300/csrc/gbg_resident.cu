@@ -34,7 +34,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "gbg_common.cuh"
+#include "gbg_sort.cuh"
 
 struct gbg_field_s {
   int device = 0;
@@ -537,10 +537,12 @@ __global__ void __launch_bounds__(kThreads)
 // The bins' work lists: bricks holding a point, and bricks whose 27 neighbours (periodic)
 // hold one -- the bricks a stencil of up to 8 nodes can reach when every brick (and the
 // last, partial one) is at least 4 cells wide (reach_ok).  Their order is whatever the
-// atomics give: each list only says which bricks to visit.
-__global__ void k_brick_lists(const uint32_t *__restrict__ cell_start, int64_t nbx, int64_t nby, int64_t nbz,
-                              int64_t bvol, int reach_ok, uint32_t *__restrict__ active,
-                              uint32_t *__restrict__ reach, uint32_t *__restrict__ lists_n) {
+// atomics give: each list only says which bricks to visit.  The launch also places the sort's longest runs (one
+// of its own that returns at once for most sets took 4 of the 535 us of a 128^3 x 3 step).
+__global__ void __launch_bounds__(kRunThreads)
+    k_brick_lists(const uint32_t *__restrict__ cell_start, int64_t nbx, int64_t nby, int64_t nbz, int64_t bvol,
+                  int reach_ok, uint32_t *__restrict__ active, uint32_t *__restrict__ reach,
+                  uint32_t *__restrict__ lists_n, HugeRuns runs) {
   const int64_t nbricks = nbx * nby * nbz;
   auto holds = [&](int64_t b) { return __ldg(cell_start + (b + 1) * bvol) > __ldg(cell_start + b * bvol); };
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbricks; b += (int64_t)gridDim.x * blockDim.x) {
@@ -555,6 +557,7 @@ __global__ void k_brick_lists(const uint32_t *__restrict__ cell_start, int64_t n
       near = holds((step(bz, d / 9 - 1, nbz) * nby + step(by, (d / 3) % 3 - 1, nby)) * nbx + step(bx, d % 3 - 1, nbx));
     if (near) reach[atomicAdd(lists_n + 1, 1u)] = (uint32_t)b;
   }
+  place_huge(runs);
 }
 
 __global__ void k_order_from_perm(const uint32_t *__restrict__ perm, int32_t *__restrict__ order, int64_t m) {
@@ -3262,10 +3265,11 @@ gbg_status bins_build_impl(gbg_bins_s *b, const T *positions, int64_t npoints, i
   // place the points, and a per-cell pass puts each cell's points in index order (the
   // stable order) with their records
   GBG_TRY(exclusive_scan_u32(b->cell_start, b->cell_start, b->nkeys + 1, b->scan_tmp, st));
+  HugeRuns runs;
   GBG_TRY(stable_counting_sort(b->keys, b->rank, b->cell_start, npoints, b->perm, b->lists_n + 2, b->sort_tmp, st,
-                               b->rec_user, b->rec));
-  k_brick_lists<<<launch_blocks(b->nbricks, kThreads), kThreads, 0, st>>>(
-      b->cell_start, b->nb[0], b->nb[1], b->nb[2], b->bvol, b->reach_ok ? 1 : 0, b->active, b->reach, b->lists_n);
+                               b->rec_user, b->rec, &runs));
+  k_brick_lists<<<std::max(launch_blocks(b->nbricks, kRunThreads), runs.shares), kRunThreads, 0, st>>>(
+      b->cell_start, b->nb[0], b->nb[1], b->nb[2], b->bvol, b->reach_ok ? 1 : 0, b->active, b->reach, b->lists_n, runs);
   note_launch();
   GBG_CUDA_TRY(cudaGetLastError());
   return GBG_OK;

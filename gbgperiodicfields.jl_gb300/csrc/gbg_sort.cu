@@ -8,7 +8,7 @@
 // identical run to run.
 #include <algorithm>
 
-#include "gbg_common.cuh"
+#include "gbg_sort.cuh"
 
 namespace gbg {
 
@@ -23,7 +23,6 @@ constexpr int kRsThreads = 256;
 constexpr int kRsItems = 16;
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsTile = kRsThreads * kRsItems;  // 4096
-constexpr int kRsBins = 256;
 
 // Block-wide exclusive scan of one value per thread; returns the block total via *total.
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *warp_sums,
@@ -318,58 +317,8 @@ __global__ void k_place_stable(const uint32_t *__restrict__ keys, const uint32_t
   }
 }
 
-// Where a tile's items go when they are placed by digit, in their order within one: base[d] is the next free
-// place of digit d, and is moved on.  Items of digit kRsBins go nowhere.  A warp's items are consecutive, 32 at
-// a time; every thread of the CTA calls it, and may use wh again after it.
-template <int WARPS, int ITEMS>
-__device__ __forceinline__ void tile_places(const uint32_t (&digit)[ITEMS], uint32_t (&pos)[ITEMS],
-                                            uint32_t (&wh)[WARPS][kRsBins], uint32_t *base) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t lower = (1u << lane) - 1u;
-  for (int k = threadIdx.x; k < WARPS * kRsBins; k += WARPS * 32) (&wh[0][0])[k] = 0u;
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r)
-    if (digit[r] < kRsBins) atomicAdd(&wh[warp][digit[r]], 1u);
-  __syncthreads();
-  if (threadIdx.x < kRsBins) {
-    uint32_t run = base[threadIdx.x];
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-      const uint32_t x = wh[w][threadIdx.x];
-      wh[w][threadIdx.x] = run;
-      run += x;
-    }
-    base[threadIdx.x] = run;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < ITEMS; ++r) {
-    const bool valid = digit[r] < kRsBins;
-    const uint32_t peers = __match_any_sync(0xffffffffu, digit[r]);
-    pos[r] = 0;
-    if (valid) pos[r] = wh[warp][digit[r]] + __popc(peers & lower);
-    __syncwarp();
-    if (valid && lane == 31 - __clz(peers)) wh[warp][digit[r]] += __popc(peers);
-    __syncwarp();
-  }
-  __syncthreads();
-}
-
 // A run of more points than this is not sorted by one CTA (which would take 0.1 ms).
 constexpr int64_t kHugeRun = 16384;
-constexpr int kRunThreads = 512, kRunWarps = kRunThreads / 32, kRunItems = 4, kRunTile = kRunThreads * kRunItems;
-
-// The points that a block of the huge runs' placement takes: an even share, a whole number of tiles.
-__device__ __forceinline__ int64_t huge_share(int64_t n) {
-  return ((n + gridDim.x - 1) / gridDim.x + kRunTile - 1) / kRunTile * kRunTile;
-}
-// The place of point p's run in the list of huge runs, or kRsBins.
-__device__ __forceinline__ uint32_t huge_digit(const uint32_t *keys, const uint32_t *starts, const uint32_t *huge_id,
-                                               int64_t p, uint32_t limit) {
-  const uint32_t k = __ldg(keys + p), a = __ldg(starts + k);
-  return __ldg(starts + k + 1) - a > limit ? huge_id[a] : (uint32_t)kRsBins;
-}
 
 // The long runs, one CTA each at a time: a stable LSD radix sort of the run's point indices between its
 // slots of perm_u and of perm, eight bits a pass, and the records in their order.  One launch that
@@ -388,7 +337,7 @@ __global__ void __launch_bounds__(kRunThreads)
   if (nhuge) {
     if (threadIdx.x < kRsBins) base[threadIdx.x] = 0u;
     __syncthreads();
-    const int64_t share = huge_share(n), from = blockIdx.x * share, to = min(n, from + share);
+    const int64_t share = huge_share(n, gridDim.x), from = blockIdx.x * share, to = min(n, from + share);
     for (int64_t p = from + threadIdx.x; p < to; p += kRunThreads) {
       const uint32_t d = huge_digit(keys, starts, perm_u, p, limit);
       if (d < kRsBins) atomicAdd(&base[d], 1u);
@@ -445,44 +394,7 @@ __global__ void __launch_bounds__(kRunThreads)
   }
 }
 
-// The huge runs: every block goes through its share of the points in their order and places those of huge
-// runs behind the ones that earlier blocks counted, all such runs at once (there are at most 254, `limit` being
-// at least n / 255).  1e6 points of 1e7 in one cell: the bins built in 1.2 ms, 7.7 with that cell sorted by one
-// CTA.
-__global__ void __launch_bounds__(kRunThreads)
-    k_place_huge(const uint32_t *big, const uint32_t *__restrict__ huge, const uint32_t *__restrict__ keys,
-                 const uint32_t *__restrict__ starts, const uint32_t *__restrict__ huge_id, uint32_t *__restrict__ perm,
-                 const float4 *__restrict__ rec_user, float4 *__restrict__ rec, int64_t n, uint32_t limit,
-                 const uint32_t *__restrict__ counts) {
-  const uint32_t nhuge = big[4];
-  if (nhuge == 0u) return;
-  __shared__ uint32_t wh[kRunWarps][kRsBins], base[kRsBins];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < nhuge) {
-    uint32_t at = huge[threadIdx.x];
-    for (unsigned b = 0; b < blockIdx.x; ++b) at += counts[b * kRsBins + threadIdx.x];
-    base[threadIdx.x] = at;
-  }
-  const int64_t share = huge_share(n), from = blockIdx.x * share, to = min(n, from + share);
-  for (int64_t t0 = from; t0 < to; t0 += kRunTile) {
-    const int64_t seg = t0 + warp * (32 * kRunItems) + lane;
-    uint32_t digit[kRunItems], pos[kRunItems];
-    bool some = false;
-#pragma unroll
-    for (int r = 0; r < kRunItems; ++r) {
-      digit[r] = seg + 32 * r < to ? huge_digit(keys, starts, huge_id, seg + 32 * r, limit) : (uint32_t)kRsBins;
-      some |= digit[r] < kRsBins;
-    }
-    if (!__syncthreads_or(some)) continue;
-    tile_places<kRunWarps>(digit, pos, wh, base);
-#pragma unroll
-    for (int r = 0; r < kRunItems; ++r)
-      if (digit[r] < kRsBins) {
-        perm[pos[r]] = (uint32_t)(seg + 32 * r);
-        if (rec) rec[pos[r]] = rec_user[seg + 32 * r];
-      }
-  }
-}
+__global__ void __launch_bounds__(kRunThreads) k_place_huge(HugeRuns h) { place_huge(h); }
 
 }  // namespace
 
@@ -563,7 +475,8 @@ gbg_status radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, ui
 
 gbg_status stable_counting_sort(const uint32_t *keys, uint32_t *rank, const uint32_t *starts, int64_t n, uint32_t *perm,
                                 uint32_t *big, uint32_t *temp, cudaStream_t stream, const float4 *rec_user,
-                                float4 *rec) {
+                                float4 *rec, HugeRuns *rest) {
+  if (rest) *rest = HugeRuns{};
   if (n <= 0) return GBG_OK;
   if (n > 0x7fffffffLL) return set_error(GBG_EUNSUPPORTED, "counting sort: more than 2^31-1 points");
   const int blocks = launch_blocks(n, 256);
@@ -583,9 +496,13 @@ gbg_status stable_counting_sort(const uint32_t *keys, uint32_t *rank, const uint
                                                         counts);
     note_launch();
     if (n > kHugeRun) {
-      k_place_huge<<<run_blocks, kRunThreads, 0, stream>>>(big, huge, keys, starts, temp, perm, rec_user, rec, n, limit,
-                                                           counts);
-      note_launch();
+      const HugeRuns runs{big, huge, keys, starts, temp, perm, rec_user, rec, n, limit, counts, run_blocks};
+      if (rest) {
+        *rest = runs;
+      } else {
+        k_place_huge<<<run_blocks, kRunThreads, 0, stream>>>(runs);
+        note_launch();
+      }
     }
   }
   GBG_CUDA_TRY(cudaGetLastError());
